@@ -227,7 +227,7 @@ static void free_engine(PgaEngine* e) {
   void* ptrs[] = {e->dRules, e->dParams, e->dSucc, e->dExpPool, e->dState, e->dNodes, e->dNodeRot, e->dLevelClock,
                   e->dTail, e->dTailLinks, e->dScratch,
                   e->dTermLinks, e->dLevelStart, e->dScratchCount, e->dSortTemp, e->dKeysA,
-                  e->dValsA, e->dValsB, e->dArrival, e->dLeafAabb, e->dLeafAabbSorted, e->dNodeOther, e->dNodeGrad, e->dChildKey, e->dPageNext,
+                  e->dValsA, e->dValsB, e->dOpenTrees, e->dNodeGrad, e->dChildKey, e->dPageNext,
                   e->dSlots, e->dBlockSums, e->dGroupCount};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -240,6 +240,7 @@ static void free_engine(PgaEngine* e) {
 }
 
 size_t pga_lbvh_temp_bytes(uint64_t n);  // lbvh.cu
+size_t pga_lbvh_open_bytes(uint64_t n);  // lbvh.cu
 
 PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* config, PgaEngine** out) {
   if (!table || !out || !table->entries || !table->procs || table->numEntries == 0) {
@@ -498,12 +499,9 @@ PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* co
   e->sortTempBytes = pga_lbvh_temp_bytes(c.maxTerminals);
   ALLOC(e->dSortTemp, e->sortTempBytes);
   ALLOC(e->dKeysA, c.maxTerminals * sizeof(unsigned long long));
-  ALLOC(e->dLeafAabb, c.maxTerminals * 6 * sizeof(float));
-  ALLOC(e->dLeafAabbSorted, c.maxTerminals * 6 * sizeof(float));
-  ALLOC(e->dNodeOther, c.maxTerminals * sizeof(int32_t));
   ALLOC(e->dValsA, c.maxTerminals * sizeof(uint32_t));
   ALLOC(e->dValsB, c.maxTerminals * sizeof(uint32_t));
-  ALLOC(e->dArrival, c.maxTerminals * sizeof(uint32_t));
+  ALLOC(e->dOpenTrees, pga_lbvh_open_bytes(c.maxTerminals));
 #undef ALLOC
   err = cudaMemcpy(e->dRules, e->hRules.data(), e->hRules.size() * sizeof(DevRule), cudaMemcpyHostToDevice);
   if (err == cudaSuccess)

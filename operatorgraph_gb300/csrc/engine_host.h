@@ -65,10 +65,7 @@ struct PgaEngine {
   unsigned long long* dKeysA = nullptr;
   uint32_t* dValsA = nullptr;
   uint32_t* dValsB = nullptr;
-  uint32_t* dArrival = nullptr;
-  float* dLeafAabb = nullptr;        // LBVH leaf boxes in terminal order
-  float* dLeafAabbSorted = nullptr;  // the same in sorted (leaf) order
-  int32_t* dNodeOther = nullptr;     // LBVH internal node i: the other end of its leaf range (one end is i)
+  void* dOpenTrees = nullptr;  // the LBVH tiles' open subtrees and their counts
 
   // Adjoint scratch: per work item the gradient of (translation, size), its
   // child key and the next page of the same child; the child slots (slotCap

@@ -1,4 +1,5 @@
-// LBVH over terminal boxes: Morton keys, radix sort, Karras topology, refit.
+// LBVH over terminal boxes: Morton keys, radix sort, and the tree (Karras's
+// topology and node numbers, with the boxes) joined bottom up in one kernel.
 //
 // Restates ContextSensitivity::GPU::BVHConstructor::construct
 // (include/pga/core/GPUBVHConstructor.cuh:44-331) for the terminal records of
@@ -8,8 +9,8 @@
 //    instead of the emission index, which depends on queue order;
 //  * the Karras codes are morton30 << 32 | sorted position, as the reference's
 //    `(code << 32) | j` with j replaced by that deterministic position;
-//  * AABBs start from -FLT_MAX instead of FLT_MIN (AABB.cuh:20) and a fence
-//    orders each node's AABB store before its parent's arrival counter.
+//  * AABBs start from -FLT_MAX instead of FLT_MIN (AABB.cuh:20) and the two
+//    climbers that meet at a node are ordered by an acquire-release exchange.
 // The reference sorts with thrust::sort (GPUBVHConstructor.cuh:311-312); here
 // the sort is this file's own onesweep radix sort (see k_onesweep).
 #include <cuda_runtime.h>
@@ -41,8 +42,12 @@ struct Bounds {
 
 // Leaf AABB: corners of the terminal box (8) or quad (4), as
 // BoundingVolumeConstructor<AABB>::construct (BoundingVolumeConstructor.cuh:22-76)
-// with the scale folded into the terminal matrix.
-__device__ __forceinline__ void leaf_aabb(const float4 r[3], bool quad, float mn[3], float mx[3]) {
+// with the scale folded into the terminal matrix.  Rounding is monotone, so the
+// smallest corner sum is the sum with every term negative and the largest the
+// one with every term positive; where those are finite so is every corner, and
+// the eight corners need not be formed.
+__device__ __noinline__ void leaf_aabb_corners(float4 r0, float4 r1, float4 r2, bool quad, float mn[3], float mx[3]) {
+  const float4 r[3] = {r0, r1, r2};
 #pragma unroll
   for (int k = 0; k < 3; k++) { mn[k] = FLT_MAX; mx[k] = -FLT_MAX; }
   for (int cz = 0; cz < (quad ? 1 : 2); cz++)
@@ -58,6 +63,19 @@ __device__ __forceinline__ void leaf_aabb(const float4 r[3], bool quad, float mn
           mx[k] = fmaxf(mx[k], v);
         }
       }
+}
+__device__ __forceinline__ void leaf_aabb(const float4 r[3], bool quad, float mn[3], float mx[3]) {
+  bool finite = true;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const float hx = fabsf(__fmul_rn(r[k].x, 0.5f)), hy = fabsf(__fmul_rn(r[k].y, 0.5f));
+    const float hz = fabsf(__fmul_rn(r[k].z, quad ? 0.0f : 0.5f));
+    const float h = __fadd_rn(__fadd_rn(hx, hy), hz);
+    mn[k] = __fsub_rn(r[k].w, h);
+    mx[k] = __fadd_rn(r[k].w, h);
+    finite = finite && fabsf(mn[k]) < FLT_MAX && fabsf(mx[k]) < FLT_MAX;
+  }
+  if (!finite) leaf_aabb_corners(r[0], r[1], r[2], quad, mn, mx);
 }
 
 // Leaf count of a build: the host value `n`, or, when the count lives on the
@@ -89,40 +107,29 @@ __device__ __forceinline__ void hist_add(uint32_t* h, uint32_t d, bool valid) {
 }
 
 // generateMortonCodes (GPUBVHConstructor.cuh:66-86) on terminal centres.
-// Also writes each terminal's AABB (6 floats, terminal order) while its record
-// is in registers.  The sort's values start as the terminal index, which its
-// first pass generates, so none are written here.
+// The sort's values start as the terminal index, which its first pass
+// generates, so none are written here.
 // With a device count, the keys in [count, capacity) are padding: all ones,
 // after every real key in the stable radix sort (a real key can equal it only
 // in the sorted top bits, and it comes first there by input order).
 __global__ void __launch_bounds__(kLbvhThreads) k_morton(const PgaTerminal* __restrict__ t, unsigned long long cap,
                                                          const unsigned long long* __restrict__ dN, Bounds b,
-                                                         unsigned long long* __restrict__ keys,
-                                                         float* __restrict__ leafBox) {
+                                                         unsigned long long* __restrict__ keys) {
   unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cap) return;
   if (i >= leaf_count(dN, cap)) {
     keys[i] = ~0ull;
     return;
   }
-  const float4* p = reinterpret_cast<const float4*>(t + i);
-  float4 r[3] = {__ldg(p + 0), __ldg(p + 1), __ldg(p + 2)};
-  uint4 meta = __ldg(reinterpret_cast<const uint4*>(p + 3));
-  float mn[3], mx[3];
-  leaf_aabb(r, (meta.x >> 31) != 0, mn, mx);
-  float2* lb = reinterpret_cast<float2*>(leafBox + i * 6);
-  lb[0] = make_float2(mn[0], mn[1]);
-  lb[1] = make_float2(mn[2], mx[0]);
-  lb[2] = make_float2(mx[1], mx[2]);
-  float c[3] = {r[0].w, r[1].w, r[2].w};
+  const float c[3] = {__ldg(&t[i].m[3]), __ldg(&t[i].m[7]), __ldg(&t[i].m[11])};
+  const uint2 path = __ldg(reinterpret_cast<const uint2*>(&t[i].path));
   uint32_t code = 0;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     float nc = __fdiv_rn(__fsub_rn(c[k], b.mn[k]), b.sz[k]);
     code |= spread(__float2uint_rz(__fmul_rn(nc, 1023.0f))) << k;
   }
-  uint64_t path = ((uint64_t)meta.w << 32) | meta.z;
-  keys[i] = ((unsigned long long)code << 34) | (path >> 30);
+  keys[i] = ((unsigned long long)code << 34) | ((((uint64_t)path.y << 32) | path.x) >> 30);
 }
 
 // The four digit histograms of keys [0, n) (kSortPasses x kBins, zeroed
@@ -379,390 +386,784 @@ __device__ __forceinline__ uint64_t term_path(const PgaTerminal* t, uint32_t i) 
   return ((uint64_t)v.y << 32) | v.x;
 }
 
-// The radix sort orders the keys' top bits [kSortLowBit, 64) only, which
-// leaves runs of equal top bits in input order (terminals in one Morton cell
-// whose path hashes share their top 10 bits: short runs, but about half of
-// the keys of a crowded scene lie in one).  The final order inside a run is
-// by the whole key (the Morton code and the path hash's top 34 bits), then,
-// for equal keys, by the full path hash, then by terminal index:
-// lexicographic in (Morton code, path hash, terminal), the order a full
-// 64-bit sort plus tie fix gives.  Each member of a run counts the members
-// that come before it and writes its key and value at run start + that count
-// into tieKeys / tieVals; one bit per position in tieMask marks the members.
-// The Karras pass takes a marked position's value from tieVals and the refit
-// writes its key from tieKeys, so the keys' top bits, all the Karras codes
-// read, do not change while a later kernel reads them.
+// ------------------------------------------------------------------ the tree
 //
-// A warp ranks its 32 keys inside a window of kTieReach keys either side
-// (lane l holds window positions l and 32 + l): run boundaries from two
-// ballots of "equal to the left neighbour", and each member compares the low
-// 32 bits of its key (the rest is equal inside a run) with those of its run's
-// members, staged in shared memory.  A run that reaches the window's edge, or
-// that holds equal keys (then the paths decide), is ranked by the member
-// alone in global memory, reading a terminal record only for equal keys.
-constexpr int kTieReach = 16;
-__device__ __noinline__ void tie_rank_global(const unsigned long long* __restrict__ keys,
-                                             const uint32_t* __restrict__ vals, const PgaTerminal* __restrict__ t,
-                                             unsigned long long n, unsigned long long i,
-                                             unsigned long long* __restrict__ tieKeys,
-                                             uint32_t* __restrict__ tieVals) {
-  const unsigned long long ki = keys[i], k = ki >> kSortLowBit;
-  unsigned long long s = i, e = i + 1;
-  while (s > 0 && (keys[s - 1] >> kSortLowBit) == k) s--;
-  while (e < n && (keys[e] >> kSortLowBit) == k) e++;
-  const uint32_t vi = vals[i];
-  bool havePath = false;
-  uint64_t pi = 0;
-  unsigned long long before = 0;
-  for (unsigned long long b = s; b < e; b++) {
-    const unsigned long long kb = keys[b];
-    if (kb != ki) {
-      before += kb < ki;
-    } else if (b != i) {
-      if (!havePath) {
-        pi = term_path(t, vi);
-        havePath = true;
-      }
-      const uint32_t vb = vals[b];
-      const uint64_t pb = term_path(t, vb);
-      before += pb < pi || (pb == pi && vb < vi);
-    }
-  }
-  tieKeys[s + before] = ki;
-  tieVals[s + before] = vi;
-}
+// buildRadixTree and propagateBVH (GPUBVHConstructor.cuh:88-261) in one
+// bottom-up kernel.  A block takes kTile consecutive sorted leaves, puts the
+// leaves of equal sorted bits in their final order, gathers the leaves'
+// records and joins neighbouring subtrees in shared memory: subtree [l, r] is
+// joined across its boundary with the longer common prefix (the agglomerative
+// construction of Apetrei, 2014), the second of the two climbers that reach a
+// boundary goes on.  A joined node has the index Karras gives it: its right
+// end when it is a left child, its left end otherwise.  Subtrees whose parent
+// reaches past the tile stay open (one for every node that crosses the tile's
+// ends: about a dozen, at most kMaxOpen) and are left to k_join, which joins
+// those of kGroup tiles at a time, then of kGroup groups, up to the root.
+//
+// This replaces four kernels (tie ranks, Karras's searches, and a refit in
+// two).  They were bound by latency: dependent probes per node, and climbs to
+// the root through counters at GPU scope; and they moved each leaf's box
+// through memory three times and each node's links twice.  Here a leaf costs
+// its key, value and record read once (76 bytes) and the results written once
+// (52 bytes).  Measured with k_join: 51 -> 21 us at 20,011 leaves, 251 -> 166
+// us at 3.0M, 421 -> 311 us for the city's 5.9M, of which 135 us are the bytes
+// at the copy rate and the rest the climb (93 us) and its barriers.  Tile of
+// 256: a climb in it is eight to fifteen steps, and six blocks of it fit on an
+// SM (five 276 us, eight, with spills, 321 us on the city; six 264), so that
+// the gathers and climbs of different tiles overlap.  Groups of 32: two levels
+// of joining for a million leaves, three for 268M.
 
-__global__ void __launch_bounds__(kLbvhThreads) k_tie_rank(const unsigned long long* __restrict__ keys,
-                                                           const uint32_t* __restrict__ vals,
-                                                           const PgaTerminal* __restrict__ t, unsigned long long cap,
-                                                           const unsigned long long* __restrict__ dN,
-                                                           unsigned long long* __restrict__ tieKeys,
-                                                           uint32_t* __restrict__ tieVals,
-                                                           uint32_t* __restrict__ tieMask) {
-  constexpr unsigned kAll = 0xFFFFFFFFu;
-  __shared__ uint32_t sWin[kLbvhThreads / 32 * 64];
-  const long long n = (long long)leaf_count(dN, cap);
-  const int lane = (int)(threadIdx.x & 31u);
-  const long long w0 = ((long long)blockIdx.x * kLbvhThreads + threadIdx.x) & ~31ll;
-  if (w0 >= n) return;  // the whole warp
-  // window position q <-> key w0 - kTieReach + q; lane holds q = lane (a) and q = 32 + lane (b)
-  const long long ga = w0 - kTieReach + lane, gb = ga + 32;
-  const bool va = ga >= 0 && ga < n, vb = gb < n;
-  const unsigned long long ka = va ? keys[ga] : 0ull, kb = vb ? keys[gb] : 0ull;
-  const unsigned long long ta = ka >> kSortLowBit, tb = kb >> kSortLowBit;
-  // left neighbours: a's is lane - 1's a; b's is lane - 1's b, lane 0's is lane 31's a
-  const unsigned long long la = __shfl_up_sync(kAll, ta, 1);
-  const int lva = __shfl_up_sync(kAll, (int)va, 1);
-  const int src = (lane + 31) & 31;
-  const unsigned long long lb = __shfl_sync(kAll, lane == 31 ? ta : tb, src);
-  const int lvb = __shfl_sync(kAll, lane == 31 ? (int)va : (int)vb, src);
-  const bool eqa = lane > 0 && va && lva && la == ta;
-  const bool eqb = vb && lvb && lb == tb;
-  const unsigned long long eq = (unsigned long long)__ballot_sync(kAll, eqa) |
-                                ((unsigned long long)__ballot_sync(kAll, eqb) << 32);
-  // this lane's key sits at window position p (eq bit q: q and q - 1 in one run)
-  const int p = kTieReach + lane;
-  const long long i = w0 + lane;
-  const bool inRun = i < n && (((eq >> p) & 1ull) || ((eq >> (p + 1)) & 1ull));
-  const unsigned members = __ballot_sync(kAll, inRun);
-  if (lane == 0) tieMask[w0 >> 5] = members;
-  if (members == 0u) return;  // the whole warp
-  const unsigned long long upto = (2ull << p) - 1ull;  // positions [0, p]
-  const int s = 63 - __clzll(~eq & upto);              // eq bit 0 is clear: the run's first position
-  const unsigned long long past = ~eq & ~upto;
-  const int e = past ? __ffsll((long long)past) - 2 : 63;  // the run's last position
-  const bool inWindow = inRun && s > 0 && e < 63;
-  // the window's low key halves in this warp's slice of shared memory
-  uint32_t* win = sWin + (threadIdx.x >> 5) * 64;
-  win[lane] = (uint32_t)ka;
-  win[32 + lane] = (uint32_t)kb;
-  __syncwarp();
-  uint32_t before = 0;
-  bool equal = false;
-  if (inWindow) {
-    const uint32_t li = win[p];
-    for (int q = s; q <= e; q++) {
-      const uint32_t v = win[q];
-      before += v < li;
-      equal |= v == li && q != p;
-    }
-  }
-  if (!inRun) return;
-  if (inWindow && !equal) {
-    const long long dst = w0 - kTieReach + s + (long long)before;
-    tieKeys[dst] = keys[i];
-    tieVals[dst] = vals[i];
-  } else {
-    tie_rank_global(keys, vals, t, (unsigned long long)n, (unsigned long long)i, tieKeys, tieVals);
-  }
-}
+constexpr uint32_t kTile = kLbvhThreads;  // leaves per block
+constexpr uint32_t kGroup = 32;           // tiles, then groups, joined by the last to finish
+constexpr uint32_t kHalo = 32;            // keys either side of a tile that its tie runs may reach into
+// A tile's open subtrees hang off the two paths from its end leaves up to the
+// tile's topmost crossing node, at most one on each level of a path; the
+// codes have 30 Morton and 30 position bits.
+constexpr uint32_t kMaxOpen = 128;
+constexpr uint32_t kJoin = 512;  // open subtrees joined at once
 
-__device__ __forceinline__ bool tie_member(const uint32_t* tieMask, unsigned long long i) {
-  return (__ldg(tieMask + (i >> 5)) >> (i & 31u)) & 1u;
-}
+struct __align__(16) OpenTree {
+  float box[6];
+  uint32_t left;  // first leaf (the next open subtree's is this one's end)
+  int32_t delta;  // common prefix of the codes at left - 1 and left; -1 at the first leaf
+};
+static_assert(sizeof(OpenTree) == 32, "two 16-byte words");
 
-__device__ __forceinline__ unsigned long long karras_code(const unsigned long long* keys, long long j) {
-  return ((keys[j] >> 34) << 32) | (unsigned long long)j;
-}
+struct TreeArgs {
+  const unsigned long long* keys;  // sorted by their top bits (kSortLowBit and up)
+  const uint32_t* vals;
+  const PgaTerminal* t;
+  unsigned long long cap;
+  const unsigned long long* dN;
+  int32_t* nodes;
+  uint32_t* leafParents;
+  float* aabbs;
+  uint32_t* leafTerminal;
+  unsigned long long* outKeys;
+  OpenTree* open;       // kMaxOpen per tile
+  uint32_t* openCount;  // per tile
+  uint32_t* joins;      // arrivals per group, level after level (zero before the launch)
+};
 
-// buildRadixTree (GPUBVHConstructor.cuh:88-213), one thread per internal node,
-// with bounds checks on every probe.
-// Also gathers the leaves' terminal indices (a tie-run member's from
-// tieVals) and boxes into sorted order (one independent load per leaf here
-// instead of a dependent one ahead of the refit's climb), writes the other
-// end of each node's leaf range (one end is the node's own index) and clears
-// the refit's arrival counters.  Fewer than two leaves make no tree.
-__global__ void __launch_bounds__(kLbvhThreads) k_karras(const unsigned long long* __restrict__ keys, long long cap,
-                                                         const unsigned long long* __restrict__ dN,
-                                                         int32_t* __restrict__ nodes, uint32_t* __restrict__ leafParents,
-                                                         uint32_t* __restrict__ sortedVals, const uint32_t* __restrict__ vals,
-                                                         const uint32_t* __restrict__ tieMask,
-                                                         const uint32_t* __restrict__ tieVals,
-                                                         const float* __restrict__ leafBox,
-                                                         float* __restrict__ sortedBox,
-                                                         int32_t* __restrict__ nodeOther, uint32_t* __restrict__ arrival) {
-  const long long n = (long long)leaf_count(dN, (unsigned long long)cap);
-  if (n < 2) return;
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    const uint32_t v = tie_member(tieMask, (unsigned long long)i) ? tieVals[i] : vals[i];
-    sortedVals[i] = v;
-    const float2* src = reinterpret_cast<const float2*>(leafBox + (size_t)v * 6);
-    float2* dst = reinterpret_cast<float2*>(sortedBox + (size_t)i * 6);
-    const float2 a = __ldg(src), b = __ldg(src + 1), c = __ldg(src + 2);
-    dst[0] = a;
-    dst[1] = b;
-    dst[2] = c;
-  }
-  if (i >= n - 1) return;
-  arrival[i] = 0u;
-  const unsigned long long ci = karras_code(keys, i);
-  auto delta = [&](long long j) -> int { return __clzll(ci ^ karras_code(keys, j)); };
-  long long d, len;
-  if (i == 0) {
-    d = 1;
-    len = n - 1;
-  } else {
-    int t1 = delta(i - 1), t2 = delta(i + 1);
-    int dmin = min(t1, t2);
-    d = (t2 - t1 >= 0) ? 1 : -1;
-    long long step = 128, j;
-    while ((j = i + d * step) >= 0 && j < n && delta(j) > dmin) step <<= 2;
-    len = 0;
-    for (step >>= 1; step > 0; step >>= 1) {
-      j = i + (len + step) * d;
-      if (j < 0 || j >= n) continue;
-      if (delta(j) > dmin) len += step;
-    }
-  }
-  long long j = i + len * d;
-  int dnode = delta(j);
-  long long step = 1ll << max(0, 31 - __clz((unsigned)len));
-  step >>= (step == len);
-  long long s = 0;
-  for (; step > 0; step >>= 1) {
-    long long k = i + (s + step) * d;
-    if (k < 0 || k >= n) continue;
-    if (delta(k) > dnode) s += step;
-  }
-  long long gamma = i + s * d + min(d, 0ll);
-  long long left = (min(i, j) == gamma) ? gamma : -gamma;
-  long long right = (max(i, j) == gamma + 1) ? (gamma + 1) : -(gamma + 1);
-  nodes[i * 3 + 1] = (int32_t)left;
-  nodes[i * 3 + 2] = (int32_t)right;
-  if (left < 0) nodes[(-left) * 3 + 0] = (int32_t)i;
-  else leafParents[left] = (uint32_t)i;
-  if (right < 0) nodes[(-right) * 3 + 0] = (int32_t)i;
-  else leafParents[right] = (uint32_t)i;
-  if (i == 0) nodes[0] = -1;
-  nodeOther[i] = (int32_t)j;
-}
-
-// Arrival counter bump at GPU scope with only the ordering the step needs.
-// A climber publishes a box through memory only when it comes from an
-// internal node (it stored that node's box itself): release.  A climber that
-// goes on reads its sibling's box through memory only when the sibling is an
-// internal node (stored by another thread): acquire.  Leaf boxes come from an
-// earlier kernel and need neither, so a step between two leaves is relaxed.
-__device__ __forceinline__ uint32_t arrive(uint32_t* p, bool release, bool acquire) {
-  uint32_t old;
-  if (release && acquire)
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-  else if (release)
-    asm volatile("atom.release.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-  else if (acquire)
-    asm volatile("atom.acquire.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-  else
-    asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(p) : "memory");
-  return old;
-}
-
-// The same for a node whose two climbers are threads of one block: the
-// counter and the boxes live in shared memory, ordered at block scope.
-__device__ __forceinline__ uint32_t arrive_block(uint32_t* p) {
-  uint32_t old;
-  asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
-               : "=r"(old)
-               : "r"((uint32_t)__cvta_generic_to_shared(p))
-               : "memory");
-  return old;
+// Common prefix of the codes at positions j - 1 and j: Morton code, then
+// position (`(code << 32) | j`, GPUBVHConstructor.cuh:85).
+__device__ __forceinline__ int boundary_delta(uint32_t c0, uint32_t c1, uint32_t j) {
+  const uint32_t x = c0 ^ c1;
+  return x != 0u ? __clz(x) : 32 + __clz((j - 1u) ^ j);
 }
 
 __device__ __forceinline__ void load_box(const float* p, float mn[3], float mx[3]) {
   const float2* q = reinterpret_cast<const float2*>(p);
-  const float2 a = __ldcg(q), b = __ldcg(q + 1), c = __ldcg(q + 2);
+  const float2 a = q[0], b = q[1], c = q[2];
   mn[0] = a.x; mn[1] = a.y; mn[2] = b.x; mx[0] = b.y; mx[1] = c.x; mx[2] = c.y;
 }
-
-// propagateBVH (GPUBVHConstructor.cuh:215-261): one thread per leaf climbs;
-// the second thread to reach a node merges its children and goes on.  The
-// climber keeps the box of the child it comes from in registers and reads
-// only the sibling's; the union is min/max(left, right) in that order.
-//
-// Two kernels.  In k_refit_local thread j handles sorted leaf j, so a block
-// holds leaves [B, B + 256).  Its threads first stage their leaves' boxes and
-// the records of internal nodes [B, B + 256) (links and the other end of the
-// leaf range) in shared memory: one round of independent, coalesced loads.
-// A node whose leaf range lies inside [B, B + 256) is reached only by threads
-// of the block: its arrival counter and box sit in shared memory (index
-// node - B; a Karras node's index is one end of its range) with block-scope
-// ordering.  A climber that reaches a node whose range crosses the block's
-// boundary (a few percent of the nodes; all their ancestors cross too) stops
-// there and queues the child it comes from.  k_refit_global then carries the
-// queued climbers up through those nodes with arrival counters at GPU scope,
-// so no block of the first kernel waits on a long climb to the root.  Every
-// node's box is also stored to aabbs, the output.  Each leaf's thread also
-// writes the final key of a tie-run member.
-__device__ __forceinline__ void load_box_ldg(const float* __restrict__ p, float mn[3], float mx[3]) {
-  const float2* q = reinterpret_cast<const float2*>(p);
-  const float2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-  mn[0] = a.x; mn[1] = a.y; mn[2] = b.x; mx[0] = b.y; mx[1] = c.x; mx[2] = c.y;
-}
-
 __device__ __forceinline__ void store_box(float* p, const float mn[3], const float mx[3]) {
   float2* o = reinterpret_cast<float2*>(p);
-  __stcg(o + 0, make_float2(mn[0], mn[1]));
-  __stcg(o + 1, make_float2(mn[2], mx[0]));
-  __stcg(o + 2, make_float2(mx[1], mx[2]));
+  o[0] = make_float2(mn[0], mn[1]);
+  o[1] = make_float2(mn[2], mx[0]);
+  o[2] = make_float2(mx[1], mx[2]);
 }
 
-// The union in (left, right) order of the climber's box (mn, mx; from the
-// left child when fromLeft) and its sibling's.
-__device__ __forceinline__ void merge_box(bool fromLeft, float mn[3], float mx[3], const float smn[3],
-                                          const float smx[3]) {
+// A tile's forest in shared memory: leaves in order, delta[e] the common
+// prefix at leaf e's left boundary (delta[count]: at the tile's right end).
+struct Forest {
+  float* box;      // per leaf; an open subtree's box ends up at its first leaf
+  float* nodeBox;  // per joined node, at its right end (left child) or left end
+  uint32_t* flag;  // per boundary (e, e + 1): the far end + 1 of a climber that waits for its sibling
+  const signed char* delta;
+  uint32_t* open;  // bit per leaf: an open subtree starts here
+};
+
+// Climbs with subtree [l, r] (box mn, mx) for at most `steps` joins.  Returns
+// true when it made them all and can go on from the [l, r] it leaves, false
+// when it is done: its sibling's climber goes on, its parent reaches past the
+// forest, or it made the root.  links: parent, left, right of the node with
+// index base + e; leafUp: the parent of leaf base + e.
+__device__ __forceinline__ bool climb(const Forest& f, int& l, int& r, float mn[3], float mx[3],
+                                      int steps, int count, uint32_t base, int32_t* links, uint32_t* leafUp) {
+  for (int step = 0; step < steps; step++) {
+    const bool up = f.delta[r + 1] > f.delta[l];  // [l, r] is its parent's left child
+    const int s = up ? r : l - 1;                 // the parent joins at boundary (s, s + 1)
+    if (s < 0 || s + 1 >= count) {
+      store_box(f.box + l * 6, mn, mx);
+      atomicOr(f.open + (l >> 5), 1u << (l & 31));
+      return false;
+    }
+    uint32_t old;
+    asm volatile("atom.acq_rel.cta.shared::cta.exch.b32 %0, [%1], %2;"
+                 : "=r"(old)
+                 : "r"((uint32_t)__cvta_generic_to_shared(f.flag + s)), "r"((uint32_t)(up ? l : r) + 1u)
+                 : "memory");
+    if (old == 0u) return false;  // the sibling's climber goes on
+    f.flag[s] = 0u;
+    const int far = (int)old - 1;
+    const int sib = up ? s + 1 : s;
+    float smn[3], smx[3];
+    load_box((far == sib ? f.box : f.nodeBox) + sib * 6, smn, smx);
+    const bool leftOne = (up ? l : far) == s, rightOne = (up ? far : r) == s + 1;  // single entries
+    l = up ? l : far;
+    r = up ? far : r;
+    // the union in (left, right) order
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const float lmn = up ? mn[k] : smn[k], rmn = up ? smn[k] : mn[k];
+      const float lmx = up ? mx[k] : smx[k], rmx = up ? smx[k] : mx[k];
+      mn[k] = fminf(lmn, rmn);
+      mx[k] = fmaxf(lmx, rmx);
+    }
+    const int dl = f.delta[l], dr = f.delta[r + 1];
+    const int at = dr > dl ? r : l;
+    store_box(f.nodeBox + at * 6, mn, mx);
+    const int32_t gs = (int32_t)base + s, id = (int32_t)base + at;
+    links[at * 3 + 1] = leftOne ? gs : -gs;
+    links[at * 3 + 2] = rightOne ? gs + 1 : -(gs + 1);
+    *(leftOne ? reinterpret_cast<int32_t*>(leafUp) + s : links + s * 3) = id;
+    *(rightOne ? reinterpret_cast<int32_t*>(leafUp) + s + 1 : links + (s + 1) * 3) = id;
+    if (dl < 0 && dr < 0) {
+      links[0] = -1;
+      return false;
+    }
+  }
+  return true;
+}
+
+// After the climbs: a climber still waiting at boundary (s, s + 1) has a
+// sibling that stayed open, so its subtree ([far, s], or [s + 1, far]) is open
+// too.  The whole block, between barriers.
+__device__ __forceinline__ void open_waiting(const Forest& f, int count) {
+  for (int s = (int)threadIdx.x; s + 1 < count; s += (int)kTile) {
+    const uint32_t w = f.flag[s];
+    if (w == 0u) continue;
+    const int far = (int)w - 1;
+    const int l = far <= s ? far : s + 1;
+    if (far != (far <= s ? s : s + 1)) {  // a joined node: its box to its first entry
+      float mn[3], mx[3];
+      load_box(f.nodeBox + (far <= s ? s : s + 1) * 6, mn, mx);
+      store_box(f.box + l * 6, mn, mx);
+    }
+    atomicOr(f.open + (l >> 5), 1u << (l & 31));
+  }
+}
+
+// Rank of entry e among the open subtrees (bits below e) and their number.
+__device__ __forceinline__ uint32_t open_rank(const uint32_t* open, int e) {
+  uint32_t n = __popc(open[e >> 5] & ((1u << (e & 31)) - 1u));
+  for (int w = 0; w < (e >> 5); w++) n += __popc(open[w]);
+  return n;
+}
+
+// The terminal index at sorted position i (bounded by the leaf count, should a
+// look-back wait of the sort have given up and left old contents).
+__device__ __forceinline__ uint32_t leaf_value(const TreeArgs& a, unsigned long long i, unsigned long long n) {
+  return min(__ldg(a.vals + i), (uint32_t)n - 1u);
+}
+
+// The leaves' final order.  The radix sort orders the keys' top bits
+// [kSortLowBit, 64) only (Morton code and the path hash's top 10 bits) and
+// leaves runs of equal top bits in input order; inside a run the order is by
+// the full path hash, then by terminal index: what a full 64-bit sort with a
+// path tie fix gives.  Most runs are short: a tile's threads see the tile's
+// paths and those of kHalo keys either side in shared memory (window position
+// q is leaf base - kHalo + q), and each member of a run counts the members
+// before it.  A run that reaches past the window is ordered by the whole
+// block (tie_select).
+struct TieWindow {
+  uint64_t path[kTile + 2 * kHalo];
+  uint32_t val[kTile + 2 * kHalo];
+};
+constexpr int kWindowWords = (int)(kTile + 2 * kHalo) / 32;
+
+// The run around window position q: its first and last position.  eq holds a
+// bit per position: equal to the left neighbour (bit 0 of the window clear
+// unless the run goes on to the left of it).
+__device__ __forceinline__ void tie_run(const uint32_t* eq, int q, int& s, int& e) {
+  int w = q >> 5;
+  uint32_t m = ~eq[w] & (0xFFFFFFFFu >> (31 - (q & 31)));
+  while (m == 0u && w > 0) m = ~eq[--w];
+  s = m != 0u ? w * 32 + 31 - __clz(m) : 0;
+  w = (q + 1) >> 5;
+  if (w >= kWindowWords) {
+    e = q;
+    return;
+  }
+  m = ~eq[w] & (0xFFFFFFFFu << ((q + 1) & 31));
+  while (m == 0u && w + 1 < kWindowWords) m = ~eq[++w];
+  e = m != 0u ? w * 32 + __ffs(m) - 2 : kWindowWords * 32 - 1;
+}
+
+// (path, value) number `rank` in order among those of sorted positions
+// [lo, hi): a radix select by the whole block, 8 bits a round from the top
+// (digits: 256 words of shared memory).
+__device__ __noinline__ void tie_select(const TreeArgs& a, unsigned long long n, unsigned long long lo, unsigned long long hi,
+                                        unsigned long long rank, uint32_t* digits, uint64_t& path, uint32_t& val) {
+  __shared__ uint32_t sDigit, sBefore;
+  uint64_t p = 0;
+  uint32_t v = 0;
+  for (int round = 0; round < 12; round++) {
+    for (uint32_t k = threadIdx.x; k < 256u; k += kTile) digits[k] = 0u;
+    __syncthreads();
+    const int shift = round < 8 ? 56 - 8 * round : 24 - 8 * (round - 8);
+    for (unsigned long long i = lo + threadIdx.x; i < hi; i += kTile) {
+      const uint32_t vi = leaf_value(a, i, n);
+      const uint64_t pi = term_path(a.t, vi);
+      if (round < 8) {
+        if (round == 0 || (pi >> (shift + 8)) == (p >> (shift + 8))) atomicAdd(digits + ((pi >> shift) & 255u), 1u);
+      } else if (pi == p && (round == 8 || (vi >> (shift + 8)) == (v >> (shift + 8)))) {
+        atomicAdd(digits + ((vi >> shift) & 255u), 1u);
+      }
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      uint32_t before = 0, d = 0;
+      while (d < 255u && before + digits[d] <= rank) before += digits[d++];
+      sDigit = d;
+      sBefore = before;
+    }
+    __syncthreads();
+    rank -= sBefore;
+    if (round < 8) p |= (uint64_t)sDigit << shift;
+    else v |= sDigit << shift;
+  }
+  path = p;
+  val = v;
+}
+
+__device__ __forceinline__ void gather_leaf(const PgaTerminal* t, uint32_t v, float mn[3], float mx[3],
+                                            uint64_t& path) {
+  const float4* p = reinterpret_cast<const float4*>(t + v);
+  const float4 r[3] = {__ldg(p + 0), __ldg(p + 1), __ldg(p + 2)};
+  const uint4 meta = __ldg(reinterpret_cast<const uint4*>(p + 3));
+  leaf_aabb(r, (meta.x >> 31) != 0, mn, mx);
+  path = ((uint64_t)meta.w << 32) | meta.z;
+}
+
+#ifndef PGA_TREE_BLOCKS
+#define PGA_TREE_BLOCKS 6
+#endif
+__global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  __shared__ __align__(16) float sBox[kTile * 6];
+  // the joined nodes' boxes; before the climb, the window and the final paths
+  __shared__ __align__(16) float sNodeBox[kTile * 6];
+  __shared__ int32_t links[kTile * 3];
+  __shared__ uint32_t leafUp[kTile];
+  __shared__ uint32_t fVal[kTile];
+  __shared__ uint32_t sFlag[kTile];
+  __shared__ uint32_t sQueue[kTile / 2 + kTile / 4];
+  __shared__ signed char sDelta[kTile + 2];
+  __shared__ uint32_t sOpen[kTile / 32];
+  __shared__ uint32_t sEq[kWindowWords];
+  __shared__ int sLong;  // bit 0 / 1: the run at the tile's left / right end reaches past the window
+  __shared__ uint32_t sCount, sQueued[2];
+  TieWindow& win = *reinterpret_cast<TieWindow*>(sNodeBox);
+  uint64_t* fPath = reinterpret_cast<uint64_t*>(sNodeBox + sizeof(TieWindow) / 4);
+  static_assert(sizeof(TieWindow) + kTile * 8 <= kTile * 24, "window and paths in the node boxes' place");
+  const unsigned long long n = leaf_count(a.dN, a.cap);
+  const unsigned long long base = (unsigned long long)blockIdx.x * kTile;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  if (base + tid >= n && base + tid < a.cap) a.outKeys[base + tid] = ~0ull;  // padding past a device count
+  if (n < 2 || base >= n) return;
+  const uint32_t cnt = (uint32_t)min((unsigned long long)kTile, n - base);
+  const bool valid = tid < cnt;
+  const unsigned long long k = base + tid;
+
+  unsigned long long key = 0;
+  uint32_t val = 0;
+  uint64_t path = 0;
+  float mn[3], mx[3];
+  bool eq = false;
+  if (valid) {
+    key = __ldg(a.keys + k);
+    val = leaf_value(a, k, n);
+    int d = -1;
+    if (k > 0) {
+      const unsigned long long before = __ldg(a.keys + k - 1);
+      d = boundary_delta((uint32_t)(before >> 34), (uint32_t)(key >> 34), (uint32_t)k);
+      eq = (before >> kSortLowBit) == (key >> kSortLowBit);
+    }
+    sDelta[tid] = (signed char)d;
+    gather_leaf(a.t, val, mn, mx, path);
+    win.path[kHalo + tid] = path;
+    win.val[kHalo + tid] = val;
+    store_box(sBox + tid * 6, mn, mx);
+    fPath[tid] = path;
+    fVal[tid] = val;
+  }
+  bool eqEnd = false;
+  if (tid == cnt - 1) {  // the tile's right end
+    int d = -1;
+    if (k + 1 < n) {
+      const unsigned long long after = __ldg(a.keys + k + 1);
+      d = boundary_delta((uint32_t)(key >> 34), (uint32_t)(after >> 34), (uint32_t)(k + 1));
+      eqEnd = (after >> kSortLowBit) == (key >> kSortLowBit);  // then cnt == kTile
+    }
+    sDelta[cnt] = (signed char)d;
+  }
+  const unsigned eqs = __ballot_sync(kAll, eq);
+  if (lane == 0) sEq[1 + warp] = eqs;
+  if (tid < kTile / 32) sOpen[tid] = 0u;
+  if (tid == 0) {
+    sEq[0] = 0u;
+    sLong = 0;
+    sQueued[0] = sQueued[1] = 0u;
+  }
+  if (tid == cnt - 1) sEq[kWindowWords - 1] = eqEnd ? 1u : 0u;
+  if (__syncthreads_or(eq || eqEnd)) {
+    // the halo keys that belong to the runs at the tile's ends
+    bool halo = false;
+    int hq = 0;
+    if (warp == 0 && (sEq[1] & 1u)) {
+      const unsigned long long top = __shfl_sync(kAll, key, 0) >> kSortLowBit;
+      const long long i = (long long)base - kHalo + lane;
+      const bool same = i >= 0 && (__ldg(a.keys + max(i, 0ll)) >> kSortLowBit) == top;
+      const int have = __clz((int)~__ballot_sync(kAll, same));  // consecutive ones from lane 31 down
+      halo = (int)lane >= 32 - have;
+      hq = (int)lane;
+      if (lane == 0) {
+        const bool more = have == 32 && base > kHalo && (__ldg(a.keys + base - kHalo - 1) >> kSortLowBit) == top;
+        sEq[0] = (have >= 2 ? kAll << (33 - have) : 0u) | (more ? 1u : 0u);
+        if (more) atomicOr(&sLong, 1);
+      }
+      if (halo) val = leaf_value(a, (unsigned long long)i, n);
+    } else if (warp == 1 && (sEq[kWindowWords - 1] & 1u)) {
+      const unsigned long long top = __ldg(a.keys + base + kTile - 1) >> kSortLowBit;
+      const unsigned long long i = base + kTile + lane;
+      const bool same = i < n && (__ldg(a.keys + min(i, n - 1)) >> kSortLowBit) == top;
+      const unsigned m = __ballot_sync(kAll, same);
+      const int have = m == kAll ? 32 : __ffs((int)~m) - 1;
+      halo = (int)lane < have;
+      hq = (int)(kHalo + kTile + lane);
+      if (lane == 0) {
+        const unsigned long long past = base + kTile + kHalo;
+        const bool more = have == 32 && past < n && (__ldg(a.keys + past) >> kSortLowBit) == top;
+        sEq[kWindowWords - 1] = have == 32 ? kAll : (1u << have) - 1u;
+        if (more) atomicOr(&sLong, 2);
+      }
+      if (halo) val = leaf_value(a, (unsigned long long)i, n);
+    }
+    uint64_t hPath = 0;
+    if (halo) {
+      hPath = term_path(a.t, val);
+      win.path[hq] = hPath;
+      win.val[hq] = val;
+    }
+    __syncthreads();
+    const int isLong = sLong;
+    // this thread's leaf, then (two warps) its halo key
+    for (int turn = 0; turn < 2; turn++) {
+      const int q = turn == 0 ? (int)(kHalo + tid) : hq;
+      if (turn == 0 ? !valid : !halo) continue;
+      const bool left = (sEq[q >> 5] >> (q & 31)) & 1u;
+      const bool right = q + 1 < kWindowWords * 32 && ((sEq[(q + 1) >> 5] >> ((q + 1) & 31)) & 1u);
+      if (!left && !right) continue;
+      int s, e;
+      tie_run(sEq, q, s, e);
+      if ((isLong & 1) && s < (int)kHalo) continue;
+      if ((isLong & 2) && e >= (int)(kHalo + kTile)) continue;
+      const uint64_t p = win.path[q];
+      const uint32_t v = win.val[q];
+      int pos = s - (int)kHalo;
+      for (int x = s; x <= e; x++) {
+        const uint64_t px = win.path[x];
+        pos += (px < p || (px == p && win.val[x] < v)) ? 1 : 0;
+      }
+      if (pos < 0 || pos >= (int)cnt) continue;  // a neighbouring tile's leaf
+      if (turn == 1) {
+        uint64_t again;
+        gather_leaf(a.t, v, mn, mx, again);
+      }
+      store_box(sBox + pos * 6, mn, mx);
+      fPath[pos] = p;
+      fVal[pos] = v;
+    }
+    // runs that reach past the window: the members whose places are in this tile
+    for (int side = 0; side < 2; side++) {
+      if (!(isLong & (1 << side))) continue;
+      __shared__ unsigned long long sRun[2];
+      __syncthreads();
+      const unsigned long long end = side == 0 ? base : base + cnt - 1;
+      if (tid == 0) {
+        const unsigned long long top = a.keys[end] >> kSortLowBit;
+        unsigned long long lo = 0, hi = end;  // first position with these top bits
+        while (lo < hi) {
+          const unsigned long long mid = (lo + hi) >> 1;
+          if ((a.keys[mid] >> kSortLowBit) < top) lo = mid + 1;
+          else hi = mid;
+        }
+        sRun[0] = lo;
+        lo = end + 1;
+        hi = n;  // first position past them
+        while (lo < hi) {
+          const unsigned long long mid = (lo + hi) >> 1;
+          if ((a.keys[mid] >> kSortLowBit) <= top) lo = mid + 1;
+          else hi = mid;
+        }
+        sRun[1] = lo;
+        sCount = 0u;
+      }
+      __syncthreads();
+      const unsigned long long lo = sRun[0], hi = sRun[1];
+      const unsigned long long first = max(lo, base), last = min(hi, base + cnt) - 1;
+      uint64_t p0, p1;
+      uint32_t v0, v1;
+      tie_select(a, n, lo, hi, first - lo, sFlag, p0, v0);
+      tie_select(a, n, lo, hi, last - lo, sFlag, p1, v1);
+      for (unsigned long long i = lo + tid; i < hi; i += kTile) {
+        const uint32_t v = leaf_value(a, i, n);
+        const uint64_t p = term_path(a.t, v);
+        if (p < p0 || (p == p0 && v < v0) || p > p1 || (p == p1 && v > v1)) continue;
+        const uint32_t at = atomicAdd(&sCount, 1u);
+        if (at > last - first) continue;  // never: the selects bound the members by their ranks
+        win.path[at] = p;
+        win.val[at] = v;
+      }
+      __syncthreads();
+      const int m = (int)min((unsigned long long)sCount, last - first + 1);
+      if ((int)tid < m) {
+        const uint64_t p = win.path[tid];
+        const uint32_t v = win.val[tid];
+        uint32_t pos = (uint32_t)(first - base);  // at most first - base + m - 1 after the loop
+        for (int x = 0; x < m; x++) pos += (win.path[x] < p || (win.path[x] == p && win.val[x] < v)) ? 1u : 0u;
+        uint64_t again;
+        gather_leaf(a.t, v, mn, mx, again);
+        store_box(sBox + pos * 6, mn, mx);
+        fPath[pos] = p;
+        fVal[pos] = v;
+      }
+      __syncthreads();
+      if (isLong == 3 && hi >= base + cnt) break;  // one run over the whole tile
+    }
+    __syncthreads();
+  }
+  const Forest f{sBox, sNodeBox, sFlag, sDelta, sOpen};
+  if (valid) {
+    a.leafTerminal[k] = fVal[tid];
+    a.outKeys[k] = ((key >> 34) << 34) | (fPath[tid] >> 30);
+    load_box(sBox + tid * 6, mn, mx);
+  }
+  __syncthreads();  // the node boxes take the window's place
+  // First the leaves that are each other's sibling: joined by the left one's
+  // thread.  Any other leaf waits at its boundary or, at the tile's ends, stays
+  // open; no two climbers meet in this step, so it needs no exchange.
+  int l = (int)tid, r = (int)tid;
+  bool on = false;
+  if (valid) {
+    const bool up = sDelta[tid + 1] > sDelta[tid];
+    const bool inside = tid + 1 < cnt;
+    const bool nextDown = inside && !(sDelta[tid + 2] > sDelta[tid + 1]);
+    uint32_t wait = 0;  // at boundary (tid, tid + 1)
+    if (inside && up && !nextDown) wait = tid + 1;
+    if (inside && !up && nextDown) wait = tid + 2;
+    sFlag[tid] = wait;
+    if ((up && !inside) || (!up && tid == 0)) atomicOr(&sOpen[tid >> 5], 1u << lane);
+    on = up && nextDown;
+  }
+  if (on) {
+    float smn[3], smx[3];
+    load_box(sBox + (tid + 1) * 6, smn, smx);
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      mn[q] = fminf(mn[q], smn[q]);
+      mx[q] = fmaxf(mx[q], smx[q]);
+    }
+    const int dl = sDelta[tid], dr = sDelta[tid + 2];
+    const int at = (int)tid + (dr > dl ? 1 : 0);
+    store_box(sNodeBox + at * 6, mn, mx);
+    links[at * 3 + 1] = (int32_t)k;
+    links[at * 3 + 2] = (int32_t)k + 1;
+    leafUp[tid] = leafUp[tid + 1] = (uint32_t)base + (uint32_t)at;
+    if (dl < 0 && dr < 0) {  // two leaves in all
+      links[0] = -1;
+      on = false;
+    }
+  }
+  // Then the climb, in rounds: every join ends one of two climbers, so the
+  // lanes left are few and far apart; they are packed into the first warps
+  // before they go on.
+  for (int round = 0; round < 2; round++) {
+    const unsigned going = __ballot_sync(kAll, on);
+    uint32_t at = 0;
+    if (lane == 0 && going) at = atomicAdd(&sQueued[round], (uint32_t)__popc(going));
+    at = __shfl_sync(kAll, at, 0) + __popc(going & ((1u << lane) - 1u));
+    uint32_t* queue = sQueue + (round == 0 ? 0 : kTile / 2);  // subtrees of two leaves or more, then of four
+    if (on) queue[at] = (uint32_t)l | ((uint32_t)(round == 0 ? l + 1 : r) << 16);
+    __syncthreads();
+    on = tid < sQueued[round];
+    if (on) {
+      const uint32_t w = queue[tid];
+      l = (int)(w & 0xFFFFu);
+      r = (int)(w >> 16);
+      load_box(sNodeBox + (sDelta[r + 1] > sDelta[l] ? r : l) * 6, mn, mx);
+      on = climb(f, l, r, mn, mx, round == 0 ? 2 : (int)cnt, (int)cnt, (uint32_t)base, links, leafUp);
+    }
+  }
+  __syncthreads();
+  open_waiting(f, (int)cnt);
+  // Out, coalesced.  Open subtrees' parents and the nodes that cross the
+  // tile's ends have no value yet: what goes out for them is written again by
+  // the join that makes them, after this tile has arrived.
+  const uint32_t inner = (uint32_t)min((unsigned long long)cnt, n - 1 - base);
+  if (valid) a.leafParents[k] = leafUp[tid];
+  for (uint32_t w = tid; w < inner * 3; w += kTile) a.nodes[base * 3 + w] = links[w];
+  {
+    float2* dst = reinterpret_cast<float2*>(a.aabbs + base * 6);
+    const float2* src = reinterpret_cast<const float2*>(sNodeBox);
+    for (uint32_t w = tid; w < inner * 3; w += kTile) dst[w] = src[w];
+  }
+  if (n <= kTile) return;
+  __syncthreads();
+  // The open subtrees, in leaf order, for k_join.
+  const unsigned long long slot = blockIdx.x;
+  if (valid && ((sOpen[tid >> 5] >> lane) & 1u)) {
+    const uint32_t at = open_rank(sOpen, (int)tid);
+    load_box(sBox + tid * 6, mn, mx);
+    if (at < kMaxOpen) {
+      float4* o = reinterpret_cast<float4*>(a.open + slot * kMaxOpen + at);
+      o[0] = make_float4(mn[0], mn[1], mn[2], mx[0]);
+      o[1] = make_float4(mx[1], mx[2], __uint_as_float((uint32_t)k), __int_as_float(sDelta[tid]));
+    }
+  }
+  if (tid == 0) {
+    uint32_t m = 0;
+    for (uint32_t w = 0; w < kTile / 32; w++) m += __popc(sOpen[w]);
+    a.openCount[slot] = min(m, kMaxOpen);
+  }
+}
+
+// Joins the open subtrees of kGroup tiles a block, publishes what is still
+// open, and the last of kGroup blocks to do so goes on with their group.  A
+// kernel of its own: in k_tree's blocks the fence and the arrival held a
+// tile's place on its SM for a quarter of its time (city of 5.9M leaves: 98 of
+// 363 us).
+//
+// Open subtrees of neighbouring tiles join one after another, so a climb
+// through them is 30 dependent steps long (city: 64 us, 20,011 leaves: 20 us
+// for its two levels).  Here every join of a group is found on its own: the
+// node at boundary c (before entry c) spans the entries up to the nearest
+// smaller prefix on either side, found by descending a table of range minima,
+// and its box comes from prefix and suffix boxes of 32-entry runs: 47 and 14 us.
+constexpr int kJoinLevels = 10;             // range minima of 2^k boundaries, k < kJoinLevels
+
+__device__ __forceinline__ void grow_box(float mn[3], float mx[3], const float* p) {
+  float a[3], b[3];
+  load_box(p, a, b);
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    const float lmn = fromLeft ? mn[k] : smn[k], rmn = fromLeft ? smn[k] : mn[k];
-    const float lmx = fromLeft ? mx[k] : smx[k], rmx = fromLeft ? smx[k] : mx[k];
-    mn[k] = fminf(lmn, rmn);
-    mx[k] = fmaxf(lmx, rmx);
+    mn[k] = fminf(mn[k], a[k]);
+    mx[k] = fmaxf(mx[k], b[k]);
   }
 }
 
-__global__ void __launch_bounds__(kLbvhThreads) k_refit_local(const float* __restrict__ sortedBox, long long cap,
-                                                              const unsigned long long* __restrict__ dN,
-                                                              const int32_t* __restrict__ nodes,
-                                                              const int32_t* __restrict__ nodeOther,
-                                                              const uint32_t* __restrict__ leafParents,
-                                                              float* __restrict__ aabbs,
-                                                              int32_t* __restrict__ queue, uint32_t* __restrict__ queued,
-                                                              const uint32_t* __restrict__ tieMask,
-                                                              const unsigned long long* __restrict__ tieKeys,
-                                                              unsigned long long* __restrict__ keys) {
-  __shared__ uint32_t blockArrive[kLbvhThreads];
-  __shared__ float blockBox[kLbvhThreads * 6];  // internal nodes [B, E)
-  __shared__ float sLeafBox[kLbvhThreads * 6];  // leaves [B, E)
-  __shared__ int4 sNode[kLbvhThreads];          // internal nodes [B, E): parent, left, right, other end
-  const long long n = (long long)leaf_count(dN, (unsigned long long)cap);
-  if (n < 2) return;
-  const long long B = (long long)blockIdx.x * kLbvhThreads;
-  if (B >= n) return;  // the whole block
-  const long long E = min(B + kLbvhThreads, n);
-  const long long leaf = B + threadIdx.x;
-  blockArrive[threadIdx.x] = 0u;
-  float mn[3], mx[3];
-  long long cur = -1;
-  if (leaf < n) {
-    if (tie_member(tieMask, (unsigned long long)leaf)) keys[leaf] = tieKeys[leaf];
-    load_box_ldg(sortedBox + (size_t)leaf * 6, mn, mx);
-    float* q = &sLeafBox[threadIdx.x * 6];
-    q[0] = mn[0]; q[1] = mn[1]; q[2] = mn[2]; q[3] = mx[0]; q[4] = mx[1]; q[5] = mx[2];
-    cur = __ldg(leafParents + leaf);
-  }
-  if (leaf < n - 1)
-    sNode[threadIdx.x] = make_int4(__ldg(nodes + leaf * 3 + 0), __ldg(nodes + leaf * 3 + 1),
-                                   __ldg(nodes + leaf * 3 + 2), __ldg(nodeOther + leaf));
-  __syncthreads();
-  if (leaf >= n) return;
-  int32_t from = (int32_t)leaf;  // child id as the node table stores it: leaf j -> j, internal k -> -k
-  for (int level = 0; level < kLbvhThreads; level++) {
-    bool local = cur >= B && cur < E;
-    int4 rec = make_int4(0, 0, 0, 0);
-    if (local) {
-      rec = sNode[cur - B];
-      local = min(cur, (long long)rec.w) >= B && max(cur, (long long)rec.w) < E;
+__global__ void __launch_bounds__(kTile) k_join(TreeArgs a) {
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  constexpr uint32_t kPer = kJoin / kTile;  // boundaries per thread
+  __shared__ __align__(16) float sBox[kJoin * 6];
+  __shared__ __align__(16) float sBefore[kJoin * 6];  // from the run's first entry to this one
+  __shared__ __align__(16) float sAfter[kJoin * 6];   // from this entry to the run's last
+  __shared__ uint32_t sLeft[kJoin + 1];
+  __shared__ signed char sMin[kJoinLevels][kJoin + 1];  // [0]: the prefix at each entry's left boundary
+  __shared__ uint32_t sClosed[kJoin / 32];              // bit c: the node at boundary c lies in the group
+  __shared__ uint32_t sOpen[kJoin / 32];                // bit e: an open subtree starts at entry e
+  __shared__ uint32_t sAt[kGroup];
+  __shared__ uint32_t sCount, sTaken, sLast;
+  signed char* delta = sMin[0];
+  const unsigned long long n = leaf_count(a.dN, a.cap);
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+  if (n <= (unsigned long long)blockIdx.x * kGroup * kTile || n <= kTile) return;
+  unsigned long long items = (n + kTile - 1) / kTile;  // tiles, then groups of the level being joined
+  unsigned long long g = blockIdx.x, stride = 1;       // the group, and the tiles per item of this level
+  uint32_t* joins = a.joins;
+  for (;;) {
+    const unsigned long long first = g * kGroup;
+    const uint32_t size = (uint32_t)min((unsigned long long)kGroup, items - first);
+    // The group's open subtrees, as many slots at a time as fit (always
+    // several: what stays open of those joined so far is at most kMaxOpen).
+    uint32_t carry = 0, next = 0;
+    bool whole = false;
+    while (!whole) {
+      if (warp == 0) {
+        const uint32_t j = next + lane;
+        const uint32_t c = j < size ? __ldcg(a.openCount + (first + j) * stride) : 0u;
+        uint32_t x = c;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const uint32_t y = __shfl_up_sync(kAll, x, d);
+          if (lane >= (uint32_t)d) x += y;
+        }
+        const unsigned fits = __ballot_sync(kAll, j < size && carry + x <= kJoin);  // a prefix of the lanes
+        const uint32_t take = __popc(fits);
+        sAt[lane] = carry + x - c;  // where slot j's entries go
+        if (lane == take - 1u) sCount = carry + x;
+        if (lane == 0) sTaken = take;
+      }
+      if (tid < kJoin / 32) sClosed[tid] = sOpen[tid] = 0u;
+      __syncthreads();
+      const uint32_t take = sTaken, count = sCount;
+      // slots four at a time per warp, eight lanes to a slot
+      for (uint32_t j = warp * 4 + (lane >> 3); j < take; j += kTile / 8) {
+        const unsigned long long at = (first + next + j) * stride;
+        const uint32_t to = sAt[j], c = (j + 1 < take ? sAt[j + 1] : count) - to;
+        for (uint32_t x = lane & 7u; x < c; x += 8) {
+          const float4* o = reinterpret_cast<const float4*>(a.open + at * kMaxOpen + x);
+          const float4 p = __ldcg(o), q = __ldcg(o + 1);
+          float* b = sBox + (to + x) * 6;
+          b[0] = p.x; b[1] = p.y; b[2] = p.z; b[3] = p.w; b[4] = q.x; b[5] = q.y;
+          sLeft[to + x] = __float_as_uint(q.z);
+          delta[to + x] = (signed char)__float_as_int(q.w);
+        }
+      }
+      next += take;
+      whole = next >= size;
+      if (tid == 0) {
+        const unsigned long long end = min(n, (first + next) * stride * kTile);
+        sLeft[count] = (uint32_t)end;
+        delta[count] = (signed char)(end < n ? boundary_delta((uint32_t)(__ldg(a.keys + end - 1) >> 34),
+                                                              (uint32_t)(__ldg(a.keys + end) >> 34), (uint32_t)end)
+                                             : -1);
+      }
+      __syncthreads();
+      // prefix and suffix boxes of the runs (a warp per run)
+      for (uint32_t run = warp; run * 32 < count; run += kTile / 32) {
+        const uint32_t e = run * 32 + lane;
+        float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
+        if (e < count) load_box(sBox + e * 6, mn, mx);
+        float pn[3] = {mn[0], mn[1], mn[2]}, px[3] = {mx[0], mx[1], mx[2]};
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+#pragma unroll
+          for (int k = 0; k < 3; k++) {
+            const float un = __shfl_up_sync(kAll, pn[k], d), ux = __shfl_up_sync(kAll, px[k], d);
+            const float dn = __shfl_down_sync(kAll, mn[k], d), dx = __shfl_down_sync(kAll, mx[k], d);
+            // (a lane past the end gets its own value back)
+            pn[k] = fminf(un, pn[k]);
+            px[k] = fmaxf(ux, px[k]);
+            mn[k] = fminf(mn[k], dn);
+            mx[k] = fmaxf(mx[k], dx);
+          }
+        }
+        if (e < count) {
+          store_box(sBefore + e * 6, pn, px);
+          store_box(sAfter + e * 6, mn, mx);
+        }
+      }
+      // range minima: sMin[k][c] over boundaries [c, c + 2^k)
+#pragma unroll
+      for (int k = 1; k < kJoinLevels; k++) {
+        const int half = 1 << (k - 1);
+        for (int c = (int)tid; c + 2 * half <= (int)count + 1; c += (int)kTile)
+          sMin[k][c] = min(sMin[k - 1][c], sMin[k - 1][c + half]);
+        __syncthreads();
+      }
+      float mn[kPer][3], mx[kPer][3];
+      int from[kPer], to[kPer];  // the entries of the node at boundary c; from < 0: it reaches past the group
+#pragma unroll
+      for (uint32_t u = 0; u < kPer; u++) {
+        const int c = (int)(u * kTile + tid);
+        from[u] = -1;
+        to[u] = -1;
+        if (c == 0 || c >= (int)count) continue;
+        const int v = delta[c];
+        int p = c, q = c + 1;  // [p, c) and [c + 1, q) hold no smaller prefix
+#pragma unroll
+        for (int k = kJoinLevels - 1; k >= 0; k--) {
+          const int w = 1 << k;
+          if (p >= w && sMin[k][p - w] >= v) p -= w;
+          if (q + w <= (int)count + 1 && sMin[k][q] >= v) q += w;
+        }
+        if (p == 0 || q > (int)count) continue;
+        const int l = p - 1, r = q - 1;
+        from[u] = l;
+        to[u] = r;
+        atomicOr(&sClosed[c >> 5], 1u << (c & 31));
+        load_box(sAfter + l * 6, mn[u], mx[u]);
+        if ((l >> 5) == (r >> 5)) {
+          load_box(sBox + l * 6, mn[u], mx[u]);
+          for (int x = l + 1; x <= r; x++) grow_box(mn[u], mx[u], sBox + x * 6);
+        } else {
+          for (int x = (l >> 5) + 1; x < (r >> 5); x++) grow_box(mn[u], mx[u], sAfter + x * 32 * 6);
+          grow_box(mn[u], mx[u], sBefore + r * 6);
+        }
+        const bool left = delta[r + 1] > delta[l];  // a left child: its index is its right end
+        const int32_t gl = (int32_t)sLeft[l], gr = (int32_t)sLeft[r + 1] - 1, gs = (int32_t)sLeft[c] - 1;
+        const int32_t id = left ? gr : gl;
+        a.nodes[(size_t)id * 3 + 1] = gl == gs ? gs : -gs;
+        a.nodes[(size_t)id * 3 + 2] = gs + 1 == gr ? gr : -(gs + 1);
+        *(gl == gs ? reinterpret_cast<int32_t*>(a.leafParents) + gs : a.nodes + (size_t)gs * 3) = id;
+        *(gs + 1 == gr ? reinterpret_cast<int32_t*>(a.leafParents) + gr : a.nodes + (size_t)(gs + 1) * 3) = id;
+        store_box(a.aabbs + (size_t)id * 6, mn[u], mx[u]);
+        if (delta[l] < 0 && delta[r + 1] < 0) a.nodes[0] = -1;
+      }
+      __syncthreads();
+      // A subtree (an entry, or a node made here) is open when its parent, at
+      // the boundary of its larger prefix, is not in the group.
+#pragma unroll
+      for (uint32_t u = 0; u < kPer; u++) {
+        const int e = (int)(u * kTile + tid);
+        if (e < (int)count) {
+          const int c = delta[e + 1] > delta[e] ? e + 1 : e;
+          if (c >= (int)count || !((sClosed[c >> 5] >> (c & 31)) & 1u)) atomicOr(&sOpen[e >> 5], 1u << (e & 31));
+        }
+        if (from[u] >= 0) {
+          const int l = from[u], r = to[u];
+          const int c = delta[r + 1] > delta[l] ? r + 1 : l;
+          const bool root = delta[l] < 0 && delta[r + 1] < 0;
+          if (!root && (c >= (int)count || !((sClosed[c >> 5] >> (c & 31)) & 1u))) {
+            store_box(sBox + l * 6, mn[u], mx[u]);
+            atomicOr(&sOpen[l >> 5], 1u << (l & 31));
+          }
+        }
+      }
+      __syncthreads();
+      // The subtrees still open, in order: to the front of the forest for the
+      // next slots, or out to the group's place (its first tile's).
+      uint32_t keepAt[kPer], keepLeft[kPer];
+      int keepDelta[kPer];
+#pragma unroll
+      for (uint32_t u = 0; u < kPer; u++) {
+        const uint32_t x = u * kTile + tid;
+        keepAt[u] = kJoin;
+        if (x < count && ((sOpen[x >> 5] >> (x & 31u)) & 1u)) {
+          keepAt[u] = open_rank(sOpen, (int)x);
+          keepLeft[u] = sLeft[x];
+          keepDelta[u] = delta[x];
+          load_box(sBox + x * 6, mn[u], mx[u]);
+        }
+      }
+      carry = 0;
+      for (uint32_t w = 0; w < kJoin / 32; w++) carry += __popc(sOpen[w]);
+      carry = min(carry, kMaxOpen);
+      __syncthreads();
+#pragma unroll
+      for (uint32_t u = 0; u < kPer; u++) {
+        if (keepAt[u] >= kMaxOpen) continue;
+        if (whole) {
+          float4* o = reinterpret_cast<float4*>(a.open + first * stride * kMaxOpen + keepAt[u]);
+          __stcg(o, make_float4(mn[u][0], mn[u][1], mn[u][2], mx[u][0]));
+          __stcg(o + 1, make_float4(mx[u][1], mx[u][2], __uint_as_float(keepLeft[u]), __int_as_float(keepDelta[u])));
+        } else {
+          sLeft[keepAt[u]] = keepLeft[u];
+          delta[keepAt[u]] = (signed char)keepDelta[u];
+          store_box(sBox + keepAt[u] * 6, mn[u], mx[u]);
+        }
+      }
+      __syncthreads();
     }
-    if (!local) {  // the node's range crosses the block's boundary: k_refit_global goes on from here
-      queue[atomicAdd(queued, 1u)] = from;
-      return;
+    const unsigned long long groups = (items + kGroup - 1) / kGroup;
+    if (groups == 1) return;
+    if (tid == 0) __stcg(a.openCount + first * stride, carry);
+    items = groups;
+    stride *= kGroup;
+    const uint32_t peers = (uint32_t)min((unsigned long long)kGroup, items - g / kGroup * kGroup);
+    __syncthreads();
+    if (tid == 0) {
+      __threadfence();  // the block's stores, ordered before it by the barrier, before its arrival
+      sLast = atomicAdd(joins + g / kGroup, 1u) == peers - 1u ? 1u : 0u;
+      __threadfence();
     }
-    if (arrive_block(&blockArrive[cur - B]) == 0) return;
-    const bool fromLeft = rec.y == from;
-    const int32_t sib = fromLeft ? rec.z : rec.y;  // inside [B, E): the node is local
-    const float* q = sib >= 0 ? &sLeafBox[(sib - B) * 6] : &blockBox[(-(long long)sib - B) * 6];
-    const float smn[3] = {q[0], q[1], q[2]}, smx[3] = {q[3], q[4], q[5]};
-    merge_box(fromLeft, mn, mx, smn, smx);
-    store_box(aabbs + (size_t)cur * 6, mn, mx);
-    float* o = &blockBox[(cur - B) * 6];
-    o[0] = mn[0]; o[1] = mn[1]; o[2] = mn[2]; o[3] = mx[0]; o[4] = mx[1]; o[5] = mx[2];
-    if (cur == 0) return;
-    from = -(int32_t)cur;
-    cur = rec.x;
-  }
-}
-
-// The queued climbers (*queued of them, each the child it comes from) up
-// through the nodes that cross block boundaries: arrival counters at GPU
-// scope, the boxes of the children the first kernel finished read from
-// aabbs / sortedBox (written before this launch), those of this kernel with
-// release / acquire on the counter.  Grid-stride over the queue.
-__global__ void __launch_bounds__(kLbvhThreads) k_refit_global(const float* __restrict__ sortedBox, long long cap,
-                                                               const unsigned long long* __restrict__ dN,
-                                                               const int32_t* __restrict__ nodes,
-                                                               const uint32_t* __restrict__ leafParents,
-                                                               uint32_t* __restrict__ arrival, float* aabbs,
-                                                               const int32_t* __restrict__ queue,
-                                                               const uint32_t* __restrict__ queued) {
-  const long long n = (long long)leaf_count(dN, (unsigned long long)cap);
-  if (n < 2) return;
-  const uint32_t count = *queued;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
-    int32_t from = queue[k];
-    float mn[3], mx[3];
-    long long cur;
-    if (from >= 0) {
-      load_box_ldg(sortedBox + (size_t)from * 6, mn, mx);
-      cur = leafParents[from];
-    } else {
-      load_box(aabbs + (size_t)(-(long long)from) * 6, mn, mx);
-      cur = nodes[(size_t)(-(long long)from) * 3 + 0];
-    }
-    bool published = false;  // the climber's box was stored by this kernel
-    for (long long guard = 0; guard < n && cur >= 0; guard++) {
-      const int32_t parent = __ldg(nodes + cur * 3 + 0), l = __ldg(nodes + cur * 3 + 1), r = __ldg(nodes + cur * 3 + 2);
-      const bool fromLeft = l == from;
-      const int32_t sib = fromLeft ? r : l;
-      float smn[3], smx[3];
-      if (sib >= 0) load_box_ldg(sortedBox + (size_t)sib * 6, smn, smx);
-      if (arrive(&arrival[cur], published, sib < 0) == 0) break;
-      if (sib < 0) load_box(aabbs + (size_t)(-(long long)sib) * 6, smn, smx);
-      merge_box(fromLeft, mn, mx, smn, smx);
-      store_box(aabbs + (size_t)cur * 6, mn, mx);
-      published = true;
-      if (cur == 0) break;
-      from = -(int32_t)cur;
-      cur = parent;
-    }
+    __syncthreads();
+    if (!sLast) return;
+    g /= kGroup;
+    joins += (items + kGroup - 1) / kGroup;
   }
 }
 
@@ -770,29 +1171,42 @@ __global__ void __launch_bounds__(kLbvhThreads) k_refit_global(const float* __re
 
 using namespace pga;
 
-// Sort scratch: the digit histograms, the passes' tile counters and look-back
-// words (zeroed by one memset per build), then the digit bases.
+// Sort scratch: the digit histograms, the passes' tile counters, the tree's
+// arrival counters and the look-back words (zeroed by one memset per build),
+// then the digit bases.
 static unsigned long long sort_tiles(unsigned long long n) { return (n + kSortTile - 1) / kSortTile; }
+static unsigned long long tree_tiles(unsigned long long n) { return (n + kTile - 1) / kTile; }
+static unsigned long long tree_joins(unsigned long long n) {
+  unsigned long long sum = 0;
+  for (unsigned long long items = tree_tiles(n); items > 1;) {
+    items = (items + kGroup - 1) / kGroup;
+    sum += items;
+  }
+  return (sum + 1) & ~1ull;  // the look-back words after them are 8 bytes wide
+}
 
 extern "C" size_t pga_lbvh_temp_bytes(uint64_t n) {
-  const unsigned long long tiles = sort_tiles(n ? n : 1);
-  return (size_t)(kSortPasses * kBins + 64 + (unsigned long long)kSortPasses * tiles * kBins + kSortPasses * kBins) *
+  n = n ? n : 1;
+  return (size_t)(kSortPasses * kBins + 64 + tree_joins(n) + (unsigned long long)kSortPasses * sort_tiles(n) * kBins +
+                  kSortPasses * kBins) *
          sizeof(uint32_t);
+}
+
+// The tiles' open subtrees, then their counts.
+extern "C" size_t pga_lbvh_open_bytes(uint64_t n) {
+  return (size_t)tree_tiles(n ? n : 1) * (kMaxOpen * sizeof(OpenTree) + sizeof(uint32_t));
 }
 
 namespace pga {
 
-// Scratch of one build: keys, two value arrays, arrival counters, leaf boxes
-// (terminal and sorted order), the other ends of the node ranges, the radix sort's
-// scratch, and the word a sort wait that gives up raises PGA_ERR_TIMEOUT in.
+// Scratch of one build: keys, two value arrays, the tiles' open subtrees, the
+// radix sort's scratch, and the word a sort wait that gives up raises
+// PGA_ERR_TIMEOUT in.
 struct LbvhScratch {
   unsigned long long* keysA;
   uint32_t* valsA;
   uint32_t* valsB;
-  uint32_t* arrival;
-  float* leafBox;
-  float* sortedBox;
-  int32_t* nodeOther;
+  void* open;
   void* sortTemp;
   size_t sortTempBytes;
   int* err;
@@ -803,9 +1217,9 @@ constexpr uint32_t kSortSpinLimit = 1u << 22;
 
 // The launches of a build over `cap` leaves, or over min(*dN, cap) when dN is
 // a device count (then `cap` sizes the grids and the sort): Morton codes, the
-// digit histograms and bases, four sort passes (keys ping-pong
-// between out->keys and keysA, ending in out->keys), the tie-run ranks,
-// Karras and the two refit kernels.
+// digit histograms and bases, four sort passes (keys ping-pong between keysA
+// and out->keys, ending in keysA) and the tree, which writes the final keys
+// to out->keys.
 static PgaStatus launch_lbvh(const PgaTerminal* t, unsigned long long cap, const unsigned long long* dN,
                              const PgaBounds* bounds, const PgaLbvh* out, const LbvhScratch& w, cudaStream_t s) {
   Bounds b;
@@ -820,27 +1234,28 @@ static PgaStatus launch_lbvh(const PgaTerminal* t, unsigned long long cap, const
   }
   uint32_t* hist = static_cast<uint32_t*>(w.sortTemp);
   uint32_t* counters = hist + kSortPasses * kBins;
-  uint32_t* status = counters + 64;
+  uint32_t* joins = counters + 64;
+  uint32_t* status = joins + tree_joins(cap);
   uint32_t* gBase = status + (size_t)kSortPasses * tiles * kBins;
   PGA_CUDA_TRY(cudaMemsetAsync(hist, 0, (size_t)(gBase - hist) * sizeof(uint32_t), s));
   int dev = 0, sms = 0;
   PGA_CUDA_TRY(cudaGetDevice(&dev));
   PGA_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const unsigned blocks = (unsigned)((cap + kLbvhThreads - 1) / kLbvhThreads);
-  unsigned long long* keys = (unsigned long long*)out->keys;
-  k_morton<<<blocks, kLbvhThreads, 0, s>>>(t, cap, dN, b, keys, w.leafBox);
+  unsigned long long* outKeys = (unsigned long long*)out->keys;
+  k_morton<<<blocks, kLbvhThreads, 0, s>>>(t, cap, dN, b, w.keysA);
   PGA_CUDA_TRY(cudaGetLastError());
   const unsigned histBlocks =
       (unsigned)std::min<unsigned long long>((cap + kHistThreads - 1) / kHistThreads, (unsigned long long)sms * 4);
-  k_digit_hist<<<histBlocks, kHistThreads, 0, s>>>(keys, cap, hist);
+  k_digit_hist<<<histBlocks, kHistThreads, 0, s>>>(w.keysA, cap, hist);
   PGA_CUDA_TRY(cudaGetLastError());
   k_sort_bases<<<1, kBins, 0, s>>>(hist, gBase);
   PGA_CUDA_TRY(cudaGetLastError());
   PGA_CUDA_TRY(cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOnesweepSmem));
   // The first pass reads the identity values (terminal index); the values
   // then ping-pong valsB -> valsA -> valsB -> valsA.
-  unsigned long long* kIn = keys;
-  unsigned long long* kOut = w.keysA;
+  unsigned long long* kIn = w.keysA;
+  unsigned long long* kOut = outKeys;
   uint32_t* vIn = nullptr;
   uint32_t* vOut = w.valsB;
   unsigned long long* words = reinterpret_cast<unsigned long long*>(status);
@@ -853,34 +1268,23 @@ static PgaStatus launch_lbvh(const PgaTerminal* t, unsigned long long cap, const
     vIn = vOut;
     vOut = vOut == w.valsB ? w.valsA : w.valsB;
   }
-  static_assert(kSortPasses % 2 == 0, "an even number of passes ends in out->keys and valsA");
-  // The tie runs' order goes to keysA / valsB (free after the sort), the
-  // member bits over the look-back words (free too; tiles * kBins * passes
-  // words >= cap / 32).
-  uint32_t* tieMask = status;
-  k_tie_rank<<<blocks, kLbvhThreads, 0, s>>>(keys, w.valsA, t, cap, dN, w.keysA, w.valsB, tieMask);
+  static_assert(kSortPasses % 2 == 0, "an even number of passes ends in keysA and valsA");
+  OpenTree* open = static_cast<OpenTree*>(w.open);
+  const TreeArgs a{w.keysA,    w.valsA,           t,       cap,  dN, out->nodes, out->leafParents, out->aabbs,
+                   out->leafTerminal, outKeys, open, reinterpret_cast<uint32_t*>(open + (size_t)blocks * kMaxOpen),
+                   joins};
+  k_tree<<<blocks, kTile, 0, s>>>(a);
   PGA_CUDA_TRY(cudaGetLastError());
-  k_karras<<<blocks, kLbvhThreads, 0, s>>>(keys, (long long)cap, dN, out->nodes, out->leafParents, out->leafTerminal,
-                                           w.valsA, tieMask, w.valsB, w.leafBox, w.sortedBox, w.nodeOther, w.arrival);
-  PGA_CUDA_TRY(cudaGetLastError());
-  // The refit's queue of climbers that leave their block goes to valsB (free
-  // after Karras), its length to the sort scratch's counter word kSortPasses.
-  uint32_t* queued = counters + kSortPasses;
-  k_refit_local<<<blocks, kLbvhThreads, 0, s>>>(w.sortedBox, (long long)cap, dN, out->nodes, w.nodeOther,
-                                                out->leafParents, out->aabbs, reinterpret_cast<int32_t*>(w.valsB),
-                                                queued, tieMask, w.keysA, keys);
-  PGA_CUDA_TRY(cudaGetLastError());
-  const unsigned globalBlocks = std::min<unsigned>(blocks, (unsigned)sms * (2048 / kLbvhThreads));
-  k_refit_global<<<globalBlocks, kLbvhThreads, 0, s>>>(w.sortedBox, (long long)cap, dN, out->nodes,
-                                                       out->leafParents, w.arrival, out->aabbs,
-                                                       reinterpret_cast<const int32_t*>(w.valsB), queued);
-  PGA_CUDA_TRY(cudaGetLastError());
+  if (blocks > 1) {
+    k_join<<<(blocks + kGroup - 1) / kGroup, kTile, 0, s>>>(a);
+    PGA_CUDA_TRY(cudaGetLastError());
+  }
   return PGA_OK;
 }
 
 static LbvhScratch engine_scratch(PgaEngine* e) {
-  return LbvhScratch{e->dKeysA,     e->dValsA,     e->dValsB,    e->dArrival,      e->dLeafAabb,
-                     e->dLeafAabbSorted, e->dNodeOther, e->dSortTemp, e->sortTempBytes, &e->dState->status};
+  return LbvhScratch{e->dKeysA, e->dValsA, e->dValsB, e->dOpenTrees, e->dSortTemp, e->sortTempBytes,
+                     &e->dState->status};
 }
 
 static bool lbvh_out_ok(const PgaLbvh* out) {
@@ -940,8 +1344,8 @@ extern "C" PgaStatus pga_lbvh_build_counted(PgaEngine* e, const PgaTerminal* dTe
 // address is cached per device ordinal for the life of the process: the
 // library assumes that each device's primary context lives as long as the
 // process (after cudaDeviceReset the cached address is stale).  All calls
-// share the array and it keeps the last call's contents: the arrival counters
-// that must start at zero are cleared on every call, and calls that overlap
+// share the array and it keeps the last call's contents: the counters that
+// must start at zero are cleared on every call, and calls that overlap
 // on the GPU (on different streams, or from different threads) race on it.
 
 namespace pga {
@@ -986,8 +1390,7 @@ extern "C" PgaStatus pga_lbvh_build_static(const PgaTerminal* dTerminals, uint64
     base = static_cast<unsigned char*>(g_staticAddr[dev]);
   }
   if (n == 0) return PGA_OK;  // set-up only
-  // Carve the scratch: keys, two value arrays, arrival counters, leaf boxes
-  // (terminal and sorted order), the other ends of the node ranges, sort temp.
+  // Carve the scratch: keys, two value arrays, the tiles' open subtrees, sort temp.
   size_t temp = pga_lbvh_temp_bytes(n);
   size_t off = 0;
   unsigned long long* keysA = reinterpret_cast<unsigned long long*>(base + off);
@@ -996,14 +1399,8 @@ extern "C" PgaStatus pga_lbvh_build_static(const PgaTerminal* dTerminals, uint64
   off += align256(n * sizeof(uint32_t));
   uint32_t* valsB = reinterpret_cast<uint32_t*>(base + off);
   off += align256(n * sizeof(uint32_t));
-  uint32_t* arrival = reinterpret_cast<uint32_t*>(base + off);
-  off += align256(n * sizeof(uint32_t));
-  float* leafBox = reinterpret_cast<float*>(base + off);
-  off += align256(n * 6 * sizeof(float));
-  float* sortedBox = reinterpret_cast<float*>(base + off);
-  off += align256(n * 6 * sizeof(float));
-  int32_t* nodeOther = reinterpret_cast<int32_t*>(base + off);
-  off += align256(n * sizeof(int32_t));
+  void* open = base + off;
+  off += align256(pga_lbvh_open_bytes(n));
   void* sortTemp = base + off;
   off += align256(temp);
   int* err = reinterpret_cast<int*>(base + off);  // a sort wait that gives up marks it (unreported)
@@ -1012,6 +1409,6 @@ extern "C" PgaStatus pga_lbvh_build_static(const PgaTerminal* dTerminals, uint64
     set_error("pga_lbvh_build_static: fixed scratch too small for the radix sort of " + std::to_string(n) + " keys");
     return PGA_ERR_INVALID_ARGUMENT;
   }
-  const LbvhScratch w{keysA, valsA, valsB, arrival, leafBox, sortedBox, nodeOther, sortTemp, temp, err};
+  const LbvhScratch w{keysA, valsA, valsB, open, sortTemp, temp, err};
   return launch_lbvh(dTerminals, n, nullptr, bounds, out, w, (cudaStream_t)stream);
 }
