@@ -85,13 +85,21 @@ __device__ __forceinline__ unsigned long long leaf_count(const unsigned long lon
   return dN ? min(*dN, n) : n;
 }
 
-// The radix sort orders the keys' top bits [kSortLowBit, 64) only (the Morton
-// code and the path hash's top 10 bits): four passes of 10-bit digits.
-constexpr int kSortLowBit = 24;
+// The radix sort orders the leaves by Morton code (30 bits) and, below it, by
+// the path hash's top 10 bits: four passes of 10-bit digits.  The first takes
+// its digit from the hash (an array of its own, read by that pass only); after
+// it a leaf is its code and its terminal index, 8 bytes a pass each way.  The
+// full keys (Morton code << 34 | path hash >> 30) are formed by the tree
+// kernel, which gathers the records anyway.
 constexpr int kRadixBits = 10;
 constexpr uint32_t kBins = 1u << kRadixBits;
-constexpr int kSortPasses = (64 - kSortLowBit) / kRadixBits;
-static_assert(kSortLowBit + kSortPasses * kRadixBits == 64, "the passes cover bits [kSortLowBit, 64)");
+constexpr int kSortPasses = 4;
+constexpr int kHashShift = 54;  // path >> kHashShift: the hash digit
+static_assert(30 == (kSortPasses - 1) * kRadixBits && 64 - kHashShift == kRadixBits, "the passes cover code and hash");
+
+__device__ __forceinline__ uint32_t code_digit(uint32_t code, int q) {  // pass q = 1 .. 3
+  return (code >> ((q - 1) * kRadixBits)) & (kBins - 1u);
+}
 
 // Histogram of one digit of a warp's 32 keys into shared memory: one add for
 // the whole warp when every lane has the same digit (the Morton code's high
@@ -105,111 +113,125 @@ __device__ __forceinline__ void hist_add(uint32_t* h, uint32_t d, bool valid) {
     atomicAdd(h + d, 1u);
   }
 }
-
-// generateMortonCodes (GPUBVHConstructor.cuh:66-86) on terminal centres.
-// The sort's values start as the terminal index, which its first pass
-// generates, so none are written here.
-// With a device count, the keys in [count, capacity) are padding: all ones,
-// after every real key in the stable radix sort (a real key can equal it only
-// in the sorted top bits, and it comes first there by input order).
-__global__ void __launch_bounds__(kLbvhThreads) k_morton(const PgaTerminal* __restrict__ t, unsigned long long cap,
-                                                         const unsigned long long* __restrict__ dN, Bounds b,
-                                                         unsigned long long* __restrict__ keys) {
-  unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= cap) return;
-  if (i >= leaf_count(dN, cap)) {
-    keys[i] = ~0ull;
-    return;
-  }
-  const float c[3] = {__ldg(&t[i].m[3]), __ldg(&t[i].m[7]), __ldg(&t[i].m[11])};
-  const uint2 path = __ldg(reinterpret_cast<const uint2*>(&t[i].path));
-  uint32_t code = 0;
+__device__ __forceinline__ void hist_leaf(uint32_t* sh, uint32_t code, uint32_t hash, bool valid) {
+  hist_add(sh, hash, valid);
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    float nc = __fdiv_rn(__fsub_rn(c[k], b.mn[k]), b.sz[k]);
-    code |= spread(__float2uint_rz(__fmul_rn(nc, 1023.0f))) << k;
-  }
-  keys[i] = ((unsigned long long)code << 34) | ((((uint64_t)path.y << 32) | path.x) >> 30);
+  for (int q = 1; q < kSortPasses; q++) hist_add(sh + q * kBins, code_digit(code, q), valid);
 }
 
-// The four digit histograms of keys [0, n) (kSortPasses x kBins, zeroed
-// before the launch): each block counts a contiguous run of keys into shared
-// memory, kHistUnroll keys per thread in flight, then adds its nonzero bins.
+// generateMortonCodes (GPUBVHConstructor.cuh:66-86) on terminal centres, and
+// the hash digits.  The sort's values start as the terminal index, which its
+// first pass generates, so none are written here.
+// With a device count, the entries in [count, capacity) are padding: all ones,
+// after every real one in the stable radix sort.
+// HIST: also counts the digits (k_digit_hist's work), for builds small enough
+// that a launch more costs more than the shared-memory counts in this one (at
+// 152M leaves the counts take 0.6 ms here and 0.4 ms in a pass of their own).
 constexpr int kHistThreads = 512;
-constexpr int kHistUnroll = 4;
-__global__ void __launch_bounds__(kHistThreads) k_digit_hist(const unsigned long long* __restrict__ keys,
+template <bool HIST>
+__global__ void __launch_bounds__(HIST ? kHistThreads : kLbvhThreads)
+    k_morton(const PgaTerminal* __restrict__ t, unsigned long long cap, const unsigned long long* __restrict__ dN,
+             Bounds b, uint32_t* __restrict__ codes, uint16_t* __restrict__ hashes, uint32_t* __restrict__ hist) {
+  __shared__ uint32_t sh[HIST ? kSortPasses * kBins : 1];
+  if (HIST) {
+    for (uint32_t k = threadIdx.x; k < kSortPasses * kBins; k += kHistThreads) sh[k] = 0u;
+    __syncthreads();
+  }
+  const unsigned long long n = leaf_count(dN, cap);
+  const unsigned long long i = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+  uint32_t code = ~0u, hash = kBins - 1u;
+  if (i < n) {
+    const float c[3] = {__ldg(&t[i].m[3]), __ldg(&t[i].m[7]), __ldg(&t[i].m[11])};
+    hash = __ldg(reinterpret_cast<const uint32_t*>(&t[i].path) + 1) >> (kHashShift - 32);
+    code = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      float nc = __fdiv_rn(__fsub_rn(c[k], b.mn[k]), b.sz[k]);
+      code |= spread(__float2uint_rz(__fmul_rn(nc, 1023.0f))) << k;
+    }
+  }
+  if (i < cap) {
+    codes[i] = code;
+    hashes[i] = (uint16_t)hash;
+  }
+  if (HIST) {
+    hist_leaf(sh, code, hash, i < cap);
+    __syncthreads();
+    for (uint32_t k = threadIdx.x; k < kSortPasses * kBins; k += kHistThreads)
+      if (sh[k] != 0u) atomicAdd(hist + k, sh[k]);
+  }
+}
+
+// The four digit histograms of entries [0, n) (kSortPasses x kBins, zeroed
+// before the launch): each block counts a contiguous run into shared memory,
+// four entries per thread and load, then adds its nonzero bins.
+__global__ void __launch_bounds__(kHistThreads) k_digit_hist(const uint32_t* __restrict__ codes,
+                                                             const uint16_t* __restrict__ hashes,
                                                              unsigned long long n, uint32_t* __restrict__ hist) {
   __shared__ uint32_t sh[kSortPasses * kBins];
   for (uint32_t k = threadIdx.x; k < kSortPasses * kBins; k += kHistThreads) sh[k] = 0u;
   __syncthreads();
-  const unsigned long long per = (n + gridDim.x - 1) / gridDim.x;
+  const unsigned long long per = ((n + gridDim.x - 1) / gridDim.x + 3) & ~3ull;  // whole groups of four
   const unsigned long long lo = min(n, (unsigned long long)blockIdx.x * per), hi = min(n, lo + per);
   // every lane of a warp runs the same iterations (hist_add is warp-wide)
-  for (unsigned long long i0 = lo; i0 < hi; i0 += (unsigned long long)kHistThreads * kHistUnroll) {
-    unsigned long long key[kHistUnroll];
+  for (unsigned long long i0 = lo; i0 < hi; i0 += (unsigned long long)kHistThreads * 4) {
+    const unsigned long long i = i0 + threadIdx.x * 4ull;
+    uint32_t code[4] = {0u, 0u, 0u, 0u}, hash[4] = {0u, 0u, 0u, 0u};
+    if (i + 4 <= hi) {
+      const uint4 c = __ldg(reinterpret_cast<const uint4*>(codes + i));
+      const ushort4 h = __ldg(reinterpret_cast<const ushort4*>(hashes + i));
+      code[0] = c.x; code[1] = c.y; code[2] = c.z; code[3] = c.w;
+      hash[0] = h.x; hash[1] = h.y; hash[2] = h.z; hash[3] = h.w;
+    } else {
 #pragma unroll
-    for (int u = 0; u < kHistUnroll; u++) {
-      const unsigned long long i = i0 + (unsigned long long)u * kHistThreads + threadIdx.x;
-      key[u] = i < hi ? __ldcs(keys + i) : 0ull;
+      for (int u = 0; u < 4; u++)
+        if (i + u < hi) {
+          code[u] = __ldg(codes + i + u);
+          hash[u] = __ldg(hashes + i + u);
+        }
     }
 #pragma unroll
-    for (int u = 0; u < kHistUnroll; u++) {
-      const bool valid = i0 + (unsigned long long)u * kHistThreads + threadIdx.x < hi;
-#pragma unroll
-      for (int q = 0; q < kSortPasses; q++)
-        hist_add(sh + q * kBins, (uint32_t)(key[u] >> (kSortLowBit + q * kRadixBits)) & (kBins - 1u), valid);
-    }
+    for (int u = 0; u < 4; u++) hist_leaf(sh, code[u], hash[u], i + u < hi);
   }
   __syncthreads();
   for (uint32_t k = threadIdx.x; k < kSortPasses * kBins; k += kHistThreads)
     if (sh[k] != 0u) atomicAdd(hist + k, sh[k]);
 }
 
-// Exclusive scans of the four digit histograms: gBase[q][d] = where digit d's
-// keys start in pass q's output.  One block of kBins threads.
-__global__ void __launch_bounds__(kBins) k_sort_bases(const uint32_t* __restrict__ hist, uint32_t* __restrict__ gBase) {
-  __shared__ uint32_t warpSum[kBins / 32];
-  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  for (int q = 0; q < kSortPasses; q++) {
-    const uint32_t v = hist[q * kBins + threadIdx.x];
-    uint32_t x = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
-      if (lane >= (uint32_t)d) x += y;
-    }
-    if (lane == 31) warpSum[warp] = x;
-    __syncthreads();
-    uint32_t before = 0;
-    for (uint32_t w = 0; w < warp; w++) before += warpSum[w];
-    gBase[q * kBins + threadIdx.x] = before + x - v;
-    __syncthreads();
-  }
-}
-
 // One pass of the radix sort ("onesweep", Adinets & Merrill 2022), stable:
-// keys and values of [0, n) ordered by digit (key >> shift) & (kBins - 1).
-// A block takes the next tile of kSortTile keys from an atomic counter, so a
-// tile's predecessors were taken by blocks that started earlier.  Its warps
-// rank their keys by digit in input order (warp-private 16-bit histograms;
-// the lanes sharing a digit found with one ballot per digit bit) and the tile
-// goes to shared memory in digit order.  Thread t owns bins 2t and 2t + 1 and
-// publishes their counts as one 64-bit word (each half carries the flag), so
-// one walk serves both bins: decoupled look-back over the earlier tiles'
-// words until one carries an inclusive prefix.  Keys then go out in
-// contiguous runs per digit.  valsIn == nullptr means the identity (value =
-// index).  A look-back wait gives up after spinLimit polls, raising
-// PGA_ERR_TIMEOUT in *err (the order is then unspecified).
+// entries [0, n) ordered by their digit.  FIRST: the digit is the hash and the
+// value the index; else the digit is code >> shift.
+// A block takes the next tile of 512 x ITEMS entries from an atomic counter,
+// so a tile's predecessors were taken by blocks that started earlier.  Its
+// warps rank their entries by digit in input order (warp-private 16-bit
+// histograms; the lanes sharing a digit found with one ballot per digit bit)
+// and the tile goes to shared memory in digit order.  Thread t owns bins 2t
+// and 2t + 1 and publishes their counts as one 64-bit word (each half carries
+// the flag), so one walk serves both bins: decoupled look-back over the
+// earlier tiles' words until one carries an inclusive prefix.  Entries then go
+// out in contiguous runs per digit.  Where the digits start (hist: the pass's
+// digit counts) is scanned with the tile's own bins.  A look-back wait gives
+// up after spinLimit polls, raising PGA_ERR_TIMEOUT in *err (the order is then
+// unspecified).
+//
+// What bounds a pass is the rate at which inclusive prefixes move along the
+// tiles: a look-back step reads kLookback words and takes 0.7 us, so about 20
+// tiles a microsecond.  Hence the tile: ITEMS = 16 (8,192 entries, two blocks
+// an SM in 105 KB of shared memory each) for large builds; 12-byte entries in
+// tiles of 5,120 took 88 us a pass for the city's 5.9M leaves.  Up to
+// kSmallSort leaves every tile has a block of its own on the chip at ITEMS =
+// 4, and a pass takes as long as one tile: fewer serial ranking rounds.
 constexpr int kSortThreads = 512;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortItems = 10;
-constexpr uint32_t kSortTile = kSortThreads * kSortItems;
-constexpr uint32_t kHistStride = kBins + 16;  // u16 per warp histogram; bin kBins counts keys past n
+constexpr int kSmallItems = 4, kLargeItems = 16;
+constexpr unsigned long long kSmallSort = 304ull * kSortThreads * kSmallItems;  // two blocks on each of 152 SMs
+constexpr uint32_t kHistStride = kBins + 16;  // u16 per warp histogram; bin kBins counts entries past n
 constexpr uint32_t kFlagAggregate = 1u << 30, kFlagPrefix = 2u << 30, kCountMask = (1u << 30) - 1u;
 constexpr int kLookback = 16;  // predecessor words loaded at once by a look-back step
 static_assert(kBins == 2 * kSortThreads, "each thread owns two bins");
-constexpr size_t kOnesweepSmem =
-    (size_t)kSortTile * 8 + (size_t)kSortTile * 4 + (size_t)kSortWarps * kHistStride * 2 + (size_t)kBins * 8;
+constexpr size_t onesweep_smem(int items) {
+  return (size_t)kSortThreads * items * 8 + (size_t)kSortWarps * kHistStride * 2 + (size_t)kBins * 8;
+}
 
 __device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned long long v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
@@ -223,43 +245,46 @@ __device__ __forceinline__ unsigned long long pair_word(uint32_t flag, uint32_t 
   return ((unsigned long long)(flag | c1) << 32) | (flag | c0);
 }
 
+template <int ITEMS, bool FIRST>
 __global__ void __launch_bounds__(kSortThreads, 2)
-    k_onesweep(const unsigned long long* __restrict__ keysIn, const uint32_t* __restrict__ valsIn,
-               unsigned long long* __restrict__ keysOut, uint32_t* __restrict__ valsOut, unsigned long long n,
-               uint32_t shift, const uint32_t* __restrict__ gBase, unsigned long long* status,
+    k_onesweep(const uint32_t* __restrict__ codesIn, const uint16_t* __restrict__ hashes,
+               const uint32_t* __restrict__ valsIn, uint32_t* __restrict__ codesOut, uint32_t* __restrict__ valsOut,
+               unsigned long long n, uint32_t shift, const uint32_t* __restrict__ hist, unsigned long long* status,
                uint32_t* tileCounter, int* err, uint32_t spinLimit) {
+  constexpr uint32_t kTileItems = kSortThreads * ITEMS;
+  static_assert(kTileItems <= 1u << 16, "ranks and tile-local indexes of 16 bits");
   extern __shared__ __align__(16) unsigned char smem_sort[];
-  unsigned long long* sKeys = reinterpret_cast<unsigned long long*>(smem_sort);
-  uint32_t* sVals = reinterpret_cast<uint32_t*>(sKeys + kSortTile);
-  uint16_t* sHist = reinterpret_cast<uint16_t*>(sVals + kSortTile);
+  uint32_t* sCodes = reinterpret_cast<uint32_t*>(smem_sort);
+  uint32_t* sVals = sCodes + kTileItems;  // FIRST: digit << 16 | index in the tile
+  uint16_t* sHist = reinterpret_cast<uint16_t*>(sVals + kTileItems);
   uint32_t* sStart = reinterpret_cast<uint32_t*>(sHist + kSortWarps * kHistStride);
   int32_t* sDst = reinterpret_cast<int32_t*>(sStart + kBins);
   __shared__ uint32_t sTile;
-  __shared__ uint32_t sWarpSum[kSortWarps];
+  __shared__ unsigned long long sWarpSum[kSortWarps];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) sTile = atomicAdd(tileCounter, 1u);
-  uint16_t* hist = sHist + warp * kHistStride;
-  for (uint32_t k = lane; k < kHistStride / 2; k += 32) reinterpret_cast<uint32_t*>(hist)[k] = 0u;
+  const uint2 all = __ldg(reinterpret_cast<const uint2*>(hist) + threadIdx.x);  // this thread's bins, whole input
+  uint16_t* mine = sHist + warp * kHistStride;
+  for (uint32_t k = lane; k < kHistStride / 2; k += 32) reinterpret_cast<uint32_t*>(mine)[k] = 0u;
   __syncthreads();
   const uint32_t tile = sTile;
-  const unsigned long long tileBase = (unsigned long long)tile * kSortTile;
-  const unsigned long long warpBase = tileBase + (unsigned long long)warp * (32u * kSortItems);
+  const unsigned long long tileBase = (unsigned long long)tile * kTileItems;
+  const uint32_t count = (uint32_t)min((unsigned long long)kTileItems, n - tileBase);
+  const uint32_t local = warp * (32u * ITEMS) + lane;  // + 32 k: this thread's entries in the tile
   unsigned lt;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-  unsigned long long key[kSortItems];
-  uint32_t val[kSortItems];
-  uint32_t rank[kSortItems];
+  uint32_t code[ITEMS];
+  uint32_t digit[ITEMS];  // FIRST only; then the digit's low half holds the rank
 #pragma unroll
-  for (int k = 0; k < kSortItems; k++) {
-    const unsigned long long i = warpBase + (unsigned)k * 32u + lane;
-    key[k] = i < n ? __ldcs(keysIn + i) : 0ull;
-    val[k] = valsIn == nullptr ? (uint32_t)i : (i < n ? __ldcs(valsIn + i) : 0u);
+  for (int k = 0; k < ITEMS; k++) {
+    const uint32_t x = local + 32u * k;
+    code[k] = x < count ? __ldcs(codesIn + tileBase + x) : 0u;
+    digit[k] = (FIRST && x < count) ? (uint32_t)__ldcs(hashes + tileBase + x) : 0u;
   }
 #pragma unroll
-  for (int k = 0; k < kSortItems; k++) {
-    const unsigned long long i = warpBase + (unsigned)k * 32u + lane;
-    const bool valid = i < n;
-    const uint32_t d = valid ? (uint32_t)(key[k] >> shift) & (kBins - 1u) : kBins;
+  for (int k = 0; k < ITEMS; k++) {
+    const bool valid = local + 32u * k < count;
+    const uint32_t d = valid ? (FIRST ? digit[k] : (code[k] >> shift) & (kBins - 1u)) : kBins;
     // the lanes with the same digit (and validity): one ballot per digit bit
     unsigned peers = __ballot_sync(0xFFFFFFFFu, valid);
     if (!valid) peers = ~peers;
@@ -271,57 +296,63 @@ __global__ void __launch_bounds__(kSortThreads, 2)
     const int leader = __ffs(peers) - 1;
     uint32_t old = 0;
     if ((int)lane == leader) {
-      old = hist[d];
-      hist[d] = (uint16_t)(old + __popc(peers));
+      old = mine[d];
+      mine[d] = (uint16_t)(old + __popc(peers));
     }
     old = __shfl_sync(0xFFFFFFFFu, old, leader);
-    rank[k] = old + __popc(peers & lt);
+    digit[k] = (d << 16) | (old + __popc(peers & lt));
     __syncwarp();
   }
   __syncthreads();
   // Thread t owns bins 2t and 2t + 1: the warps' exclusive prefixes in place,
   // the tile's count of each bin, published for the later tiles.
-  uint32_t tot[2];
+  uint32_t tot[2] = {0u, 0u};
 #pragma unroll
-  for (int q = 0; q < 2; q++) {
-    const uint32_t d = 2u * threadIdx.x + q;
-    uint32_t run = 0;
-    for (int w = 0; w < kSortWarps; w++) {
-      uint16_t* h = sHist + w * kHistStride;
-      const uint32_t c = h[d];
-      h[d] = (uint16_t)run;
-      run += c;
-    }
-    tot[q] = run;
+  for (int w = 0; w < kSortWarps; w++) {
+    uint32_t* h = reinterpret_cast<uint32_t*>(sHist + w * kHistStride) + threadIdx.x;
+    const uint32_t c = *h;
+    *h = tot[0] | (tot[1] << 16);
+    tot[0] += c & 0xFFFFu;
+    tot[1] += c >> 16;
   }
   unsigned long long* st = status + (size_t)tile * (kBins / 2) + threadIdx.x;
   st_relaxed64(st, pair_word(tile == 0 ? kFlagPrefix : kFlagAggregate, tot[0], tot[1]));
-  // The tile's bin starts: an exclusive scan of the bins in order.
+  // Exclusive scans over the bins: the tile's bin starts (low half) and the
+  // whole input's (high half).
+  uint32_t base0, base1;
   {
-    const uint32_t v = tot[0] + tot[1];
-    uint32_t x = v;
+    const unsigned long long v = ((unsigned long long)(all.x + all.y) << 32) | (tot[0] + tot[1]);
+    unsigned long long x = v;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, d);
+      const unsigned long long y = __shfl_up_sync(0xFFFFFFFFu, x, d);
       if (lane >= (uint32_t)d) x += y;
     }
     if (lane == 31) sWarpSum[warp] = x;
     __syncthreads();
-    uint32_t before = 0;
+    unsigned long long before = x - v;
     for (uint32_t w = 0; w < warp; w++) before += sWarpSum[w];
-    sStart[2u * threadIdx.x] = before + x - v;
-    sStart[2u * threadIdx.x + 1] = before + x - v + tot[0];
+    sStart[2u * threadIdx.x] = (uint32_t)before;
+    sStart[2u * threadIdx.x + 1] = (uint32_t)before + tot[0];
+    base0 = (uint32_t)(before >> 32);
+    base1 = base0 + all.x;
   }
   __syncthreads();
   // The tile in digit order in shared memory (before the look-back: it needs
   // only the tile's own counts).
+  uint32_t val[ITEMS];
 #pragma unroll
-  for (int k = 0; k < kSortItems; k++) {
-    const unsigned long long i = warpBase + (unsigned)k * 32u + lane;
-    if (i < n) {
-      const uint32_t d = (uint32_t)(key[k] >> shift) & (kBins - 1u);
-      const uint32_t pos = sStart[d] + hist[d] + rank[k];
-      sKeys[pos] = key[k];
+  for (int k = 0; k < ITEMS; k++) {
+    const uint32_t x = local + 32u * k;
+    if (FIRST) val[k] = (digit[k] & 0xFFFF0000u) | x;
+    else val[k] = x < count ? __ldcs(valsIn + tileBase + x) : 0u;
+  }
+#pragma unroll
+  for (int k = 0; k < ITEMS; k++) {
+    if (local + 32u * k < count) {
+      const uint32_t d = digit[k] >> 16;
+      const uint32_t pos = sStart[d] + mine[d] + (digit[k] & 0xFFFFu);
+      sCodes[pos] = code[k];
       sVals[pos] = val[k];
     }
   }
@@ -366,18 +397,18 @@ __global__ void __launch_bounds__(kSortThreads, 2)
     }
     st_relaxed64(st, pair_word(kFlagPrefix, prefix0 + tot[0], prefix1 + tot[1]));
   }
-  sDst[2u * threadIdx.x] = (int32_t)(__ldg(gBase + 2u * threadIdx.x) + prefix0);
-  sDst[2u * threadIdx.x + 1] = (int32_t)(__ldg(gBase + 2u * threadIdx.x + 1) + prefix1);
+  sDst[2u * threadIdx.x] = (int32_t)(base0 + prefix0 - sStart[2u * threadIdx.x]);
+  sDst[2u * threadIdx.x + 1] = (int32_t)(base1 + prefix1 - sStart[2u * threadIdx.x + 1]);
   __syncthreads();
   // Out: consecutive positions of one digit go to consecutive places.
-  const uint32_t count = (uint32_t)min((unsigned long long)kSortTile, n - tileBase);
+#pragma unroll 4
   for (uint32_t p = threadIdx.x; p < count; p += kSortThreads) {
-    const unsigned long long kk = sKeys[p];
-    const uint32_t d = (uint32_t)(kk >> shift) & (kBins - 1u);
-    const long long o = (long long)sDst[d] + (long long)(p - sStart[d]);
-    if (o < 0 || (unsigned long long)o >= n) continue;  // only after a look-back that gave up
-    keysOut[o] = kk;
-    valsOut[o] = sVals[p];
+    const uint32_t c = sCodes[p], v = sVals[p];
+    const uint32_t d = FIRST ? v >> 16 : (c >> shift) & (kBins - 1u);
+    const uint32_t o = (uint32_t)sDst[d] + p;
+    if (o >= n) continue;  // only after a look-back that gave up
+    codesOut[o] = c;
+    valsOut[o] = FIRST ? (uint32_t)tileBase + (v & 0xFFFFu) : v;
   }
 }
 
@@ -430,7 +461,7 @@ struct __align__(16) OpenTree {
 static_assert(sizeof(OpenTree) == 32, "two 16-byte words");
 
 struct TreeArgs {
-  const unsigned long long* keys;  // sorted by their top bits (kSortLowBit and up)
+  const uint32_t* codes;  // Morton codes, sorted (and below them by the hash digit)
   const uint32_t* vals;
   const PgaTerminal* t;
   unsigned long long cap;
@@ -558,15 +589,14 @@ __device__ __forceinline__ uint32_t leaf_value(const TreeArgs& a, unsigned long 
   return min(__ldg(a.vals + i), (uint32_t)n - 1u);
 }
 
-// The leaves' final order.  The radix sort orders the keys' top bits
-// [kSortLowBit, 64) only (Morton code and the path hash's top 10 bits) and
-// leaves runs of equal top bits in input order; inside a run the order is by
-// the full path hash, then by terminal index: what a full 64-bit sort with a
-// path tie fix gives.  Most runs are short: a tile's threads see the tile's
-// paths and those of kHalo keys either side in shared memory (window position
-// q is leaf base - kHalo + q), and each member of a run counts the members
-// before it.  A run that reaches past the window is ordered by the whole
-// block (tie_select).
+// The leaves' final order.  The radix sort orders the Morton code and the path
+// hash's top 10 bits only and leaves runs of equal ones in input order; inside
+// a run the order is by the full path hash, then by terminal index: what a
+// full 64-bit sort with a path tie fix gives.  Most runs are short: a tile's
+// threads see the tile's paths and those of kHalo leaves either side in shared
+// memory (window position q is leaf base - kHalo + q), and each member of a
+// run counts the members before it.  A run that reaches past the window is
+// ordered by the whole block (tie_select).
 struct TieWindow {
   uint64_t path[kTile + 2 * kHalo];
   uint32_t val[kTile + 2 * kHalo];
@@ -589,6 +619,21 @@ __device__ __forceinline__ void tie_run(const uint32_t* eq, int q, int& s, int& 
   m = ~eq[w] & (0xFFFFFFFFu << ((q + 1) & 31));
   while (m == 0u && w + 1 < kWindowWords) m = ~eq[++w];
   e = m != 0u ? w * 32 + __ffs(m) - 2 : kWindowWords * 32 - 1;
+}
+
+// What the sort ordered at position i: Morton code, then hash digit.
+__device__ __forceinline__ uint64_t tie_key(const TreeArgs& a, unsigned long long n, unsigned long long i) {
+  return ((uint64_t)__ldg(a.codes + i) << kRadixBits) | (term_path(a.t, leaf_value(a, i, n)) >> kHashShift);
+}
+
+// Whether the leaf at position i has code c and hash digit h; its value and
+// path when the code agrees.
+__device__ __forceinline__ bool tie_leaf(const TreeArgs& a, unsigned long long n, unsigned long long i, uint32_t c,
+                                         uint32_t h, uint32_t& val, uint64_t& path) {
+  if (__ldg(a.codes + i) != c) return false;
+  val = leaf_value(a, i, n);
+  path = term_path(a.t, val);
+  return (uint32_t)(path >> kHashShift) == h;
 }
 
 // (path, value) number `rank` in order among those of sorted positions
@@ -667,19 +712,17 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
   const bool valid = tid < cnt;
   const unsigned long long k = base + tid;
 
-  unsigned long long key = 0;
+  uint32_t code = 0, before = ~0u;  // this leaf's and its left neighbour's
   uint32_t val = 0;
   uint64_t path = 0;
   float mn[3], mx[3];
-  bool eq = false;
   if (valid) {
-    key = __ldg(a.keys + k);
+    code = __ldg(a.codes + k);
     val = leaf_value(a, k, n);
     int d = -1;
     if (k > 0) {
-      const unsigned long long before = __ldg(a.keys + k - 1);
-      d = boundary_delta((uint32_t)(before >> 34), (uint32_t)(key >> 34), (uint32_t)k);
-      eq = (before >> kSortLowBit) == (key >> kSortLowBit);
+      before = __ldg(a.codes + k - 1);
+      d = boundary_delta(before, code, (uint32_t)k);
     }
     sDelta[tid] = (signed char)d;
     gather_leaf(a.t, val, mn, mx, path);
@@ -689,61 +732,75 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
     fPath[tid] = path;
     fVal[tid] = val;
   }
-  bool eqEnd = false;
+  bool sameEnd = false;
   if (tid == cnt - 1) {  // the tile's right end
     int d = -1;
     if (k + 1 < n) {
-      const unsigned long long after = __ldg(a.keys + k + 1);
-      d = boundary_delta((uint32_t)(key >> 34), (uint32_t)(after >> 34), (uint32_t)(k + 1));
-      eqEnd = (after >> kSortLowBit) == (key >> kSortLowBit);  // then cnt == kTile
+      const uint32_t after = __ldg(a.codes + k + 1);
+      d = boundary_delta(code, after, (uint32_t)(k + 1));
+      sameEnd = after == code;  // then cnt == kTile
     }
     sDelta[cnt] = (signed char)d;
   }
-  const unsigned eqs = __ballot_sync(kAll, eq);
-  if (lane == 0) sEq[1 + warp] = eqs;
   if (tid < kTile / 32) sOpen[tid] = 0u;
   if (tid == 0) {
     sEq[0] = 0u;
     sLong = 0;
     sQueued[0] = sQueued[1] = 0u;
   }
-  if (tid == cnt - 1) sEq[kWindowWords - 1] = eqEnd ? 1u : 0u;
-  if (__syncthreads_or(eq || eqEnd)) {
-    // the halo keys that belong to the runs at the tile's ends
+  if (tid == cnt - 1) sEq[kWindowWords - 1] = 0u;
+  const bool same = valid && k > 0 && before == code;
+  if (__syncthreads_or(same || sameEnd)) {
+    // Equal to the left neighbour?  (The first leaf's and the right end's
+    // neighbours are in other tiles.)
+    bool eq = same;
+    if (same) {
+      const uint64_t other = tid > 0 ? win.path[kHalo + tid - 1] : term_path(a.t, leaf_value(a, k - 1, n));
+      eq = (other >> kHashShift) == (path >> kHashShift);
+    }
+    const unsigned eqs = __ballot_sync(kAll, eq);
+    if (lane == 0) sEq[1 + warp] = eqs;
+    if (sameEnd && (term_path(a.t, leaf_value(a, k + 1, n)) >> kHashShift) == (path >> kHashShift))
+      sEq[kWindowWords - 1] = 1u;
+    __syncthreads();
+    // the halo leaves that belong to the runs at the tile's ends
     bool halo = false;
     int hq = 0;
+    uint64_t hPath = 0;
     if (warp == 0 && (sEq[1] & 1u)) {
-      const unsigned long long top = __shfl_sync(kAll, key, 0) >> kSortLowBit;
+      const uint32_t c = __shfl_sync(kAll, code, 0);
+      const uint32_t h = (uint32_t)(win.path[kHalo] >> kHashShift);
       const long long i = (long long)base - kHalo + lane;
-      const bool same = i >= 0 && (__ldg(a.keys + max(i, 0ll)) >> kSortLowBit) == top;
-      const int have = __clz((int)~__ballot_sync(kAll, same));  // consecutive ones from lane 31 down
+      const bool in = i >= 0 && tie_leaf(a, n, (unsigned long long)max(i, 0ll), c, h, val, hPath);
+      const int have = __clz((int)~__ballot_sync(kAll, in));  // consecutive ones from lane 31 down
       halo = (int)lane >= 32 - have;
       hq = (int)lane;
       if (lane == 0) {
-        const bool more = have == 32 && base > kHalo && (__ldg(a.keys + base - kHalo - 1) >> kSortLowBit) == top;
+        uint32_t v;
+        uint64_t p;
+        const bool more = have == 32 && base > kHalo && tie_leaf(a, n, base - kHalo - 1, c, h, v, p);
         sEq[0] = (have >= 2 ? kAll << (33 - have) : 0u) | (more ? 1u : 0u);
         if (more) atomicOr(&sLong, 1);
       }
-      if (halo) val = leaf_value(a, (unsigned long long)i, n);
     } else if (warp == 1 && (sEq[kWindowWords - 1] & 1u)) {
-      const unsigned long long top = __ldg(a.keys + base + kTile - 1) >> kSortLowBit;
+      const uint32_t c = __ldg(a.codes + base + kTile - 1);
+      const uint32_t h = (uint32_t)(win.path[kHalo + kTile - 1] >> kHashShift);
       const unsigned long long i = base + kTile + lane;
-      const bool same = i < n && (__ldg(a.keys + min(i, n - 1)) >> kSortLowBit) == top;
-      const unsigned m = __ballot_sync(kAll, same);
+      const bool in = i < n && tie_leaf(a, n, min(i, n - 1), c, h, val, hPath);
+      const unsigned m = __ballot_sync(kAll, in);
       const int have = m == kAll ? 32 : __ffs((int)~m) - 1;
       halo = (int)lane < have;
       hq = (int)(kHalo + kTile + lane);
       if (lane == 0) {
         const unsigned long long past = base + kTile + kHalo;
-        const bool more = have == 32 && past < n && (__ldg(a.keys + past) >> kSortLowBit) == top;
+        uint32_t v;
+        uint64_t p;
+        const bool more = have == 32 && past < n && tie_leaf(a, n, past, c, h, v, p);
         sEq[kWindowWords - 1] = have == 32 ? kAll : (1u << have) - 1u;
         if (more) atomicOr(&sLong, 2);
       }
-      if (halo) val = leaf_value(a, (unsigned long long)i, n);
     }
-    uint64_t hPath = 0;
     if (halo) {
-      hPath = term_path(a.t, val);
       win.path[hq] = hPath;
       win.val[hq] = val;
     }
@@ -783,11 +840,11 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
       __syncthreads();
       const unsigned long long end = side == 0 ? base : base + cnt - 1;
       if (tid == 0) {
-        const unsigned long long top = a.keys[end] >> kSortLowBit;
-        unsigned long long lo = 0, hi = end;  // first position with these top bits
+        const uint64_t top = tie_key(a, n, end);
+        unsigned long long lo = 0, hi = end;  // first position with this code and hash digit
         while (lo < hi) {
           const unsigned long long mid = (lo + hi) >> 1;
-          if ((a.keys[mid] >> kSortLowBit) < top) lo = mid + 1;
+          if (tie_key(a, n, mid) < top) lo = mid + 1;
           else hi = mid;
         }
         sRun[0] = lo;
@@ -795,7 +852,7 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
         hi = n;  // first position past them
         while (lo < hi) {
           const unsigned long long mid = (lo + hi) >> 1;
-          if ((a.keys[mid] >> kSortLowBit) <= top) lo = mid + 1;
+          if (tie_key(a, n, mid) <= top) lo = mid + 1;
           else hi = mid;
         }
         sRun[1] = lo;
@@ -838,7 +895,7 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
   const Forest f{sBox, sNodeBox, sFlag, sDelta, sOpen};
   if (valid) {
     a.leafTerminal[k] = fVal[tid];
-    a.outKeys[k] = ((key >> 34) << 34) | (fPath[tid] >> 30);
+    a.outKeys[k] = ((unsigned long long)code << 34) | (fPath[tid] >> 30);
     load_box(sBox + tid * 6, mn, mx);
   }
   __syncthreads();  // the node boxes take the window's place
@@ -1017,8 +1074,7 @@ __global__ void __launch_bounds__(kTile) k_join(TreeArgs a) {
       if (tid == 0) {
         const unsigned long long end = min(n, (first + next) * stride * kTile);
         sLeft[count] = (uint32_t)end;
-        delta[count] = (signed char)(end < n ? boundary_delta((uint32_t)(__ldg(a.keys + end - 1) >> 34),
-                                                              (uint32_t)(__ldg(a.keys + end) >> 34), (uint32_t)end)
+        delta[count] = (signed char)(end < n ? boundary_delta(__ldg(a.codes + end - 1), __ldg(a.codes + end), (uint32_t)end)
                                              : -1);
       }
       __syncthreads();
@@ -1171,10 +1227,12 @@ __global__ void __launch_bounds__(kTile) k_join(TreeArgs a) {
 
 using namespace pga;
 
-// Sort scratch: the digit histograms, the passes' tile counters, the tree's
-// arrival counters and the look-back words (zeroed by one memset per build),
-// then the digit bases.
-static unsigned long long sort_tiles(unsigned long long n) { return (n + kSortTile - 1) / kSortTile; }
+// Sort scratch, zeroed by one memset per build: the digit histograms, the
+// passes' tile counters, the tree's arrival counters and the look-back words.
+static unsigned long long sort_tiles(unsigned long long n) {
+  const unsigned long long tile = (unsigned long long)kSortThreads * (n <= kSmallSort ? kSmallItems : kLargeItems);
+  return (n + tile - 1) / tile;
+}
 static unsigned long long tree_tiles(unsigned long long n) { return (n + kTile - 1) / kTile; }
 static unsigned long long tree_joins(unsigned long long n) {
   unsigned long long sum = 0;
@@ -1185,11 +1243,14 @@ static unsigned long long tree_joins(unsigned long long n) {
   return (sum + 1) & ~1ull;  // the look-back words after them are 8 bytes wide
 }
 
+static size_t sort_words(unsigned long long n) {
+  return (size_t)(kSortPasses * kBins + 64 + tree_joins(n) + (unsigned long long)kSortPasses * sort_tiles(n) * kBins);
+}
+
 extern "C" size_t pga_lbvh_temp_bytes(uint64_t n) {
   n = n ? n : 1;
-  return (size_t)(kSortPasses * kBins + 64 + tree_joins(n) + (unsigned long long)kSortPasses * sort_tiles(n) * kBins +
-                  kSortPasses * kBins) *
-         sizeof(uint32_t);
+  // a smaller build may have more, smaller tiles
+  return std::max(sort_words(n), sort_words(std::min<unsigned long long>(n, kSmallSort))) * sizeof(uint32_t);
 }
 
 // The tiles' open subtrees, then their counts.
@@ -1215,11 +1276,39 @@ struct LbvhScratch {
 // Polls of a look-back wait before it gives up (each followed by a 32 ns sleep).
 constexpr uint32_t kSortSpinLimit = 1u << 22;
 
+template <int ITEMS>
+static PgaStatus launch_sort(unsigned long long n, uint32_t* codesA, uint32_t* codesB, const uint16_t* hashes,
+                             uint32_t* valsA, uint32_t* valsB, const uint32_t* hist, uint32_t* counters,
+                             unsigned long long* words, int* err, cudaStream_t s) {
+  const unsigned tiles = (unsigned)sort_tiles(n);
+  constexpr size_t smem = onesweep_smem(ITEMS);
+  PGA_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<ITEMS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  PGA_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<ITEMS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  for (int q = 0; q < kSortPasses; q++) {
+    const bool even = q % 2 == 0;
+    const uint32_t* cIn = even ? codesA : codesB;
+    uint32_t* cOut = even ? codesB : codesA;
+    const uint32_t* vIn = even ? valsA : valsB;
+    uint32_t* vOut = even ? valsB : valsA;
+    unsigned long long* w = words + (size_t)q * tiles * (kBins / 2);
+    if (q == 0)
+      k_onesweep<ITEMS, true><<<tiles, kSortThreads, smem, s>>>(cIn, hashes, nullptr, cOut, vOut, n, 0u, hist, w,
+                                                                 counters, err, kSortSpinLimit);
+    else
+      k_onesweep<ITEMS, false><<<tiles, kSortThreads, smem, s>>>(cIn, nullptr, vIn, cOut, vOut, n,
+                                                                  (uint32_t)((q - 1) * kRadixBits), hist + q * kBins, w,
+                                                                  counters + q, err, kSortSpinLimit);
+    PGA_CUDA_TRY(cudaGetLastError());
+  }
+  static_assert(kSortPasses % 2 == 0, "an even number of passes ends in codesA and valsA");
+  return PGA_OK;
+}
+
 // The launches of a build over `cap` leaves, or over min(*dN, cap) when dN is
-// a device count (then `cap` sizes the grids and the sort): Morton codes, the
-// digit histograms and bases, four sort passes (keys ping-pong between keysA
-// and out->keys, ending in keysA) and the tree, which writes the final keys
-// to out->keys.
+// a device count (then `cap` sizes the grids and the sort): Morton codes and
+// digit histograms, four sort passes (codes and values ping-pong and end in
+// the A arrays) and the tree.  The codes' two arrays share keysA; the hash
+// digits lie in out->keys until the tree writes the final keys there.
 static PgaStatus launch_lbvh(const PgaTerminal* t, unsigned long long cap, const unsigned long long* dN,
                              const PgaBounds* bounds, const PgaLbvh* out, const LbvhScratch& w, cudaStream_t s) {
   Bounds b;
@@ -1227,52 +1316,40 @@ static PgaStatus launch_lbvh(const PgaTerminal* t, unsigned long long cap, const
     b.mn[k] = bounds->min[k];
     b.sz[k] = bounds->max[k] - bounds->min[k];
   }
-  const unsigned long long tiles = sort_tiles(cap);
-  if (pga_lbvh_temp_bytes(cap) > w.sortTempBytes) {
+  if (sort_words(cap) * sizeof(uint32_t) > w.sortTempBytes) {
     set_error("LBVH: sort scratch too small for " + std::to_string(cap) + " keys");
     return PGA_ERR_INVALID_ARGUMENT;
   }
   uint32_t* hist = static_cast<uint32_t*>(w.sortTemp);
   uint32_t* counters = hist + kSortPasses * kBins;
   uint32_t* joins = counters + 64;
-  uint32_t* status = joins + tree_joins(cap);
-  uint32_t* gBase = status + (size_t)kSortPasses * tiles * kBins;
-  PGA_CUDA_TRY(cudaMemsetAsync(hist, 0, (size_t)(gBase - hist) * sizeof(uint32_t), s));
-  int dev = 0, sms = 0;
-  PGA_CUDA_TRY(cudaGetDevice(&dev));
-  PGA_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  unsigned long long* words = reinterpret_cast<unsigned long long*>(joins + tree_joins(cap));
+  PGA_CUDA_TRY(cudaMemsetAsync(hist, 0, sort_words(cap) * sizeof(uint32_t), s));
+  uint32_t* codesA = reinterpret_cast<uint32_t*>(w.keysA);
+  uint32_t* codesB = codesA + cap;
+  uint16_t* hashes = reinterpret_cast<uint16_t*>(out->keys);
   const unsigned blocks = (unsigned)((cap + kLbvhThreads - 1) / kLbvhThreads);
-  unsigned long long* outKeys = (unsigned long long*)out->keys;
-  k_morton<<<blocks, kLbvhThreads, 0, s>>>(t, cap, dN, b, w.keysA);
-  PGA_CUDA_TRY(cudaGetLastError());
-  const unsigned histBlocks =
-      (unsigned)std::min<unsigned long long>((cap + kHistThreads - 1) / kHistThreads, (unsigned long long)sms * 4);
-  k_digit_hist<<<histBlocks, kHistThreads, 0, s>>>(w.keysA, cap, hist);
-  PGA_CUDA_TRY(cudaGetLastError());
-  k_sort_bases<<<1, kBins, 0, s>>>(hist, gBase);
-  PGA_CUDA_TRY(cudaGetLastError());
-  PGA_CUDA_TRY(cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kOnesweepSmem));
-  // The first pass reads the identity values (terminal index); the values
-  // then ping-pong valsB -> valsA -> valsB -> valsA.
-  unsigned long long* kIn = w.keysA;
-  unsigned long long* kOut = outKeys;
-  uint32_t* vIn = nullptr;
-  uint32_t* vOut = w.valsB;
-  unsigned long long* words = reinterpret_cast<unsigned long long*>(status);
-  for (int q = 0; q < kSortPasses; q++) {
-    k_onesweep<<<(unsigned)tiles, kSortThreads, kOnesweepSmem, s>>>(
-        kIn, vIn, kOut, vOut, cap, (uint32_t)(kSortLowBit + q * kRadixBits), gBase + q * kBins,
-        words + (size_t)q * tiles * (kBins / 2), counters + q, w.err, kSortSpinLimit);
+  PgaStatus st;
+  if (cap <= kSmallSort) {
+    k_morton<true><<<(unsigned)((cap + kHistThreads - 1) / kHistThreads), kHistThreads, 0, s>>>(t, cap, dN, b, codesA,
+                                                                                              hashes, hist);
     PGA_CUDA_TRY(cudaGetLastError());
-    std::swap(kIn, kOut);
-    vIn = vOut;
-    vOut = vOut == w.valsB ? w.valsA : w.valsB;
+    st = launch_sort<kSmallItems>(cap, codesA, codesB, hashes, w.valsA, w.valsB, hist, counters, words, w.err, s);
+  } else {
+    k_morton<false><<<blocks, kLbvhThreads, 0, s>>>(t, cap, dN, b, codesA, hashes, hist);
+    PGA_CUDA_TRY(cudaGetLastError());
+    int dev = 0, sms = 0;
+    PGA_CUDA_TRY(cudaGetDevice(&dev));
+    PGA_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    k_digit_hist<<<(unsigned)sms * 4, kHistThreads, 0, s>>>(codesA, hashes, cap, hist);
+    PGA_CUDA_TRY(cudaGetLastError());
+    st = launch_sort<kLargeItems>(cap, codesA, codesB, hashes, w.valsA, w.valsB, hist, counters, words, w.err, s);
   }
-  static_assert(kSortPasses % 2 == 0, "an even number of passes ends in keysA and valsA");
+  if (st != PGA_OK) return st;
   OpenTree* open = static_cast<OpenTree*>(w.open);
-  const TreeArgs a{w.keysA,    w.valsA,           t,       cap,  dN, out->nodes, out->leafParents, out->aabbs,
-                   out->leafTerminal, outKeys, open, reinterpret_cast<uint32_t*>(open + (size_t)blocks * kMaxOpen),
-                   joins};
+  const TreeArgs a{codesA, w.valsA, t, cap, dN, out->nodes, out->leafParents, out->aabbs, out->leafTerminal,
+                   (unsigned long long*)out->keys, open,
+                   reinterpret_cast<uint32_t*>(open + (size_t)blocks * kMaxOpen), joins};
   k_tree<<<blocks, kTile, 0, s>>>(a);
   PGA_CUDA_TRY(cudaGetLastError());
   if (blocks > 1) {
