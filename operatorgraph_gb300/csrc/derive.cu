@@ -498,7 +498,7 @@ PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* co
   // LBVH scratch for up to maxTerminals leaves.
   e->sortTempBytes = pga_lbvh_temp_bytes(c.maxTerminals);
   ALLOC(e->dSortTemp, e->sortTempBytes);
-  ALLOC(e->dKeysA, c.maxTerminals * sizeof(unsigned long long));
+  ALLOC(e->dKeysA, (c.maxTerminals + 2) * sizeof(unsigned long long));  // two arrays of codes, 16-byte aligned
   ALLOC(e->dValsA, c.maxTerminals * sizeof(uint32_t));
   ALLOC(e->dValsB, c.maxTerminals * sizeof(uint32_t));
   ALLOC(e->dOpenTrees, pga_lbvh_open_bytes(c.maxTerminals));

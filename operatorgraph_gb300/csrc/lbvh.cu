@@ -12,7 +12,7 @@
 //  * AABBs start from -FLT_MAX instead of FLT_MIN (AABB.cuh:20) and the two
 //    climbers that meet at a node are ordered by an acquire-release exchange.
 // The reference sorts with thrust::sort (GPUBVHConstructor.cuh:311-312); here
-// the sort is this file's own onesweep radix sort (see k_onesweep).
+// the sort is this file's own radix sort (see k_sort_pass).
 #include <cuda_runtime.h>
 
 #include <cfloat>
@@ -124,9 +124,8 @@ __device__ __forceinline__ void hist_leaf(uint32_t* sh, uint32_t code, uint32_t 
 // first pass generates, so none are written here.
 // With a device count, the entries in [count, capacity) are padding: all ones,
 // after every real one in the stable radix sort.
-// HIST: also counts the digits (k_digit_hist's work), for builds small enough
-// that a launch more costs more than the shared-memory counts in this one (at
-// 152M leaves the counts take 0.6 ms here and 0.4 ms in a pass of their own).
+// HIST: also counts the digits, for the small builds' sort (the large ones
+// count them pass by pass).
 constexpr int kHistThreads = 512;
 template <bool HIST>
 __global__ void __launch_bounds__(HIST ? kHistThreads : kLbvhThreads)
@@ -162,75 +161,50 @@ __global__ void __launch_bounds__(HIST ? kHistThreads : kLbvhThreads)
   }
 }
 
-// The four digit histograms of entries [0, n) (kSortPasses x kBins, zeroed
-// before the launch): each block counts a contiguous run into shared memory,
-// four entries per thread and load, then adds its nonzero bins.
-__global__ void __launch_bounds__(kHistThreads) k_digit_hist(const uint32_t* __restrict__ codes,
-                                                             const uint16_t* __restrict__ hashes,
-                                                             unsigned long long n, uint32_t* __restrict__ hist) {
-  __shared__ uint32_t sh[kSortPasses * kBins];
-  for (uint32_t k = threadIdx.x; k < kSortPasses * kBins; k += kHistThreads) sh[k] = 0u;
-  __syncthreads();
-  const unsigned long long per = ((n + gridDim.x - 1) / gridDim.x + 3) & ~3ull;  // whole groups of four
-  const unsigned long long lo = min(n, (unsigned long long)blockIdx.x * per), hi = min(n, lo + per);
-  // every lane of a warp runs the same iterations (hist_add is warp-wide)
-  for (unsigned long long i0 = lo; i0 < hi; i0 += (unsigned long long)kHistThreads * 4) {
-    const unsigned long long i = i0 + threadIdx.x * 4ull;
-    uint32_t code[4] = {0u, 0u, 0u, 0u}, hash[4] = {0u, 0u, 0u, 0u};
-    if (i + 4 <= hi) {
-      const uint4 c = __ldg(reinterpret_cast<const uint4*>(codes + i));
-      const ushort4 h = __ldg(reinterpret_cast<const ushort4*>(hashes + i));
-      code[0] = c.x; code[1] = c.y; code[2] = c.z; code[3] = c.w;
-      hash[0] = h.x; hash[1] = h.y; hash[2] = h.z; hash[3] = h.w;
-    } else {
-#pragma unroll
-      for (int u = 0; u < 4; u++)
-        if (i + u < hi) {
-          code[u] = __ldg(codes + i + u);
-          hash[u] = __ldg(hashes + i + u);
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; u++) hist_leaf(sh, code[u], hash[u], i + u < hi);
-  }
-  __syncthreads();
-  for (uint32_t k = threadIdx.x; k < kSortPasses * kBins; k += kHistThreads)
-    if (sh[k] != 0u) atomicAdd(hist + k, sh[k]);
-}
-
-// One pass of the radix sort ("onesweep", Adinets & Merrill 2022), stable:
-// entries [0, n) ordered by their digit.  FIRST: the digit is the hash and the
-// value the index; else the digit is code >> shift.
-// A block takes the next tile of 512 x ITEMS entries from an atomic counter,
-// so a tile's predecessors were taken by blocks that started earlier.  Its
-// warps rank their entries by digit in input order (warp-private 16-bit
-// histograms; the lanes sharing a digit found with one ballot per digit bit)
-// and the tile goes to shared memory in digit order.  Thread t owns bins 2t
-// and 2t + 1 and publishes their counts as one 64-bit word (each half carries
-// the flag), so one walk serves both bins: decoupled look-back over the
-// earlier tiles' words until one carries an inclusive prefix.  Entries then go
-// out in contiguous runs per digit.  Where the digits start (hist: the pass's
-// digit counts) is scanned with the tile's own bins.  A look-back wait gives
-// up after spinLimit polls, raising PGA_ERR_TIMEOUT in *err (the order is then
-// unspecified).
+// One pass of the radix sort, stable: entries [0, n) ordered by their digit.
+// FIRST: the digit is the hash and the value the index; else the digit is
+// code >> shift.
+// A block takes a tile of 512 x ITEMS entries.  Its warps rank their entries by
+// digit in input order (warp-private 16-bit histograms) and the tile goes to
+// shared memory in digit order; thread t owns bins 2t and 2t + 1.  Entries then go out in
+// contiguous runs per digit, to the digit's start (a scan of the pass's digit
+// counts, made with the tile's own) plus the digit's count in the earlier
+// tiles.  Where that count comes from is the difference between two forms:
 //
-// What bounds a pass is the rate at which inclusive prefixes move along the
-// tiles: a look-back step reads kLookback words and takes 0.7 us, so about 20
-// tiles a microsecond.  Hence the tile: ITEMS = 16 (8,192 entries, two blocks
-// an SM in 105 KB of shared memory each) for large builds; 12-byte entries in
-// tiles of 5,120 took 88 us a pass for the city's 5.9M leaves.  Up to
-// kSmallSort leaves every tile has a block of its own on the chip at ITEMS =
-// 4, and a pass takes as long as one tile: fewer serial ranking rounds.
+// * Up to kSmallSort leaves (every tile has a block of its own on the chip):
+//   one launch a pass ("onesweep", Adinets & Merrill 2022).  A block takes the
+//   next tile from an atomic counter, so a tile's predecessors were taken by
+//   blocks that started earlier, publishes its bins' counts as one 64-bit word
+//   (each half carries the flag) and looks back over the earlier tiles' words
+//   until one carries an inclusive prefix.  A wait gives up after spinLimit
+//   polls, raising PGA_ERR_TIMEOUT in *err (the order is then unspecified).
+//   ITEMS = 4: few serial ranking rounds, a pass takes as long as one tile.
+//   Lanes sharing a digit are found through a mask per digit in which each sets
+//   its bit (20,011 leaves: 5.9 us a pass, 6.9 with ballots).
+// * Larger builds: k_sort_count and k_sort_scan before the pass (COUNTED).
+//   With hundreds of tiles in flight the look-back takes eight steps of 16
+//   words and 0.7 us each, most of a tile's instructions; a count reads 4 bytes
+//   an entry, which mostly hit L2, and its scan 4 KB a tile.  City of 5.9M
+//   leaves: four passes took 281 us with the look-back and the histograms that
+//   it needs, 224 with the counts.  Lanes sharing a digit are found with a
+//   ballot per digit bit: the masks' atomics collide where many neighbours
+//   share one (19M leaves of the mixed batch: 152 us a pass, ballots 141).
 constexpr int kSortThreads = 512;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSmallItems = 4, kLargeItems = 16;
 constexpr unsigned long long kSmallSort = 304ull * kSortThreads * kSmallItems;  // two blocks on each of 152 SMs
-constexpr uint32_t kHistStride = kBins + 16;  // u16 per warp histogram; bin kBins counts entries past n
+constexpr uint32_t kHistStride = kBins + 16;  // u16 per warp histogram (padded: the warps' rows start in other banks)
 constexpr uint32_t kFlagAggregate = 1u << 30, kFlagPrefix = 2u << 30, kCountMask = (1u << 30) - 1u;
 constexpr int kLookback = 16;  // predecessor words loaded at once by a look-back step
 static_assert(kBins == 2 * kSortThreads, "each thread owns two bins");
-constexpr size_t onesweep_smem(int items) {
-  return (size_t)kSortThreads * items * 8 + (size_t)kSortWarps * kHistStride * 2 + (size_t)kBins * 8;
+// The tile's entries, and before them the warps' digit masks in their place.
+__host__ __device__ constexpr size_t sort_entry_bytes(int items) {
+  const size_t entries = (size_t)kSortThreads * items * 8;
+  const size_t masks = items == kSmallItems ? (size_t)kSortWarps * kBins * 4 : 0;
+  return entries > masks ? entries : masks;
+}
+constexpr size_t sort_pass_smem(int items) {
+  return sort_entry_bytes(items) + (size_t)kSortWarps * kHistStride * 2 + (size_t)kBins * 8;
 }
 
 __device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned long long v) {
@@ -245,63 +219,168 @@ __device__ __forceinline__ unsigned long long pair_word(uint32_t flag, uint32_t 
   return ((unsigned long long)(flag | c1) << 32) | (flag | c0);
 }
 
-template <int ITEMS, bool FIRST>
-__global__ void __launch_bounds__(kSortThreads, 2)
-    k_onesweep(const uint32_t* __restrict__ codesIn, const uint16_t* __restrict__ hashes,
-               const uint32_t* __restrict__ valsIn, uint32_t* __restrict__ codesOut, uint32_t* __restrict__ valsOut,
-               unsigned long long n, uint32_t shift, const uint32_t* __restrict__ hist, unsigned long long* status,
-               uint32_t* tileCounter, int* err, uint32_t spinLimit) {
+// The counted form.  Group g of kSortGroups blocks counts a contiguous run of
+// tiles: rows[tile][bin] gets the bin's count in the group's earlier tiles,
+// groups[g][bin] the group's total.
+constexpr uint32_t kSortGroups = 304;  // two blocks on each of 152 SMs
+template <bool FIRST>
+__global__ void __launch_bounds__(kSortThreads) k_sort_count(const uint32_t* __restrict__ codes,
+                                                             const uint16_t* __restrict__ hashes, unsigned long long n,
+                                                             uint32_t shift, uint32_t tiles, uint32_t perGroup,
+                                                             uint32_t* __restrict__ rows,
+                                                             uint32_t* __restrict__ groups) {
+  constexpr uint32_t kTileItems = kSortThreads * kLargeItems;
+  __shared__ uint32_t sh[kBins];
+  const uint32_t first = blockIdx.x * perGroup, last = min(tiles, first + perGroup);
+  uint2* bins = reinterpret_cast<uint2*>(sh) + threadIdx.x;
+  uint2 run = make_uint2(0u, 0u);
+  *bins = run;
+  __syncthreads();
+  for (uint32_t tile = first; tile < last; tile++) {
+    const unsigned long long base = (unsigned long long)tile * kTileItems;
+    const uint32_t count = (uint32_t)min((unsigned long long)kTileItems, n - base);
+    uint32_t d[kLargeItems];
+#pragma unroll
+    for (int k = 0; k < kLargeItems / 4; k++) {
+      const uint32_t x = (k * kSortThreads + threadIdx.x) * 4u;
+      if (x + 4 <= count) {
+        if (FIRST) {
+          const ushort4 h = __ldg(reinterpret_cast<const ushort4*>(hashes + base + x));
+          d[k * 4 + 0] = h.x; d[k * 4 + 1] = h.y; d[k * 4 + 2] = h.z; d[k * 4 + 3] = h.w;
+        } else {
+          const uint4 c = __ldg(reinterpret_cast<const uint4*>(codes + base + x));
+          d[k * 4 + 0] = c.x; d[k * 4 + 1] = c.y; d[k * 4 + 2] = c.z; d[k * 4 + 3] = c.w;
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+          d[k * 4 + u] = x + u < count ? (FIRST ? (uint32_t)__ldg(hashes + base + x + u) : __ldg(codes + base + x + u)) : 0u;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kLargeItems; k++) {
+      const bool valid = ((k / 4) * kSortThreads + threadIdx.x) * 4u + (k & 3) < count;
+      hist_add(sh, FIRST ? d[k] : (d[k] >> shift) & (kBins - 1u), valid);
+    }
+    __syncthreads();
+    const uint2 c = *bins;
+    *bins = make_uint2(0u, 0u);
+    reinterpret_cast<uint2*>(rows + (size_t)tile * kBins)[threadIdx.x] = run;
+    run.x += c.x;
+    run.y += c.y;
+    __syncthreads();
+  }
+  reinterpret_cast<uint2*>(groups + (size_t)blockIdx.x * kBins)[threadIdx.x] = run;
+}
+
+// groups[g][bin] becomes the bin's count in the groups before g, totals[bin]
+// its count in all.  A block of 32 x 32 threads per 32 bins: lane = bin, each
+// warp a run of ten groups.
+__global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* __restrict__ groups, uint32_t* __restrict__ totals) {
+  constexpr uint32_t kPer = (kSortGroups + 31) / 32;
+  __shared__ uint32_t sSum[32][33];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint32_t* col = groups + blockIdx.x * 32u + lane;
+  uint32_t v[kPer], sum = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < kPer; k++) {
+    const uint32_t g = warp * kPer + k;
+    v[k] = g < kSortGroups ? col[(size_t)g * kBins] : 0u;
+  }
+#pragma unroll
+  for (uint32_t k = 0; k < kPer; k++) sum += v[k];
+  sSum[warp][lane] = sum;
+  __syncthreads();
+  uint32_t before = 0;
+  for (uint32_t w = 0; w < warp; w++) before += sSum[w][lane];
+#pragma unroll
+  for (uint32_t k = 0; k < kPer; k++) {
+    const uint32_t g = warp * kPer + k;
+    if (g < kSortGroups) col[(size_t)g * kBins] = before;
+    before += v[k];
+  }
+  if (warp == 31) totals[blockIdx.x * 32u + lane] = before;
+}
+
+struct SortPass {
+  const uint32_t* __restrict__ codesIn;
+  const uint16_t* __restrict__ hashes;
+  const uint32_t* __restrict__ valsIn;
+  uint32_t* __restrict__ codesOut;
+  uint32_t* __restrict__ valsOut;
+  unsigned long long n;
+  uint32_t shift;
+  const uint32_t* __restrict__ hist;  // the pass's digit counts
+  // the look-back's words and the tiles' counter
+  unsigned long long* status;
+  uint32_t* tileCounter;
+  int* err;
+  uint32_t spinLimit;
+  // COUNTED: the rows of k_sort_count and the groups of k_sort_scan (perGroup tiles each)
+  const uint32_t* __restrict__ rows;
+  const uint32_t* __restrict__ groups;
+  uint32_t perGroup;
+};
+
+// One tile; FULL: all of its entries exist (every tile but the last).
+template <int ITEMS, bool FIRST, bool COUNTED, bool FULL>
+__device__ __forceinline__ void sort_tile(const SortPass& a, uint32_t tile, uint32_t count, uint2 all) {
   constexpr uint32_t kTileItems = kSortThreads * ITEMS;
+  constexpr bool kMasks = !COUNTED;
   static_assert(kTileItems <= 1u << 16, "ranks and tile-local indexes of 16 bits");
   extern __shared__ __align__(16) unsigned char smem_sort[];
   uint32_t* sCodes = reinterpret_cast<uint32_t*>(smem_sort);
   uint32_t* sVals = sCodes + kTileItems;  // FIRST: digit << 16 | index in the tile
-  uint16_t* sHist = reinterpret_cast<uint16_t*>(sVals + kTileItems);
+  uint16_t* sHist = reinterpret_cast<uint16_t*>(smem_sort + sort_entry_bytes(ITEMS));
   uint32_t* sStart = reinterpret_cast<uint32_t*>(sHist + kSortWarps * kHistStride);
   int32_t* sDst = reinterpret_cast<int32_t*>(sStart + kBins);
-  __shared__ uint32_t sTile;
   __shared__ unsigned long long sWarpSum[kSortWarps];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) sTile = atomicAdd(tileCounter, 1u);
-  const uint2 all = __ldg(reinterpret_cast<const uint2*>(hist) + threadIdx.x);  // this thread's bins, whole input
   uint16_t* mine = sHist + warp * kHistStride;
-  for (uint32_t k = lane; k < kHistStride / 2; k += 32) reinterpret_cast<uint32_t*>(mine)[k] = 0u;
-  __syncthreads();
-  const uint32_t tile = sTile;
+  uint32_t* match = sCodes + warp * kBins;  // while the warps rank: per digit the lanes that have it
   const unsigned long long tileBase = (unsigned long long)tile * kTileItems;
-  const uint32_t count = (uint32_t)min((unsigned long long)kTileItems, n - tileBase);
+  const uint32_t* __restrict__ codesIn = a.codesIn + tileBase;
+  const uint32_t shift = a.shift;
   const uint32_t local = warp * (32u * ITEMS) + lane;  // + 32 k: this thread's entries in the tile
   unsigned lt;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
   uint32_t code[ITEMS];
-  uint32_t digit[ITEMS];  // FIRST only; then the digit's low half holds the rank
+  uint32_t digit[ITEMS];  // FIRST only; then digit << 16 | rank
 #pragma unroll
   for (int k = 0; k < ITEMS; k++) {
     const uint32_t x = local + 32u * k;
-    code[k] = x < count ? __ldcs(codesIn + tileBase + x) : 0u;
-    digit[k] = (FIRST && x < count) ? (uint32_t)__ldcs(hashes + tileBase + x) : 0u;
+    code[k] = FULL || x < count ? __ldcs(codesIn + x) : 0u;
+    digit[k] = FIRST && (FULL || x < count) ? (uint32_t)__ldcs(a.hashes + tileBase + x) : 0u;
   }
 #pragma unroll
   for (int k = 0; k < ITEMS; k++) {
-    const bool valid = local + 32u * k < count;
-    const uint32_t d = valid ? (FIRST ? digit[k] : (code[k] >> shift) & (kBins - 1u)) : kBins;
-    // the lanes with the same digit (and validity): one ballot per digit bit
-    unsigned peers = __ballot_sync(0xFFFFFFFFu, valid);
-    if (!valid) peers = ~peers;
+    const bool valid = FULL || local + 32u * k < count;
+    const uint32_t d = FIRST ? digit[k] : (code[k] >> shift) & (kBins - 1u);
+    unsigned peers;  // the lanes with the same digit
+    if (kMasks) {    // each sets its bit in the digit's mask
+      if (valid) atomicOr(match + d, 1u << lane);
+      __syncwarp();
+      peers = valid ? match[d] : 1u << lane;
+      __syncwarp();
+    } else {  // one ballot per digit bit
+      peers = FULL ? 0xFFFFFFFFu : __ballot_sync(0xFFFFFFFFu, valid);
+      if (!valid) peers = ~peers;
 #pragma unroll
-    for (int bit = 0; bit < kRadixBits; bit++) {
-      const unsigned on = __ballot_sync(0xFFFFFFFFu, (d >> bit) & 1u);
-      peers &= ((d >> bit) & 1u) ? on : ~on;
+      for (int bit = 0; bit < kRadixBits; bit++) {
+        const unsigned on = __ballot_sync(0xFFFFFFFFu, (d >> bit) & 1u);
+        peers &= ((d >> bit) & 1u) ? on : ~on;
+      }
     }
-    const int leader = __ffs(peers) - 1;
+    const int leader = 31 - __clz((int)peers);
     uint32_t old = 0;
-    if ((int)lane == leader) {
+    if ((int)lane == leader && valid) {
       old = mine[d];
       mine[d] = (uint16_t)(old + __popc(peers));
+      if (kMasks) match[d] = 0u;
     }
     old = __shfl_sync(0xFFFFFFFFu, old, leader);
     digit[k] = (d << 16) | (old + __popc(peers & lt));
-    __syncwarp();
+    if (!kMasks) __syncwarp();
   }
   __syncthreads();
   // Thread t owns bins 2t and 2t + 1: the warps' exclusive prefixes in place,
@@ -315,8 +394,8 @@ __global__ void __launch_bounds__(kSortThreads, 2)
     tot[0] += c & 0xFFFFu;
     tot[1] += c >> 16;
   }
-  unsigned long long* st = status + (size_t)tile * (kBins / 2) + threadIdx.x;
-  st_relaxed64(st, pair_word(tile == 0 ? kFlagPrefix : kFlagAggregate, tot[0], tot[1]));
+  unsigned long long* st = a.status + (size_t)tile * (kBins / 2) + threadIdx.x;
+  if (!COUNTED) st_relaxed64(st, pair_word(tile == 0 ? kFlagPrefix : kFlagAggregate, tot[0], tot[1]));
   // Exclusive scans over the bins: the tile's bin starts (low half) and the
   // whole input's (high half).
   uint32_t base0, base1;
@@ -338,6 +417,15 @@ __global__ void __launch_bounds__(kSortThreads, 2)
     base1 = base0 + all.x;
   }
   __syncthreads();
+  // Both bins' counts over the earlier tiles: counted before, or (below) by
+  // decoupled look-back.
+  uint32_t prefix0 = 0, prefix1 = 0;
+  if (COUNTED) {
+    const uint2 r = __ldg(reinterpret_cast<const uint2*>(a.rows + (size_t)tile * kBins) + threadIdx.x);
+    const uint2 g = __ldg(reinterpret_cast<const uint2*>(a.groups + (size_t)(tile / a.perGroup) * kBins) + threadIdx.x);
+    prefix0 = r.x + g.x;
+    prefix1 = r.y + g.y;
+  }
   // The tile in digit order in shared memory (before the look-back: it needs
   // only the tile's own counts).
   uint32_t val[ITEMS];
@@ -345,30 +433,28 @@ __global__ void __launch_bounds__(kSortThreads, 2)
   for (int k = 0; k < ITEMS; k++) {
     const uint32_t x = local + 32u * k;
     if (FIRST) val[k] = (digit[k] & 0xFFFF0000u) | x;
-    else val[k] = x < count ? __ldcs(valsIn + tileBase + x) : 0u;
+    else val[k] = FULL || x < count ? __ldcs(a.valsIn + tileBase + x) : 0u;
   }
 #pragma unroll
   for (int k = 0; k < ITEMS; k++) {
-    if (local + 32u * k < count) {
+    if (FULL || local + 32u * k < count) {
       const uint32_t d = digit[k] >> 16;
       const uint32_t pos = sStart[d] + mine[d] + (digit[k] & 0xFFFFu);
       sCodes[pos] = code[k];
       sVals[pos] = val[k];
     }
   }
-  // Decoupled look-back: both bins' counts over the earlier tiles.  The words
-  // of kLookback predecessors are loaded at once (independent loads), then
-  // summed nearest first up to the first inclusive prefix; a word not yet
-  // published stops the sum there and is polled again.
-  uint32_t prefix0 = 0, prefix1 = 0;
-  if (tile > 0) {
+  // The look-back.  The words of kLookback predecessors are loaded at once
+  // (independent loads), then summed nearest first up to the first inclusive
+  // prefix; a word not yet published stops the sum there and is polled again.
+  if (!COUNTED && tile > 0) {
     long long p = (long long)tile - 1;
     uint32_t spins = 0;
     while (p >= 0) {
       unsigned long long w[kLookback];
 #pragma unroll
       for (int k = 0; k < kLookback; k++)
-        w[k] = p - k >= 0 ? ld_relaxed64(status + (size_t)(p - k) * (kBins / 2) + threadIdx.x)
+        w[k] = p - k >= 0 ? ld_relaxed64(a.status + (size_t)(p - k) * (kBins / 2) + threadIdx.x)
                           : pair_word(kFlagPrefix, 0u, 0u);
       int used = 0;
       bool done = false, stalled = false;
@@ -388,8 +474,8 @@ __global__ void __launch_bounds__(kSortThreads, 2)
       if (done) break;
       p -= used;
       if (stalled) {
-        if (++spins > spinLimit) {
-          atomicCAS(err, 0, (int)PGA_ERR_TIMEOUT);
+        if (++spins > a.spinLimit) {
+          atomicCAS(a.err, 0, (int)PGA_ERR_TIMEOUT);
           break;
         }
         __nanosleep(32);
@@ -401,15 +487,41 @@ __global__ void __launch_bounds__(kSortThreads, 2)
   sDst[2u * threadIdx.x + 1] = (int32_t)(base1 + prefix1 - sStart[2u * threadIdx.x + 1]);
   __syncthreads();
   // Out: consecutive positions of one digit go to consecutive places.
-#pragma unroll 4
-  for (uint32_t p = threadIdx.x; p < count; p += kSortThreads) {
+#pragma unroll
+  for (int k = 0; k < ITEMS; k++) {
+    const uint32_t p = threadIdx.x + (uint32_t)k * kSortThreads;
+    if (!FULL && p >= count) break;
     const uint32_t c = sCodes[p], v = sVals[p];
     const uint32_t d = FIRST ? v >> 16 : (c >> shift) & (kBins - 1u);
     const uint32_t o = (uint32_t)sDst[d] + p;
-    if (o >= n) continue;  // only after a look-back that gave up
-    codesOut[o] = c;
-    valsOut[o] = FIRST ? (uint32_t)tileBase + (v & 0xFFFFu) : v;
+    if (!COUNTED && o >= a.n) continue;  // only after a look-back that gave up
+    a.codesOut[o] = c;
+    a.valsOut[o] = FIRST ? (uint32_t)tileBase + (v & 0xFFFFu) : v;
   }
+}
+
+template <int ITEMS, bool FIRST, bool COUNTED>
+__global__ void __launch_bounds__(kSortThreads, 2) k_sort_pass(SortPass a) {
+  constexpr uint32_t kTileItems = kSortThreads * ITEMS;
+  extern __shared__ __align__(16) unsigned char smem_sort[];
+  __shared__ uint32_t sTile;
+  if (!COUNTED && threadIdx.x == 0) sTile = atomicAdd(a.tileCounter, 1u);
+  const uint2 all = __ldg(reinterpret_cast<const uint2*>(a.hist) + threadIdx.x);  // this thread's bins, whole input
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  uint16_t* mine = reinterpret_cast<uint16_t*>(smem_sort + sort_entry_bytes(ITEMS)) + warp * kHistStride;
+  for (uint32_t k = lane; k < kBins / 8; k += 32) reinterpret_cast<uint4*>(mine)[k] = make_uint4(0u, 0u, 0u, 0u);
+  if (!COUNTED) {
+    uint32_t* match = reinterpret_cast<uint32_t*>(smem_sort) + warp * kBins;
+    for (uint32_t k = lane; k < kBins / 4; k += 32) reinterpret_cast<uint4*>(match)[k] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+  } else {
+    __syncwarp();  // the warp's histogram is clear
+  }
+  const uint32_t tile = COUNTED ? blockIdx.x : sTile;
+  const uint32_t count =
+      (uint32_t)min((unsigned long long)kTileItems, a.n - (unsigned long long)tile * kTileItems);
+  if (count == kTileItems) sort_tile<ITEMS, FIRST, COUNTED, true>(a, tile, count, all);
+  else sort_tile<ITEMS, FIRST, COUNTED, false>(a, tile, count, all);
 }
 
 __device__ __forceinline__ uint64_t term_path(const PgaTerminal* t, uint32_t i) {
@@ -1227,8 +1339,9 @@ __global__ void __launch_bounds__(kTile) k_join(TreeArgs a) {
 
 using namespace pga;
 
-// Sort scratch, zeroed by one memset per build: the digit histograms, the
-// passes' tile counters, the tree's arrival counters and the look-back words.
+// Sort scratch: the passes' digit counts and tile counters, the tree's arrival
+// counters, and the look-back words (all of it zeroed by one memset) or the
+// rows and groups of a counted pass (then only the arrival counters are).
 static unsigned long long sort_tiles(unsigned long long n) {
   const unsigned long long tile = (unsigned long long)kSortThreads * (n <= kSmallSort ? kSmallItems : kLargeItems);
   return (n + tile - 1) / tile;
@@ -1244,7 +1357,9 @@ static unsigned long long tree_joins(unsigned long long n) {
 }
 
 static size_t sort_words(unsigned long long n) {
-  return (size_t)(kSortPasses * kBins + 64 + tree_joins(n) + (unsigned long long)kSortPasses * sort_tiles(n) * kBins);
+  // small builds: the look-back words of each pass; large ones: the tiles' rows and the groups of one
+  return (size_t)(kSortPasses * kBins + 64 + tree_joins(n) +
+                  (n <= kSmallSort ? kSortPasses * sort_tiles(n) : sort_tiles(n) + kSortGroups) * kBins);
 }
 
 extern "C" size_t pga_lbvh_temp_bytes(uint64_t n) {
@@ -1276,32 +1391,54 @@ struct LbvhScratch {
 // Polls of a look-back wait before it gives up (each followed by a 32 ns sleep).
 constexpr uint32_t kSortSpinLimit = 1u << 22;
 
-template <int ITEMS>
-static PgaStatus launch_sort(unsigned long long n, uint32_t* codesA, uint32_t* codesB, const uint16_t* hashes,
-                             uint32_t* valsA, uint32_t* valsB, const uint32_t* hist, uint32_t* counters,
-                             unsigned long long* words, int* err, cudaStream_t s) {
+struct SortBuffers {
+  uint32_t *codesA, *codesB;
+  const uint16_t* hashes;
+  uint32_t *valsA, *valsB;
+  uint32_t* hist;      // digit counts of the passes
+  uint32_t* counters;  // tile counters (small)
+  uint32_t* words;     // look-back words of the passes (small), or rows and groups of one (large)
+  int* err;
+};
+
+// Pass q of the sort: from the A arrays to the B arrays and back in turn.
+template <bool SMALL, bool FIRST>
+static PgaStatus launch_sort_pass(int q, unsigned long long n, const SortBuffers& b, cudaStream_t s) {
+  constexpr int kItems = SMALL ? kSmallItems : kLargeItems;
+  constexpr size_t smem = sort_pass_smem(kItems);
+  const auto kernel = k_sort_pass<kItems, FIRST, !SMALL>;
   const unsigned tiles = (unsigned)sort_tiles(n);
-  constexpr size_t smem = onesweep_smem(ITEMS);
-  PGA_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<ITEMS, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  PGA_CUDA_TRY(cudaFuncSetAttribute(k_onesweep<ITEMS, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  for (int q = 0; q < kSortPasses; q++) {
-    const bool even = q % 2 == 0;
-    const uint32_t* cIn = even ? codesA : codesB;
-    uint32_t* cOut = even ? codesB : codesA;
-    const uint32_t* vIn = even ? valsA : valsB;
-    uint32_t* vOut = even ? valsB : valsA;
-    unsigned long long* w = words + (size_t)q * tiles * (kBins / 2);
-    if (q == 0)
-      k_onesweep<ITEMS, true><<<tiles, kSortThreads, smem, s>>>(cIn, hashes, nullptr, cOut, vOut, n, 0u, hist, w,
-                                                                 counters, err, kSortSpinLimit);
-    else
-      k_onesweep<ITEMS, false><<<tiles, kSortThreads, smem, s>>>(cIn, nullptr, vIn, cOut, vOut, n,
-                                                                  (uint32_t)((q - 1) * kRadixBits), hist + q * kBins, w,
-                                                                  counters + q, err, kSortSpinLimit);
+  const uint32_t shift = FIRST ? 0u : (uint32_t)((q - 1) * kRadixBits);
+  const bool even = q % 2 == 0;
+  const uint32_t* cIn = even ? b.codesA : b.codesB;
+  uint32_t* cOut = even ? b.codesB : b.codesA;
+  const uint32_t* vIn = even ? b.valsA : b.valsB;
+  uint32_t* vOut = even ? b.valsB : b.valsA;
+  uint32_t* hist = b.hist + q * kBins;
+  uint32_t* rows = b.words;
+  uint32_t* groups = rows + (size_t)tiles * kBins;
+  const uint32_t perGroup = (tiles + kSortGroups - 1) / kSortGroups;
+  if (!SMALL) {
+    k_sort_count<FIRST><<<kSortGroups, kSortThreads, 0, s>>>(cIn, b.hashes, n, shift, tiles, perGroup, rows, groups);
+    PGA_CUDA_TRY(cudaGetLastError());
+    k_sort_scan<<<kBins / 32, 1024, 0, s>>>(groups, hist);
     PGA_CUDA_TRY(cudaGetLastError());
   }
-  static_assert(kSortPasses % 2 == 0, "an even number of passes ends in codesA and valsA");
+  PGA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const SortPass a{cIn, b.hashes, vIn, cOut, vOut, n, shift, hist,
+                   reinterpret_cast<unsigned long long*>(b.words) + (SMALL ? (size_t)q * tiles * (kBins / 2) : 0),
+                   b.counters + q, b.err, kSortSpinLimit, rows, groups, perGroup};
+  kernel<<<tiles, kSortThreads, smem, s>>>(a);
+  PGA_CUDA_TRY(cudaGetLastError());
   return PGA_OK;
+}
+
+template <bool SMALL>
+static PgaStatus launch_sort(unsigned long long n, const SortBuffers& b, cudaStream_t s) {
+  PgaStatus st = launch_sort_pass<SMALL, true>(0, n, b, s);
+  for (int q = 1; q < kSortPasses && st == PGA_OK; q++) st = launch_sort_pass<SMALL, false>(q, n, b, s);
+  static_assert(kSortPasses % 2 == 0, "an even number of passes ends in the A arrays");
+  return st;
 }
 
 // The launches of a build over `cap` leaves, or over min(*dN, cap) when dN is
@@ -1323,27 +1460,26 @@ static PgaStatus launch_lbvh(const PgaTerminal* t, unsigned long long cap, const
   uint32_t* hist = static_cast<uint32_t*>(w.sortTemp);
   uint32_t* counters = hist + kSortPasses * kBins;
   uint32_t* joins = counters + 64;
-  unsigned long long* words = reinterpret_cast<unsigned long long*>(joins + tree_joins(cap));
-  PGA_CUDA_TRY(cudaMemsetAsync(hist, 0, sort_words(cap) * sizeof(uint32_t), s));
+  const bool small = cap <= kSmallSort;
+  uint32_t* words = joins + tree_joins(cap);
+  // large builds read none of hist, counters and words before writing them
+  uint32_t* clear = small ? hist : joins;
+  const size_t clearWords = small ? sort_words(cap) : tree_joins(cap);
+  PGA_CUDA_TRY(cudaMemsetAsync(clear, 0, clearWords * sizeof(uint32_t), s));
   uint32_t* codesA = reinterpret_cast<uint32_t*>(w.keysA);
-  uint32_t* codesB = codesA + cap;
   uint16_t* hashes = reinterpret_cast<uint16_t*>(out->keys);
+  const SortBuffers sort{codesA, codesA + ((cap + 3) & ~3ull), hashes, w.valsA, w.valsB, hist, counters, words, w.err};
   const unsigned blocks = (unsigned)((cap + kLbvhThreads - 1) / kLbvhThreads);
   PgaStatus st;
-  if (cap <= kSmallSort) {
+  if (small) {
     k_morton<true><<<(unsigned)((cap + kHistThreads - 1) / kHistThreads), kHistThreads, 0, s>>>(t, cap, dN, b, codesA,
                                                                                               hashes, hist);
     PGA_CUDA_TRY(cudaGetLastError());
-    st = launch_sort<kSmallItems>(cap, codesA, codesB, hashes, w.valsA, w.valsB, hist, counters, words, w.err, s);
+    st = launch_sort<true>(cap, sort, s);
   } else {
     k_morton<false><<<blocks, kLbvhThreads, 0, s>>>(t, cap, dN, b, codesA, hashes, hist);
     PGA_CUDA_TRY(cudaGetLastError());
-    int dev = 0, sms = 0;
-    PGA_CUDA_TRY(cudaGetDevice(&dev));
-    PGA_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    k_digit_hist<<<(unsigned)sms * 4, kHistThreads, 0, s>>>(codesA, hashes, cap, hist);
-    PGA_CUDA_TRY(cudaGetLastError());
-    st = launch_sort<kLargeItems>(cap, codesA, codesB, hashes, w.valsA, w.valsB, hist, counters, words, w.err, s);
+    st = launch_sort<false>(cap, sort, s);
   }
   if (st != PGA_OK) return st;
   OpenTree* open = static_cast<OpenTree*>(w.open);

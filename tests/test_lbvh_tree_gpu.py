@@ -1,7 +1,7 @@
 """The LBVH's bottom-up tree kernel at the sizes where its tiles (256 leaves),
 their windows (32 keys either side) and their groups (32 tiles, then 32
 groups) begin and end, and on tie runs inside a tile, over a tile's end and
-longer than a tile; bit for bit against the restatement, as the other LBVH
+longer than a tile, and either side of the sort's two forms; bit for bit against the restatement, as the other LBVH
 tests are."""
 import numpy as np
 import pytest
@@ -38,7 +38,9 @@ SIZES = [2, 3, 31, 33, 255, 256, 257, 288, 289, 512, 513, 8191, 8192, 8193, 3001
 
 
 @pytest.mark.parametrize("n,ties", [(n, t) for n in SIZES for t in ("none", "short", "equal")]
-                         + [(262144, "none"), (262145, "short"), (290017, "equal"), (90001, "long")])
+                         + [(262144, "none"), (262145, "short"), (290017, "equal"), (90001, "long")]
+                         # the sort's small and large forms, and a large one with more tiles than counting groups
+                         + [(622592, "short"), (622593, "none"), (2500001, "short")])
 def test_tree_bit_exact(n, ties):
     torch = pytest.importorskip("torch")
     if not torch.cuda.is_available():
