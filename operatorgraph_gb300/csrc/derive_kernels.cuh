@@ -28,6 +28,14 @@ struct __align__(16) Smem {
   const DevRule* rules;
   const DevParam* params;
   const int32_t* succ;
+  // The level being expanded (paged engine; thread 0 moves them on in level_barrier).
+  unsigned long long levelBase;  // first item slot of the next level: where this level's children go
+  uint32_t turn;                 // which of DevState's per-level sets this level uses
+  uint32_t taken;                // item slots this block has taken for the next level
+  uint32_t shareShift;            // 2^shareShift warps share a chunk of items
+  int32_t seen;                  // DevState::status, read while the level was expanded
+  int32_t stop;                  // some block had seen a status by the end of the level before
+  unsigned long long maxItems;   // of a level (block 0)
 };
 
 extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -955,19 +963,20 @@ __device__ __forceinline__ void store_terminal(const DeriveArgs& a, PgaTerminal*
 // marked empty); the warps' last terminal pages leave holes that a compaction
 // at the end of the launch fills, so the output is dense.
 constexpr uint32_t kTermPage = 256;
-constexpr uint32_t kNodePage = 64;
+constexpr uint32_t kNodePage = 64;  // kNodePage >> shareShift on a narrow level (see expand_level)
 constexpr uint32_t kEmptyItem = 0xFFFFFFFFu;
 
 struct WarpOut {
-  unsigned long long tPage, nPage;
-  uint32_t tFill, nFill;  // slots used in the current page (page size when there is none)
+  unsigned long long tPage, nNext;  // terminal page; next free slot of the item page
+  uint32_t tFill, nLeft;  // slots used in the terminal page (page size when there is none); slots left of the item page
   uint32_t sub;           // children per queued work item for the level being expanded
 };
 
 __device__ __forceinline__ void warpout_init(const DeriveArgs& a, WarpOut& w) {
-  w.tPage = w.nPage = ~0ull;
+  w.tPage = ~0ull;
+  w.nNext = 0;
   w.tFill = kTermPage;
-  w.nFill = kNodePage;
+  w.nLeft = 0;
   w.sub = a.subItem;
 }
 
@@ -984,23 +993,46 @@ struct Span {
   uint32_t rem;
 };
 
-__device__ __forceinline__ Span page_reserve(unsigned long long* counter, uint32_t pageSize,
-                                             unsigned long long& page, uint32_t& fill, uint32_t cnt) {
+__device__ __forceinline__ Span term_reserve(const DeriveArgs& a, WarpOut& w, uint32_t cnt) {
   Span sp;
-  sp.rem = min(pageSize - fill, cnt);
-  sp.first = page * pageSize + fill;
+  sp.rem = min(kTermPage - w.tFill, cnt);
+  sp.first = w.tPage * kTermPage + w.tFill;
   sp.next = 0;
   if (cnt > sp.rem) {
     const uint32_t need = cnt - sp.rem;
-    const uint32_t np = (need + pageSize - 1) / pageSize;
+    const uint32_t np = (need + kTermPage - 1) / kTermPage;
     unsigned long long p0 = 0;
-    if ((threadIdx.x & 31u) == 0) p0 = atomicAdd(counter, (unsigned long long)np);
+    if ((threadIdx.x & 31u) == 0) p0 = atomicAdd(&a.st->termPages, (unsigned long long)np);
     p0 = __shfl_sync(kFull, p0, 0);
-    sp.next = p0 * pageSize;
-    page = p0 + np - 1;
-    fill = need - (np - 1) * pageSize;
+    sp.next = p0 * kTermPage;
+    w.tPage = p0 + np - 1;
+    w.tFill = need - (np - 1) * kTermPage;
   } else {
-    fill += cnt;
+    w.tFill += cnt;
+  }
+  return sp;
+}
+
+__device__ __forceinline__ Span node_reserve(const DeriveArgs& a, WarpOut& w, uint32_t cnt) {
+  Span sp;
+  sp.rem = min(w.nLeft, cnt);
+  sp.first = w.nNext;
+  sp.next = 0;
+  if (cnt > sp.rem) {
+    Smem& sm = block_smem();
+    const uint32_t need = cnt - sp.rem, page = kNodePage >> sm.shareShift;
+    const uint32_t grab = (need + page - 1) & ~(page - 1);
+    unsigned long long p0 = 0;
+    if ((threadIdx.x & 31u) == 0) {
+      atomicAdd(&sm.taken, grab);
+      p0 = sm.levelBase + atomicAdd(&a.st->levelSlots[sm.turn], (unsigned long long)grab);
+    }
+    sp.next = __shfl_sync(kFull, p0, 0);
+    w.nNext = sp.next + need;
+    w.nLeft = grab - need;
+  } else {
+    w.nNext += cnt;
+    w.nLeft -= cnt;
   }
   return sp;
 }
@@ -1034,7 +1066,7 @@ __device__ __forceinline__ void emit_round(const DeriveArgs& a, WarpOut& w, int 
     const uint32_t cnt = __popc(tm), rank = __popc(tm & lanemask_lt());
     unsigned long long slot;
     if (PAGED) {
-      const Span sp = page_reserve(&a.st->termPages, kTermPage, w.tPage, w.tFill, cnt);
+      const Span sp = term_reserve(a, w, cnt);
       slot = span_slot(sp, rank);
     } else {
       unsigned long long base = 0;
@@ -1052,7 +1084,7 @@ __device__ __forceinline__ void emit_round(const DeriveArgs& a, WarpOut& w, int 
     const uint32_t pre = warp_excl_scan(m, total);
     Span sp;
     if (PAGED) {
-      sp = page_reserve(&a.st->nodePages, kNodePage, w.nPage, w.nFill, total);
+      sp = node_reserve(a, w, total);
     } else {
       unsigned long long base = 0;
       if (lane == 0) base = atomicAdd(&a.st->nodeNext, (unsigned long long)total);
@@ -1076,15 +1108,21 @@ __device__ __forceinline__ void emit_round(const DeriveArgs& a, WarpOut& w, int 
 // out during this one).
 __device__ __forceinline__ void close_node_page(const DeriveArgs& a, WarpOut& w) {
   const unsigned lane = threadIdx.x & 31u;
-  if (w.nPage != ~0ull) {
-    for (uint32_t k = w.nFill + lane; k < kNodePage; k += 32) {
-      const unsigned long long slot = w.nPage * kNodePage + k;
-      if (slot < a.nodeCap)
-        __stcg(reinterpret_cast<uint4*>(a.nodes + slot) + 3, make_uint4(kEmptyItem, 0u, 0u, 0u));
-    }
+  for (uint32_t k = lane; k < w.nLeft; k += 32) {
+    const unsigned long long slot = w.nNext + k;
+    if (slot < a.nodeCap)
+      __stcg(reinterpret_cast<uint4*>(a.nodes + slot) + 3, make_uint4(kEmptyItem, 0u, 0u, 0u));
   }
-  w.nPage = ~0ull;
-  w.nFill = kNodePage;
+  w.nLeft = 0;
+}
+
+// The warp's terminal page as it stands (page << 9 | fill, or ~0 when it is
+// full), for the compaction: stored ahead of every level's end, so that the
+// barrier that ends the last level is the compaction's too.
+__device__ __forceinline__ void publish_term_page(const DeriveArgs& a, const WarpOut& w) {
+  const unsigned long long gw = ((unsigned long long)blockIdx.x * kThreads + threadIdx.x) >> 5;
+  if ((threadIdx.x & 31u) == 0 && gw < a.numWarps)
+    a.scratch[gw] = (w.tPage != ~0ull && w.tFill < kTermPage) ? (w.tPage << 9) | w.tFill : ~0ull;
 }
 
 // Emits a new child per lane (kind from resolve); a branching child is queued
@@ -1173,10 +1211,11 @@ __device__ __forceinline__ void axiom_shape(const DeriveArgs& a, uint32_t i, Sha
   x.path = mix64((uint64_t)i + 0x9E3779B97F4A7C15ULL);
 }
 
-// Expands the work items first + 32 k + lane (k < K, item < hi) of one warp.
+// Expands the work items first + 32 k + lane (k < K, item < hi) of one warp;
+// with shift > 0, run number `part` of 2^shift of their children.
 template <bool PAGED, bool LEAF, int AFF>
 __device__ __forceinline__ void warp_items(const DeriveArgs& a, WarpOut& w, unsigned long long first,
-                                           unsigned long long hi, uint32_t K) {
+                                           unsigned long long hi, uint32_t K, uint32_t shift, uint32_t part) {
   const unsigned lane = threadIdx.x & 31u;
   for (uint32_t k = 0; k < K; k++) {
     const unsigned long long item = first + 32ull * k + lane;
@@ -1200,8 +1239,14 @@ __device__ __forceinline__ void warp_items(const DeriveArgs& a, WarpOut& w, unsi
         const uint32_t c1 = min(ext.y, all);
         c0 = ext.x;
         if (c0 < c1) {
-          expander_skip(a, E, c0);
           n = c1 - c0;
+          if (shift > 0) {
+            const uint32_t run = (n + (1u << shift) - 1u) >> shift;
+            const uint32_t skip = part * run;
+            c0 += skip;
+            n = skip < n ? min(run, n - skip) : 0u;
+          }
+          if (n > 0) expander_skip(a, E, c0);
         }
       }
     }
@@ -1286,17 +1331,39 @@ __device__ void seed_deferred(const DeriveArgs& a, WarpOut& w) {
 // allocation): on a level of at least four rounds of chunks the static order
 // covers whole rounds up to the last quarter of the level (at least two
 // rounds of chunks are left); warps then take the rest one chunk at a time
-// from the level's cursor, which the level snapshot set to lo.
+// from the level's cursor.
+//
+// A level with at most half as many items as the grid has threads is narrow:
+// 2, 4 or 8 warps (2^shift, as many as there are without a warp taking a second
+// chunk) share a chunk of 32 items, each producing a run of the items'
+// children, since an item's children, produced one after another, are what
+// such a level waits for.  Warps and not neighbouring lanes share them, so that
+// a warp's lanes still produce the same child of their items and emit shapes
+// of one rule side by side: with lanes, the mixed rules of the next levels'
+// warps cost the 8,192-axiom mix 6%.  A building's levels took 14 to 30 us
+// unshared and take 6 to 8 (derivation of 61 buildings 97 -> 40 us, 1,024
+// facades 98 -> 65, 4,096 buildings 264 -> 237).  The warps take item pages of
+// kNodePage >> shift slots, so that the slots left empty at the level's end are
+// as few as with one warp a chunk.
+__device__ __forceinline__ uint32_t share_shift(unsigned long long items) {
+  const unsigned long long threads = (unsigned long long)gridDim.x * kThreads;
+  uint32_t shift = 0;
+  while (shift < 3 && (items << (shift + 1)) <= threads) shift++;
+  return shift;
+}
+
 template <bool PAGED, bool LEAF, int AFF, bool DYN = false>
 __device__ __forceinline__ void expand_level(const DeriveArgs& a, WarpOut& w, unsigned long long lo,
-                                             unsigned long long hi, uint32_t K) {
+                                             unsigned long long hi, uint32_t K, uint32_t shift) {
   const unsigned long long warpId = ((unsigned long long)blockIdx.x * kThreads + threadIdx.x) >> 5;
   const unsigned long long numWarps = ((unsigned long long)gridDim.x * kThreads) >> 5;
+  if (shift > 0) K = 1;
+  const unsigned long long chunk = 32ull * K, stride = (numWarps >> shift) * chunk;
+  const uint32_t part = (uint32_t)warpId & ((1u << shift) - 1u);
   if constexpr (!DYN) {
-    for (unsigned long long b = lo + warpId * 32ull * K; b < hi; b += numWarps * 32ull * K)
-      warp_items<PAGED, LEAF, AFF>(a, w, b, hi, K);
+    for (unsigned long long b = lo + (warpId >> shift) * chunk; b < hi; b += stride)
+      warp_items<PAGED, LEAF, AFF>(a, w, b, hi, K, shift, part);
   } else {
-    const unsigned long long chunk = 32ull * K, stride = numWarps * chunk;
     unsigned long long dynLo = hi;  // items from dynLo on come from the cursor
     if (hi - lo >= 4 * stride) {
       const unsigned long long n = hi - lo, rest = max(n / PGA_DERIVE_DYNAMIC_SHARE, 2 * stride);
@@ -1304,15 +1371,15 @@ __device__ __forceinline__ void expand_level(const DeriveArgs& a, WarpOut& w, un
     }
     // one call site of warp_items for both orders (a second inlined copy costs
     // the kernel its register allocation)
-    for (unsigned long long b = lo + warpId * chunk;; b += stride) {
+    for (unsigned long long b = lo + (warpId >> shift) * chunk;; b += stride) {
       if (b >= dynLo) {
         if (dynLo >= hi) break;
         unsigned long long c = 0;
-        if ((threadIdx.x & 31u) == 0) c = atomicAdd(&a.st->cursor, chunk);
-        b = dynLo + (__shfl_sync(kFull, c, 0) - lo);  // the loop step never lands below dynLo again
+        if ((threadIdx.x & 31u) == 0) c = atomicAdd(&a.st->levelCursor[block_smem().turn], chunk);
+        b = dynLo + __shfl_sync(kFull, c, 0);  // the loop step never lands below dynLo again
         if (b >= hi) break;
       }
-      warp_items<PAGED, LEAF, AFF>(a, w, b, hi, K);
+      warp_items<PAGED, LEAF, AFF>(a, w, b, hi, K, shift, part);
     }
   }
 }
@@ -1321,6 +1388,12 @@ __device__ __forceinline__ void expand_level(const DeriveArgs& a, WarpOut& w, un
 // creation, which sized the dynamic shared memory for it) and fixes the block's
 // table pointers.
 __device__ __forceinline__ void setup_block(const DeriveArgs& a, Smem& sm) {
+  if (threadIdx.x == 0) {
+    sm.levelBase = 0;
+    sm.turn = sm.taken = sm.shareShift = 0;
+    sm.seen = sm.stop = 0;
+    sm.maxItems = 0;
+  }
   uint32_t dynBytes;
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynBytes));
   const size_t tableBytes = (size_t)a.tab.numEntries * sizeof(DevRule) + (size_t)a.numParams * sizeof(DevParam) +
@@ -1383,31 +1456,77 @@ __device__ bool grid_barrier(const DeriveArgs& a, Leader leader) {
   return ok != 0;
 }
 
-__device__ __forceinline__ void level_snapshot(const DeriveArgs& a, uint32_t level) {
+// The end of a level: every block adds its arrival, whether it had seen a
+// raised status, and the item slots it took to one word, and goes on when all
+// blocks' arrivals are in it.  The word then holds what each block needs to
+// know of the next level (its size, whether to stop), the same for all, so no
+// block has to set the level up for the others: with a leader that did, a
+// level of the Menger sponge (24 items) took 7-8 us, now 5.  The words, like the slot counters and cursors, are three in turn:
+// when a barrier is passed, every block has read the word of the one before,
+// and block 0 clears that set for the level after next (end_level).  Waits are
+// bounded by spinLimit; a timeout raises PGA_ERR_TIMEOUT and makes the caller
+// leave the kernel.
+constexpr uint32_t kArriveBits = 16;  // word: arrivals | blocks that saw a status << 16 | slots << 32
+__device__ bool level_barrier(const DeriveArgs& a, Smem& sm) {
+  __shared__ int ok;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    DevState* st = a.st;
+    unsigned long long* word = &st->levelWord[sm.turn];
+    const unsigned long long mine =
+        1ull | (sm.seen != 0 ? 1ull << kArriveBits : 0ull) | ((unsigned long long)sm.taken << 32);
+    __threadfence();
+    atomicAdd(word, mine);
+    unsigned long long seen;
+    uint32_t spins = 0;
+    int good = 1;
+    for (;;) {
+      // relaxed: an acquire would empty the L1 of the SM's other block, still at
+      // work, at every poll (16,384 trees tested for collisions: 107 -> 188 us)
+      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(word) : "memory");
+      if ((seen & ((1u << kArriveBits) - 1u)) == gridDim.x) break;
+      if (++spins > a.spinLimit) {
+        raise_error(st, PGA_ERR_TIMEOUT, -1);
+        good = 0;
+        break;
+      }
+      __nanosleep(32);
+    }
+    __threadfence();
+    const unsigned long long lo = min(sm.levelBase, a.nodeCap);
+    sm.levelBase += seen >> 32;
+    const unsigned long long hi = min(sm.levelBase, a.nodeCap);
+    sm.shareShift = hi > lo ? share_shift(hi - lo) : 0u;
+    sm.turn = sm.turn == 2 ? 0u : sm.turn + 1u;
+    sm.taken = 0;
+    sm.stop = ((seen >> kArriveBits) & 0xFFFFull) != 0 ? 1 : 0;
+    ok = good;
+  }
+  __syncthreads();
+  return ok != 0;
+}
+
+// What the host and the adjoint read of a level, and the clearing of the set
+// that the level after next uses: block 0, after the barrier that ended level
+// `level` (0: the seeding) and fixed the range [lo, hi) of the next.
+__device__ __forceinline__ void end_level(const DeriveArgs& a, Smem& sm, uint32_t level, unsigned long long lo,
+                                          unsigned long long hi) {
   DevState* st = a.st;
-  volatile DevState* vs = st;
-  unsigned long long lo = vs->levelHi;
-  unsigned long long hi = atomicAdd(&st->nodePages, 0ull) * kNodePage;
-  if (hi > a.nodeCap) hi = a.nodeCap;
-  vs->nodeNext = hi;
-  vs->levelLo = lo;
-  vs->levelHi = hi;
-  vs->cursor = lo;
+  const uint32_t after = sm.turn == 2 ? 0u : sm.turn + 1u;
+  st->levelSlots[after] = 0;
+  st->levelCursor[after] = 0;
+  st->levelWord[after] = 0;
+  st->nodeNext = hi;
+  st->levels = level;
+  if (level == 0) a.levelStart[0] = 0;
   if (level + 1 <= a.maxLevels) {
     a.levelStart[level + 1] = hi;
     unsigned long long now;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
     a.levelClock[level] = now;
   }
-  unsigned long long sz = hi - lo;
-  if (sz > vs->maxLevelNodes) vs->maxLevelNodes = sz;
-  bool more = hi > lo;
-  if (more && level >= a.maxLevels) {
-    raise_error(st, PGA_ERR_DEPTH, (int)level);
-    more = false;
-  }
-  vs->levels = level;
-  vs->stop = (!more || vs->status != 0) ? 1u : 0u;
+  sm.maxItems = max(sm.maxItems, hi - lo);
+  st->maxLevelNodes = sm.maxItems;
 }
 
 // Exclusive prefix sum of x[0, n) in place (shared memory, whole block);
@@ -1451,19 +1570,21 @@ __host__ __device__ constexpr size_t compact_smem_bytes(uint32_t W) {
 // many; the k-th hole (warps in index order) receives the k-th such record
 // (positions in increasing order).  Only the pages from the one holding N to
 // the last can hold records >= N: fewer than W + 1 pages, all full except the
-// partial pages among them.  After one grid barrier every block rebuilds both
+// partial pages among them.  Every block rebuilds both
 // enumerations in shared memory from the W published partial pages (no sort,
 // no further barrier) and moves its share of the records.
-__device__ void compact_terminals(const DeriveArgs& a, WarpOut& w) {
+__device__ void compact_terminals(const DeriveArgs& a) {
   const unsigned lane = threadIdx.x & 31u;
   const uint32_t W = a.numWarps;
-  const unsigned long long gw = ((unsigned long long)blockIdx.x * kThreads + threadIdx.x) >> 5;
-  unsigned long long* part = a.scratch;  // W entries: page << 9 | fill, or ~0
+  const unsigned long long* part = a.scratch;  // publish_term_page
   DevState* st = a.st;
-  unsigned long long mine = ~0ull;
-  if (w.tPage != ~0ull && w.tFill < kTermPage) mine = (w.tPage << 9) | w.tFill;
-  if (lane == 0 && gw < W) part[gw] = mine;
-  if (!grid_barrier(a, [] {})) return;
+  // read ahead of the scans (thread 0 decides for the block below)
+  unsigned long long pagesOut = 0;
+  int status = 0;
+  if (threadIdx.x == 0) {
+    pagesOut = ((volatile DevState*)st)->termPages;
+    status = ((volatile DevState*)st)->status;
+  }
   uint32_t dynBytes;  // the same in every thread of the launch
   asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dynBytes));
   if (dynBytes < compact_smem_bytes(W)) {
@@ -1492,11 +1613,10 @@ __device__ void compact_terminals(const DeriveArgs& a, WarpOut& w) {
   __shared__ unsigned long long blockPages;
   __shared__ int blockGo;
   if (threadIdx.x == 0) {
-    volatile DevState* vs = st;
-    const unsigned long long G = vs->termPages;
+    const unsigned long long G = pagesOut;
     const unsigned long long N = G * kTermPage - holes;
-    if (blockIdx.x == 0) vs->termCount = N;
-    int go = (vs->status == 0 && N <= a.cap && holes != 0) ? 1 : 0;
+    if (blockIdx.x == 0) st->termCount = N;
+    int go = (status == 0 && N <= a.cap && holes != 0) ? 1 : 0;
     // G * kTermPage - N = holes < W * kTermPage, so at most W + 1 pages hold records >= N.
     if (go && (G <= N / kTermPage || G - N / kTermPage > W + 1)) {
       raise_error(st, PGA_ERR_INTERNAL, 11);
@@ -1593,24 +1713,25 @@ __global__ void __launch_bounds__(kThreads, PGA_PERSISTENT_MIN_BLOCKS) k_derive_
     warpout_level(a, w, a.numAxioms - a.axiomBase);
     seed_axioms<true, LEAF, AFF>(a, w, a.axiomBase, a.numAxioms - a.axiomBase);
   }
-  close_node_page(a, w);
-  if (!grid_barrier(a, [&] {
-        volatile DevState* vs = a.st;
-        vs->levelHi = 0;
-        a.levelStart[0] = 0;
-        level_snapshot(a, 0);
-      }))
-    return;
+  unsigned long long hi = 0;
   for (uint32_t level = 0;; level++) {
-    volatile DevState* vs = a.st;
-    if (vs->stop) break;
-    const unsigned long long lo = vs->levelLo, hi = vs->levelHi;
-    warpout_level(a, w, hi - lo);
-    expand_level<true, LEAF, AFF, DYN>(a, w, lo, hi, a.itemsPerLane);
     close_node_page(a, w);
-    if (!grid_barrier(a, [&] { level_snapshot(a, level + 1); })) return;
+    publish_term_page(a, w);
+    if (!level_barrier(a, sm)) return;
+    const unsigned long long lo = hi;
+    hi = min(sm.levelBase, a.nodeCap);
+    const bool deep = hi > lo && level >= a.maxLevels;  // the same for all blocks, like all of this
+    const bool stop = hi <= lo || sm.stop != 0 || deep;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      end_level(a, sm, level, lo, hi);
+      if (deep) raise_error(a.st, PGA_ERR_DEPTH, (int)level);
+    }
+    if (stop) break;
+    if (threadIdx.x == 32) sm.seen = ((volatile DevState*)a.st)->status;  // counted at the level's end
+    warpout_level(a, w, hi - lo);
+    expand_level<true, LEAF, AFF, DYN>(a, w, lo, hi, a.itemsPerLane, sm.shareShift);
   }
-  compact_terminals(a, w);
+  compact_terminals(a);
   if (blockIdx.x == 0 && threadIdx.x == 0 && a.outCount != nullptr) *a.outCount = ((volatile DevState*)a.st)->termCount;
   __syncthreads();
   if (threadIdx.x == 0) atomicMax(&a.st->clockEnd, global_ns());
@@ -1630,7 +1751,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_expand_level(DeriveArgs a, unsi
   setup_block(a, sm);
   WarpOut w;
   warpout_init(a, w);
-  expand_level<false, false, 1>(a, w, lo, hi, 1);
+  expand_level<false, false, 1>(a, w, lo, hi, 1, 0);
 }
 
 __global__ void k_write_count(const DevState* st, unsigned long long* out) { *out = st->termCount; }

@@ -101,15 +101,17 @@ struct __align__(16) Node {
 
 struct DevState {
   unsigned long long termCount;   // terminals emitted (exact, after compaction in the paged engine)
-  unsigned long long nodeNext;    // queued item slots handed out (plain form)
+  unsigned long long nodeNext;    // queued item slots handed out
   unsigned long long termPages;   // terminal pages handed out (paged engine)
-  unsigned long long nodePages;   // item pages handed out (paged engine)
-  unsigned long long cursor;      // next dynamic chunk of the level being expanded (PGA_FLAG_DYNAMIC_CHUNKS)
-  unsigned long long levelLo, levelHi;
+  unsigned long long cursor;      // next dynamic chunk of the level the adjoint is sweeping
   unsigned long long maxLevelNodes;
   int32_t status, detail;
   uint32_t barrierArrive, barrierGen;
-  uint32_t levels, stop;
+  uint32_t levels, reserved;
+  // Paged engine, one set per level in turn (see level_barrier): item slots
+  // handed out while it is expanded, its next dynamic chunk
+  // (PGA_FLAG_DYNAMIC_CHUNKS), and the arrivals at its end.
+  unsigned long long levelSlots[3], levelCursor[3], levelWord[3];
   unsigned long long clockStart;  // %globaltimer when block 0 started (paged engine)
   unsigned long long clockEnd;    // %globaltimer when the last block finished
 };
