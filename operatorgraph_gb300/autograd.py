@@ -48,8 +48,9 @@ class _Derive(torch.autograd.Function):
     def backward(ctx, gM, gPaths):
         eng = ctx.engine
         gM = gM.contiguous().to(torch.float32)
-        g_blocks = torch.zeros(max(ctx.num_blocks * eng.block_stride, 1), dtype=torch.float32, device=gM.device)
-        g_sizes = torch.zeros((ctx.num_axioms, 3), dtype=torch.float32, device=gM.device)
+        # pga_adjoint overwrites both
+        g_blocks = torch.empty(max(ctx.num_blocks * eng.block_stride, 1), dtype=torch.float32, device=gM.device)
+        g_sizes = torch.empty((ctx.num_axioms, 3), dtype=torch.float32, device=gM.device)
         eng.adjoint_raw(gM.data_ptr(), g_blocks.data_ptr() if ctx.has_blocks else None, ctx.num_blocks,
                         g_sizes.data_ptr())
         return (g_blocks[: ctx.num_blocks * eng.block_stride] if ctx.has_blocks else None), g_sizes, None, None, None
@@ -67,9 +68,9 @@ def derive_transforms(engine, axioms, blocks, sizes, capacity):
 def centres_extents(M):
     """Terminal centres (n x 3) and extents (n x 3, the column lengths of the
     3 x 3 part of model * scale(size)) of transforms M (n x 12)."""
-    c = M[:, [3, 7, 11]]
-    R = M.reshape(-1, 3, 4)[:, :, :3]
-    return c, torch.sqrt((R * R).sum(dim=1))
+    m = M.reshape(-1, 3, 4)
+    R = m[:, :, :3]
+    return m[:, :, 3].contiguous(), torch.sqrt((R * R).sum(dim=1))
 
 
 class PathTarget:
@@ -79,13 +80,32 @@ class PathTarget:
         order = torch.argsort(paths)
         self.paths = paths[order]
         self.c, self.e = centres_extents(M.detach()[order])
+        self.unique = bool((self.paths[1:] != self.paths[:-1]).all())
 
     def sse(self, M, paths, check=True):
         """Sum of squared errors of centres and extents against the target;
         check=True verifies that the derivation has exactly the target's
         paths (no branch, repetition count or discard changed)."""
-        order = torch.argsort(paths)
-        if check and not torch.equal(paths[order], self.paths):
-            raise ValueError("the derivation's paths differ from the target's")
-        c, e = centres_extents(M[order])
-        return ((c - self.c) ** 2).sum() + ((e - self.e) ** 2).sum()
+        n = self.paths.shape[0]
+        if paths.shape != self.paths.shape:
+            if check:
+                raise ValueError("the derivation's paths differ from the target's")
+            c, e = centres_extents(M[torch.argsort(paths)])
+            return ((c - self.c) ** 2).sum() + ((e - self.e) ** 2).sum()
+        # The target's terminals are put in the derivation's order and not the
+        # other way round: they need no gradient, so no backward pass has to
+        # undo the gather.
+        if check and self.unique and n > 0:
+            at = torch.searchsorted(self.paths, paths).clamp_(max=n - 1)
+            found = torch.zeros(n, dtype=torch.bool, device=paths.device)
+            found[at] = self.paths[at] == paths  # a path of the target nobody has stays False
+            if not found.all():
+                raise ValueError("the derivation's paths differ from the target's")
+        else:
+            order = torch.argsort(paths)
+            if check and not torch.equal(paths[order], self.paths):
+                raise ValueError("the derivation's paths differ from the target's")
+            at = torch.empty_like(order)
+            at[order] = torch.arange(n, device=order.device)
+        c, e = centres_extents(M)
+        return ((c - self.c[at]) ** 2).sum() + ((e - self.e[at]) ** 2).sum()

@@ -221,7 +221,8 @@ const PgaProc* pga_default_procs(uint32_t* numProcs) {
 
 static void free_engine(PgaEngine* e) {
   void* phasePtrs[] = {e->dDefer[0], e->dDefer[1], e->dDeferRot[0], e->dDeferRot[1], e->dColRec, e->dColShape,
-                       e->dColNodes, e->dColParents, e->dColAabbs, e->dColLeaf, e->dColKeys, e->dPhaseCounters};
+                       e->dColNodes, e->dColParents, e->dColAabbs, e->dColLeaf, e->dColKeys, e->dPhaseCounters,
+                       e->dPhaseReport};
   for (void* p : phasePtrs)
     if (p) cudaFree(p);
   void* ptrs[] = {e->dRules, e->dParams, e->dSucc, e->dExpPool, e->dState, e->dNodes, e->dNodeRot, e->dLevelClock,
@@ -231,6 +232,7 @@ static void free_engine(PgaEngine* e) {
                   e->dSlots, e->dBlockSums, e->dGroupCount};
   for (void* p : ptrs)
     if (p) cudaFree(p);
+  if (e->hReadBack) cudaFreeHost(e->hReadBack);
   if (e->dStageAxioms) cudaFree(e->dStageAxioms);
   if (e->dStageOut) cudaFree(e->dStageOut);
   if (e->dStageCount) cudaFree(e->dStageCount);
@@ -474,6 +476,7 @@ PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* co
     ALLOC(e->dColLeaf, e->colCap * sizeof(uint32_t));
     ALLOC(e->dColKeys, e->colCap * sizeof(uint64_t));
     ALLOC(e->dPhaseCounters, 4 * sizeof(unsigned long long));
+    ALLOC(e->dPhaseReport, sizeof(PhaseReport));
   }
   ALLOC(e->dLevelStart, (c.maxLevels + 2) * sizeof(unsigned long long));
   ALLOC(e->dLevelClock, (c.maxLevels + 2) * sizeof(unsigned long long));
@@ -503,6 +506,8 @@ PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* co
   ALLOC(e->dValsB, c.maxTerminals * sizeof(uint32_t));
   ALLOC(e->dOpenTrees, pga_lbvh_open_bytes(c.maxTerminals));
 #undef ALLOC
+  err = cudaMallocHost(&e->hReadBack, std::max(sizeof(DevState), sizeof(PhaseReport)));
+  if (err != cudaSuccess) return fail(cuda_status(err, "cudaMallocHost hReadBack"));
   err = cudaMemcpy(e->dRules, e->hRules.data(), e->hRules.size() * sizeof(DevRule), cudaMemcpyHostToDevice);
   if (err == cudaSuccess)
     err = cudaMemcpy(e->dParams, e->hParams.data(), e->hParams.size() * sizeof(DevParam), cudaMemcpyHostToDevice);
@@ -646,6 +651,16 @@ static PgaStatus group_axioms(PgaEngine* e, const PgaAxiom* dAxioms, uint32_t n,
   return PGA_OK;
 }
 
+// Copies a small device record to the host once `s` has reached it, through the
+// engine's pinned buffer (a copy to pageable memory is staged by the driver).
+static PgaStatus read_back(PgaEngine* e, void* dst, const void* src, size_t bytes, cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(e->hostMutex);
+  PGA_CUDA_TRY(cudaMemcpyAsync(e->hReadBack, src, bytes, cudaMemcpyDeviceToHost, s));
+  PGA_CUDA_TRY(cudaStreamSynchronize(s));
+  memcpy(dst, e->hReadBack, bytes);
+  return PGA_OK;
+}
+
 static PgaStatus launch_persistent(PgaEngine* e, const PgaAxiom* dAxioms, uint32_t first, uint32_t end,
                                    const float* dParamBlocks, PgaTerminal* dOut, uint64_t capacity, uint64_t* dCount,
                                    cudaStream_t s, const uint32_t* order = nullptr) {
@@ -675,30 +690,50 @@ static PgaStatus launch_persistent(PgaEngine* e, const PgaAxiom* dAxioms, uint32
   return PGA_OK;
 }
 
-// Bounds of the colliders' centres (one block), for the Morton codes of their LBVH.
-__global__ void k_collider_bounds(const PgaTerminal* rec, unsigned long long n, float* out) {
-  __shared__ float sh[6][256];
+// What the host needs of a phase before the next (one block): the launch's
+// state, the colliders stored and the shapes deferred so far and, when there
+// is a next phase, the bounds of the colliders' centres for the Morton codes
+// of their LBVH.  Gathered on the device so that a phase costs one copy and one
+// wait of the host.
+__global__ void __launch_bounds__(1024) k_phase_report(const DevState* st, const unsigned long long* counters,
+                                                       const PgaTerminal* rec, unsigned long long cap,
+                                                       PhaseReport* out) {
+  __shared__ float sh[6][32];
+  const unsigned long long colliders = counters[0], deferred = counters[1];
+  const unsigned long long n = deferred != 0 ? min(colliders, cap) : 0ull;
   float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
   for (unsigned long long i = threadIdx.x; i < n; i += blockDim.x)
+#pragma unroll
     for (int k = 0; k < 3; k++) {
       const float c = rec[i].m[k * 4 + 3];
       lo[k] = fminf(lo[k], c);
       hi[k] = fmaxf(hi[k], c);
     }
-  for (int k = 0; k < 3; k++) {
-    sh[k][threadIdx.x] = lo[k];
-    sh[3 + k][threadIdx.x] = hi[k];
-  }
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1)
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      lo[k] = fminf(lo[k], __shfl_xor_sync(0xFFFFFFFFu, lo[k], d));
+      hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xFFFFFFFFu, hi[k], d));
+    }
+  if ((threadIdx.x & 31u) == 0)
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      sh[k][threadIdx.x >> 5] = lo[k];
+      sh[3 + k][threadIdx.x >> 5] = hi[k];
+    }
   __syncthreads();
-  for (unsigned w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w)
-      for (int k = 0; k < 3; k++) {
-        sh[k][threadIdx.x] = fminf(sh[k][threadIdx.x], sh[k][threadIdx.x + w]);
-        sh[3 + k][threadIdx.x] = fmaxf(sh[3 + k][threadIdx.x], sh[3 + k][threadIdx.x + w]);
-      }
-    __syncthreads();
+  if (threadIdx.x < 6) {
+    float v = sh[threadIdx.x][0];
+    for (int w = 1; w < 32; w++) v = threadIdx.x < 3 ? fminf(v, sh[threadIdx.x][w]) : fmaxf(v, sh[threadIdx.x][w]);
+    out->bounds[threadIdx.x] = v;
   }
-  if (threadIdx.x < 6) out[threadIdx.x] = sh[threadIdx.x][0];
+  if (threadIdx.x == 0) {
+    out->termCount = st->termCount;
+    out->colliders = colliders;
+    out->deferred = deferred;
+    out->status = st->status;
+  }
 }
 
 // Multi-phase derivation (MultiPhaseEvaluator::execute, CPUEvaluator.h:330-352,
@@ -740,30 +775,24 @@ static PgaStatus derive_phases(PgaEngine* e, const PgaAxiom* dAxioms, uint32_t n
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     PGA_CUDA_TRY(cudaLaunchKernelExC(&cfg, persistent_kernel(e), args));
-    DevState snap;
-    unsigned long long counters[2];
-    PGA_CUDA_TRY(cudaMemcpyAsync(&snap, e->dState, sizeof snap, cudaMemcpyDeviceToHost, s));
-    PGA_CUDA_TRY(cudaMemcpyAsync(counters, e->dPhaseCounters, sizeof counters, cudaMemcpyDeviceToHost, s));
-    PGA_CUDA_TRY(cudaStreamSynchronize(s));
+    k_phase_report<<<1, 1024, 0, s>>>(e->dState, e->dPhaseCounters, e->dColRec, e->colCap, e->dPhaseReport);
+    PGA_CUDA_TRY(cudaGetLastError());
+    PhaseReport snap;
+    const PgaStatus read = read_back(e, &snap, e->dPhaseReport, sizeof snap, s);
+    if (read != PGA_OK) return read;
     e->phasesRun = phase + 1;
     total += snap.termCount;
-    numDefer = counters[1];
+    numDefer = snap.deferred;
     if (snap.status != 0 || numDefer == 0) break;
     // The colliders stored so far, for the next phase's IfCollides.
-    visible = (uint32_t)std::min<unsigned long long>(counters[0], e->colCap);
+    visible = (uint32_t)std::min<unsigned long long>(snap.colliders, e->colCap);
     if (visible == 1) {
       PGA_CUDA_TRY(cudaMemsetAsync(e->dColLeaf, 0, sizeof(uint32_t), s));
     } else if (visible >= 2) {
-      float* dB = reinterpret_cast<float*>(e->dColAabbs);  // scratch until the LBVH writes it
-      k_collider_bounds<<<1, 256, 0, s>>>(e->dColRec, visible, dB);
-      PGA_CUDA_TRY(cudaGetLastError());
-      float hb[6];
-      PGA_CUDA_TRY(cudaMemcpyAsync(hb, dB, sizeof hb, cudaMemcpyDeviceToHost, s));
-      PGA_CUDA_TRY(cudaStreamSynchronize(s));
       PgaBounds b;
       for (int k = 0; k < 3; k++) {
-        b.min[k] = hb[k] - 1.0f;
-        b.max[k] = hb[3 + k] + 1.0f;
+        b.min[k] = snap.bounds[k] - 1.0f;
+        b.max[k] = snap.bounds[3 + k] + 1.0f;
       }
       PgaLbvh out = {e->dColNodes, e->dColParents, e->dColAabbs, e->dColLeaf, e->dColKeys};
       const PgaStatus st = pga_lbvh_build(e, e->dColRec, visible, &b, &out, s);
@@ -1012,10 +1041,9 @@ PgaStatus pga_derive_plain(PgaEngine* e, const PgaAxiom* dAxioms, uint32_t numAx
 
 PgaStatus pga_engine_sync_report(PgaEngine* e, void* stream, PgaDeriveReport* report) {
   if (!e || !report) return PGA_ERR_INVALID_ARGUMENT;
-  cudaStream_t s = (cudaStream_t)stream;
   DevState snap;
-  PGA_CUDA_TRY(cudaMemcpyAsync(&snap, e->dState, sizeof(DevState), cudaMemcpyDeviceToHost, s));
-  PGA_CUDA_TRY(cudaStreamSynchronize(s));
+  const PgaStatus read = read_back(e, &snap, e->dState, sizeof(DevState), (cudaStream_t)stream);
+  if (read != PGA_OK) return read;
   memset(report, 0, sizeof *report);
   if (e->phased) snap.termCount = e->phaseTerminals;  // over all phases
   // Terminals past the caller's capacity were dropped (never wrapped around):

@@ -3,10 +3,20 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "engine.cuh"
+
+namespace pga {
+// A phase of a multi-phase derivation as the host reads it back (k_phase_report).
+struct PhaseReport {
+  unsigned long long termCount, colliders, deferred;
+  float bounds[6];  // of the colliders' centres: min xyz, max xyz
+  int32_t status, reserved;
+};
+}  // namespace pga
 
 struct PgaEngine {
   // Lowered rule table (device).
@@ -45,6 +55,7 @@ struct PgaEngine {
   uint32_t* dColLeaf = nullptr;
   uint64_t* dColKeys = nullptr;
   unsigned long long* dPhaseCounters = nullptr;  // [0] colliders, [1] deferred, [2] terminals of a launch
+  pga::PhaseReport* dPhaseReport = nullptr;
   uint64_t colCap = 0;
   uint64_t phaseTerminals = 0;                 // terminals of the last multi-phase derivation
   uint64_t phaseTerminalsHost = 0;             // its copy for the device count
@@ -98,6 +109,9 @@ struct PgaEngine {
   PgaTerminal* dStageOut = nullptr;
   uint64_t* dStageCount = nullptr;
   size_t stageAxiomBytes = 0, stageOutBytes = 0, stageCountBytes = 0;
+  // Pinned landing place of the small records the host waits for, one caller at a time.
+  void* hReadBack = nullptr;
+  std::mutex hostMutex;
   cudaStream_t copyStream = nullptr;
   cudaEvent_t evDerived = nullptr;
 };

@@ -121,9 +121,12 @@ def _check(status, what=""):
 def _stream_handle(stream):
     import torch
 
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return ctypes.c_void_p(stream.cuda_stream)
+    if stream is not None:
+        return ctypes.c_void_p(stream.cuda_stream)
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    # the current device's current stream, without building a Stream object (20 us a call)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _dev(arr_or_tensor):
@@ -211,13 +214,12 @@ class Engine:
         if out is None:
             out = torch.empty((capacity, G.TERMINAL_DT.itemsize), dtype=torch.uint8, device="cuda")
         capacity = out.shape[0]
-        count = torch.zeros(1, dtype=torch.int64, device="cuda")
         self.derive_raw(d_ax.data_ptr(), n_ax, None if d_blk is None else d_blk.data_ptr(), out.data_ptr(), capacity,
-                        count.data_ptr(), stream, plain)
-        rep = self.report(stream)
+                        None, stream, plain)
+        rep = self.report(stream)  # waits for the derivation; its count is the one d_count would get
         if check and rep["status"] != 0:
             raise PgaError(rep["status"], f"device status (detail {rep['detail']})")
-        n = int(count.item())
+        n = rep["terminals"]
         if check and n > capacity:
             raise PgaError(2, f"{n} terminals > capacity {capacity}")
         return out, n, rep
@@ -241,8 +243,7 @@ class Engine:
             "leafTerminal": torch.empty(n, dtype=torch.int32, device=dev),
             "keys": torch.empty(n, dtype=torch.int64, device=dev),
         }
-        b = np.asarray(bounds, np.float32).reshape(6)
-        pb = PgaBounds((ctypes.c_float * 3)(*b[:3]), (ctypes.c_float * 3)(*b[3:]))
+        pb = PgaBounds.from_buffer_copy(np.asarray(bounds, np.float32).reshape(6))
         out = PgaLbvh(res["nodes"].data_ptr(), res["leafParents"].data_ptr(), res["aabbs"].data_ptr(),
                       res["leafTerminal"].data_ptr(), res["keys"].data_ptr())
         if count is None:
