@@ -691,7 +691,11 @@ __device__ __forceinline__ void page_param_grads(const DeriveArgs& a, const AdjA
 // was queued as) and pushed back through its chain and the operator that
 // created it -- summed into the item's gradient, which is stored (or, for an
 // axiom's root item, pushed into the axiom's sizes).
-__device__ void adj_page(const DeriveArgs& a, const AdjArgs& j, unsigned long long i, unsigned long long nodes) {
+//
+// The general form, one thread an item and out of line: for the rules that
+// adj_sums does not cover.
+__device__ __noinline__ void adj_page(const DeriveArgs& a, const AdjArgs& j, unsigned long long i,
+                                      unsigned long long nodes) {
   Expander E;
   uint4 ext;
   load_node(a, i, E.base, ext);
@@ -777,6 +781,239 @@ __device__ void adj_page(const DeriveArgs& a, const AdjArgs& j, unsigned long lo
   }
 }
 
+// Column `src` of x's rotation, times column q of dL/dM at gm.
+__device__ __forceinline__ float column_dot(const Shape& x, uint32_t src, const float* gm, uint32_t q) {
+#if PGA_GENERAL_FRAMES
+  return __ldg(gm + q) * frame_at(x, 0, src) + __ldg(gm + 4 + q) * frame_at(x, 1, src) +
+         __ldg(gm + 8 + q) * frame_at(x, 2, src);
+#else
+  const float v = __ldg(gm + frame_row(x.frame, src) * 4 + q);
+  return frame_neg(x.frame, src) ? -v : v;
+#endif
+}
+
+// Reverse step of the work items of kRuleSums rules.  Their children pass
+// their gradients on unchanged and enter the item's in sums (SumAcc), so
+// neither a child's state nor its chain is replayed, nothing is kept per child,
+// and the sums of lanes that share an item add up.  2^shift neighbouring lanes
+// share item i (the same i, valid and shift in all of them); `part` is the
+// lane's number among them.  Items of other rules are left to the first lane
+// and adj_page.
+//
+// With c a child, o_c its offset along the split axis, N_c its size there,
+// S the item's size, go / gN the gradients with respect to o_c and N_c:
+//  Subdivide  N_k = f_k (f_k > 0) or scale * -f_k (f_k < 0), scale = (S - sum of
+//             the positive f) / R, R = sum of -f over the negative f, and
+//             o_c = -S/2 + sum_{k<c} N_k + N_c/2.  W_k, the coefficient of dN_k,
+//             is gN_k + go_k / 2 plus go of every later child; Q = sum of
+//             W_k f_k over the negative f_k.  dL/dS = -sum(go)/2 - Q/R,
+//             dL/df_k = W_k + Q/R (f_k > 0) or -(W_k + Q/R) scale (f_k < 0).
+//  Repeat     first, middle and last pieces of sizes startExt, e2, endExt.
+//  ComponentSplit  face c: half a size along its normal, two of the sizes.
+// The replay kept each child's state, its chain and the Subdivide's terms in
+// local memory and took about three times the instructions; adjoint of 1,024
+// facades 152 -> 79 us, of the 1,500-axiom mix 810 -> 428, of the 8,192-axiom
+// mix with parameter blocks 4.65 -> 2.08 ms.
+struct SumAcc {
+  Grad g;                // translation, and the sizes that pass through
+  float go;              // Subdivide, Repeat: sum of dL/do
+  float q;               // Subdivide: Q
+  float start, mid, end; // Repeat: dL/d startExt, e2, endExt
+};
+
+__device__ __forceinline__ void adj_sums(const DeriveArgs& a, const AdjArgs& j, unsigned long long i, bool valid,
+                                         unsigned long long nodes, uint32_t shift, uint32_t part) {
+  constexpr bool kBlocks = PGA_INLINE_BLOCKS || PGA_GENERAL_FRAMES;  // tables with block parameters
+  Shape x;
+  uint4 ext = make_uint4(kEmptyItem, 0u, 0u, 0u);
+  if (valid) load_node(a, i, x, ext);
+  if (ext.x == kEmptyItem) return;
+  if (x.entry < 0 || (uint32_t)x.entry >= a.tab.numEntries) {
+    if (part == 0) raise_error(a.st, PGA_ERR_NO_TAPE, (int)i);
+    return;
+  }
+  const DevRule r = rule_at(a, (uint32_t)x.entry);
+  if (!(r.flags & kRuleSums)) {
+    if (part == 0) adj_page(a, j, i, nodes);
+    return;
+  }
+  x.kind = r.shape;
+  const uint32_t key = __ldcg(j.childKey + i);
+  const bool subdivide = r.op == PGA_OP_SUBDIVIDE || r.op == PGA_OP_SUBDIVIDE_STATIC;
+  const bool repeat = r.op == PGA_OP_REPEAT;
+  const bool scalar = (r.flags & kRuleScalar) != 0;
+  uint32_t all = r.op == PGA_OP_COMPONENT_SPLIT ? 6u : r.nSucc;
+  uint32_t axis = 0;
+  float relSum = 0.0f, scale = 0.0f;
+  RepeatSetup R{};
+  if (subdivide) {
+    all = r.op == PGA_OP_SUBDIVIDE ? r.nParams - 1u : r.nChildren;
+    axis = f2u(param(a, r, 0, x));
+    float absSum = 0.0f;
+    for (uint32_t k = 1; k <= all; k++) {
+      const float f = param(a, r, k, x);
+      absSum += f > 0.0f ? f : 0.0f;
+      relSum += f < 0.0f ? -f : 0.0f;
+    }
+    scale = relSum == 0.0f ? 0.0f : (pick3(x.s, axis) - absSum) / relSum;
+  } else if (repeat) {
+    R = repeat_setup(a, r, x, false);
+    axis = R.axis;
+    all = (R.flags & 1u) ? max(R.reps, 1u) : 0u;
+  }
+  uint32_t c0 = ext.x, c1 = min(ext.y, all);
+  if (shift > 0) {  // this lane's run of the children
+    const uint32_t run = ((c1 > c0 ? c1 - c0 : 0u) + (1u << shift) - 1u) >> shift;
+    c0 = min(c0 + part * run, c1);
+    c1 = min(c0 + run, c1);
+  }
+  SumAcc s;
+  grad_zero(s.g);
+  s.go = s.q = s.start = s.mid = s.end = 0.0f;
+  float W[kBlocks ? kSumFactors : 1];
+  if (kBlocks)
+#pragma unroll
+    for (uint32_t k = 0; k < kSumFactors; k++) W[k] = 0.0f;
+  float below = 0.0f;  // sum of the negative factors of the children before c
+  if (subdivide)
+    for (uint32_t k = 0; k < c0; k++) {
+      const float f = param(a, r, k + 1, x);
+      below += f < 0.0f ? f : 0.0f;
+    }
+  for (uint32_t c = c0; c < c1; c++) {
+    const float f = subdivide ? param(a, r, c + 1, x) : 0.0f;
+    const float relF = f < 0.0f ? f : 0.0f;
+    const uint32_t v = __ldcg(j.slots + (uint32_t)(key + c + (repeat ? 1u : 0u)));
+    if (v != kNoRecord) {  // not discarded
+      // The child's frame: the item's, or a face's, whose first two columns are
+      // columns q0 and q1 of it (ComponentSplit's faces, see expander_child).
+      uint32_t q0 = 0, q1 = 1, normal = 2;
+      bool neg0 = false, negNormal = false;
+      if (r.op == PGA_OP_COMPONENT_SPLIT) {
+        normal = c < 2 ? 2u : (c < 4 ? 0u : 1u);
+        negNormal = (c & 1u) == 0u;
+        if (c == 2 || c == 3) q0 = 2;
+        if (c >= 4) q1 = 2;
+        neg0 = c == 0 || c == 3;
+      }
+      Grad g;
+      if (v & kItemTag) {
+        g = pages_grad(j, v, nodes);
+      } else {
+        const float* gm = j.gradTerminals + (size_t)v * j.gradStride;
+#pragma unroll
+        for (int q = 0; q < 3; q++) g.t[q] = __ldg(gm + q * 4 + 3);
+        g.s[0] = column_dot(x, q0, gm, 0);
+        g.s[0] = neg0 ? -g.s[0] : g.s[0];
+        g.s[1] = column_dot(x, q1, gm, 1);
+        if (r.op == PGA_OP_COMPONENT_SPLIT) {
+          g.s[1] = c == 5 ? -g.s[1] : g.s[1];
+          g.s[2] = 0.0f;  // a face's third size is the constant 1
+        } else {
+          g.s[2] = column_dot(x, 2, gm, 2);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < 3; q++) s.g.t[q] += g.t[q];
+      if (subdivide || repeat) {
+        const float go = axis_dot(x, axis, g.t), gN = pick3(g.s, axis);
+#pragma unroll
+        for (uint32_t q = 0; q < 3; q++) s.g.s[q] += q == axis ? 0.0f : g.s[q];
+        s.go += go;
+        if (subdivide) {
+          const float own = gN + 0.5f * go;
+          s.q += go * below + own * relF;
+          if (kBlocks && !scalar)
+#pragma unroll
+            for (uint32_t k = 0; k < kSumFactors; k++) W[k] += k == c ? own : (k < c ? go : 0.0f);
+        } else {
+          const bool first = c == 0, last = c > 0 && c + 1 >= R.reps;
+          s.start += first ? 0.5f * go + gN : go;
+          s.mid += first ? 0.0f : (last ? go * (float)(R.reps - 2) : go * ((float)c - 0.5f) + gN);
+          s.end += last ? 0.5f * go + gN : 0.0f;
+        }
+      } else if (r.op == PGA_OP_COMPONENT_SPLIT) {
+        const float go = 0.5f * axis_dot(x, normal, g.t);
+        const float along = negNormal ? -go : go;
+#pragma unroll
+        for (uint32_t q = 0; q < 3; q++)
+          s.g.s[q] += (q == normal ? along : 0.0f) + (q == q0 ? g.s[0] : 0.0f) + (q == q1 ? g.s[1] : 0.0f);
+      } else {
+#pragma unroll
+        for (uint32_t q = 0; q < 3; q++) s.g.s[q] += g.s[q];
+      }
+    }
+    below += relF;
+  }
+  if (shift > 0) {
+    const unsigned lane = threadIdx.x & 31u, width = 1u << shift;
+    const unsigned group = (width == 32u ? kFull : ((1u << width) - 1u)) << (lane & ~(width - 1u));
+    for (uint32_t d = width >> 1; d > 0; d >>= 1) {
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        s.g.t[q] += __shfl_xor_sync(group, s.g.t[q], d);
+        s.g.s[q] += __shfl_xor_sync(group, s.g.s[q], d);
+      }
+      s.go += __shfl_xor_sync(group, s.go, d);
+      s.q += __shfl_xor_sync(group, s.q, d);
+      s.start += __shfl_xor_sync(group, s.start, d);
+      s.mid += __shfl_xor_sync(group, s.mid, d);
+      s.end += __shfl_xor_sync(group, s.end, d);
+      if (kBlocks && !scalar)
+#pragma unroll
+        for (uint32_t k = 0; k < kSumFactors; k++) W[k] += __shfl_xor_sync(group, W[k], d);
+    }
+    if (part != 0) return;
+  }
+  if (subdivide) {
+    const float q = relSum != 0.0f ? s.q / relSum : 0.0f;
+    const float gS = -0.5f * s.go - q;
+    s.g.s[0] += axis == 0 ? gS : 0.0f;
+    s.g.s[1] += axis == 1 ? gS : 0.0f;
+    s.g.s[2] += axis == 2 ? gS : 0.0f;
+    if (kBlocks && !scalar)
+#pragma unroll
+      for (uint32_t k = 0; k < kSumFactors; k++) {
+        if (k >= all) break;
+        const float f = param(a, r, k + 1, x);
+        const float g = f > 0.0f ? W[k] + q : (f < 0.0f ? -(W[k] + q) * scale : 0.0f);
+        param_grad(a, j, r, k + 1, x, g, nullptr);
+      }
+  } else if (repeat && all > 0) {
+    const bool start = (R.flags & 2u) != 0;
+    const uint32_t mode = f2u(param(a, r, 2, x));
+    const float S = pick3(x.s, axis);
+    float gS = -0.5f * s.go, gE = 0.0f;
+    const float ext1 = param(a, r, 1, x);
+    if (mode == 2u) {
+      if (R.reps > 0) gS += (s.start + s.mid + s.end) / (float)R.reps;
+    } else {
+      const float E = ext1 < 0.0f ? S * fabsf(ext1) : ext1;
+      const float ge1 = start ? s.start : s.end;
+      gE = (start ? s.end : s.start) + s.mid;
+      if (fmodf(S, E) == 0.0f) {
+        gE += ge1;
+      } else {
+        gS += ge1;
+        gE -= truncf(S / E) * ge1;
+      }
+    }
+    if (ext1 < 0.0f) gS += gE * fabsf(ext1);
+    s.g.s[0] += axis == 0 ? gS : 0.0f;
+    s.g.s[1] += axis == 1 ? gS : 0.0f;
+    s.g.s[2] += axis == 2 ? gS : 0.0f;
+    if (kBlocks && !scalar) param_grad(a, j, r, 1, x, ext1 < 0.0f ? gE * (-S) : gE, nullptr);
+  }
+  if (ext.z & kAxiomLink) {
+    push_to_axiom(a, j, ext.z & ~kAxiomLink, false, 0, s.g);
+    return;
+  }
+  float2* dst = reinterpret_cast<float2*>(j.nodeGrad + (size_t)i * 6);
+  __stcg(dst + 0, make_float2(s.g.t[0], s.g.t[1]));
+  __stcg(dst + 1, make_float2(s.g.t[2], s.g.s[0]));
+  __stcg(dst + 2, make_float2(s.g.s[1], s.g.s[2]));
+}
+
 // Block-wide exclusive scan of one value per thread; total receives the sum.
 __device__ __forceinline__ unsigned long long block_excl_scan(uint32_t v, unsigned long long& total) {
   __shared__ unsigned long long warpSum[kWarps];
@@ -821,16 +1058,14 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v) {
 // or overflowed forward pass leaves the gradients zero (the engine report
 // keeps the forward's status; a tape too short for the terminals or a slot
 // map larger than its buffer raises PGA_ERR_NO_TAPE).
-// Two launch shapes of the same pass.  k_adjoint keeps the compiler's
-// register choice (2 blocks of 256 per SM; the block build pins 2 blocks: left
-// free, its choice there came out at 80 registers with spills).
-// k_adjoint_wide (frame-code builds) runs 3 blocks per SM (80 registers, ~300
-// B of spills; the block build 4 blocks, 64 registers): with the level's pages handed out on demand the extra warps
-// hide more of the scattered reads on large tapes (65,536-axiom step: sizes
-// 19.2 -> 18.2 ms, all parameters 35 -> 32 ms), while on small ones the
-// spills and the larger grid's barriers cost more (1,024 facades: forward +
-// adjoint 0.264 -> 0.302 ms).  Engines choose by terminal capacity
-// (kWideAdjointTerminals).  PGA_ADJOINT_MIN_BLOCKS overrides k_adjoint's shape.
+// Two launch shapes of the same pass.  k_adjoint runs 2 blocks of 256 per SM;
+// k_adjoint_wide (frame-code builds) 3, at 80 registers: on large tapes the
+// extra warps hide more of the scattered reads (1,500-axiom mix, 3.4M
+// terminals: 490 us with 2 blocks, 428 with 3, 472 with 4; 8,192 axioms with
+// blocks 2.21 / 2.08 / 2.33 ms), on small ones the spills and the larger
+// grid's barriers cost more (1,024 facades, 0.4M terminals: 78 / 93 / 104 us).
+// Engines choose by terminal capacity (kWideAdjointTerminals, 2M).
+// PGA_ADJOINT_MIN_BLOCKS overrides k_adjoint's shape.
 #if defined(PGA_ADJOINT_MIN_BLOCKS)
 #define PGA_ADJOINT_BOUNDS __launch_bounds__(kThreads, PGA_ADJOINT_MIN_BLOCKS)
 #elif PGA_INLINE_BLOCKS
@@ -974,26 +1209,32 @@ __device__ __forceinline__ void adjoint_pass(const DeriveArgs& a, const AdjArgs&
   for (int L = (int)levels; L >= 0; L--) {
     const unsigned long long lv = a.levelStart[L], hv = min(a.levelStart[L + 1], nodes);
     if (lv >= hv) continue;  // every block reads the same bounds, so all skip the barrier alike
-    unsigned long long dynLo = hv;
-    if (hv - lv >= 4 * stride) {
-      const unsigned long long n = hv - lv;
-      dynLo = lv + ((n - max(n / PGA_ADJOINT_DYNAMIC_SHARE, 2 * stride)) / stride) * stride;
-    }
-    // one call site of adj_page for both orders
-    for (unsigned long long i = lv + tid;; i += stride) {
-      if (i >= dynLo) {
-        if (dynLo >= hv) break;
-        unsigned long long c = 0;
-        if ((threadIdx.x & 31u) == 0) c = atomicAdd(&a.st->cursor, 32ull);
-        c = dynLo + __shfl_sync(kFull, c, 0);
-        if (c >= hv) break;
-        i = c + (threadIdx.x & 31u);  // the loop step never lands below dynLo again
-        if (i >= hv) continue;        // this lane has no item in the last chunk
-      } else if (i + stride < dynLo) {  // the next item's record and key, ahead of its turn
-        prefetch_l2(a.nodes + i + stride);
-        prefetch_l2(j.childKey + i + stride);
+    const uint32_t shift = share_shift(hv - lv);
+    if (shift > 0) {  // a narrow level: 2^shift lanes to an item
+      const unsigned long long i = lv + (tid >> shift);
+      adj_sums(a, j, min(i, hv - 1), i < hv, nodes, shift, (uint32_t)tid & ((1u << shift) - 1u));
+    } else {
+      unsigned long long dynLo = hv;
+      if (hv - lv >= 4 * stride) {
+        const unsigned long long n = hv - lv;
+        dynLo = lv + ((n - max(n / PGA_ADJOINT_DYNAMIC_SHARE, 2 * stride)) / stride) * stride;
       }
-      adj_page(a, j, i, nodes);
+      // one call site of adj_sums for both orders
+      for (unsigned long long i = lv + tid;; i += stride) {
+        if (i >= dynLo) {
+          if (dynLo >= hv) break;
+          unsigned long long c = 0;
+          if ((threadIdx.x & 31u) == 0) c = atomicAdd(&a.st->cursor, 32ull);
+          c = dynLo + __shfl_sync(kFull, c, 0);
+          if (c >= hv) break;
+          i = c + (threadIdx.x & 31u);  // the loop step never lands below dynLo again
+          if (i >= hv) continue;        // this lane has no item in the last chunk
+        } else if (i + stride < dynLo) {  // the next item's record and key, ahead of its turn
+          prefetch_l2(a.nodes + i + stride);
+          prefetch_l2(j.childKey + i + stride);
+        }
+        adj_sums(a, j, i, true, nodes, 0, 0);
+      }
     }
     if (!grid_barrier(a, [&] { a.st->cursor = 0ull; })) return;
   }
@@ -1006,11 +1247,7 @@ __global__ void PGA_ADJOINT_BOUNDS k_adjoint(DeriveArgs a, AdjArgs j, unsigned l
 
 #if !PGA_GENERAL_FRAMES
 #ifndef PGA_ADJOINT_WIDE_BLOCKS
-#if PGA_INLINE_BLOCKS
-#define PGA_ADJOINT_WIDE_BLOCKS 4  // 64 registers: all parameters 33 -> 31 ms on the 65,536-axiom step
-#else
-#define PGA_ADJOINT_WIDE_BLOCKS 3  // at 4 the sizes step's adjoint lost 3%
-#endif
+#define PGA_ADJOINT_WIDE_BLOCKS 3
 #endif
 __global__ void __launch_bounds__(kThreads, PGA_ADJOINT_WIDE_BLOCKS) k_adjoint_wide(DeriveArgs a, AdjArgs j,
                                                               unsigned long long numParamFloats, uint32_t numAxioms) {

@@ -377,6 +377,49 @@ PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* co
     // replays one work item per branching shape) or when disabled.
     if (leaf && !c.recordTape && !(c.flags & PGA_FLAG_NO_INLINE)) e->leafKernel = true;
   }
+  // Rules whose children the adjoint sums in closed form (kRuleSums).  An entry
+  // is plain when every 1 -> 1 chain from it only picks branches.
+  {
+    std::vector<int8_t> plain(e->hRules.size(), -1);  // -1 unknown, -2 being looked at (a cycle: not plain)
+    auto isPlain = [&](auto&& self, int32_t t, int depth) -> bool {
+      if (t < 0 || (size_t)t >= e->hRules.size() || depth > kMaxChain) return false;
+      if (plain[(size_t)t] >= 0) return plain[(size_t)t] != 0;
+      if (plain[(size_t)t] == -2) return false;
+      const DevRule& r = e->hRules[(size_t)t];
+      bool ok = false;
+      switch (r.op) {
+        case PGA_OP_SUBDIVIDE: case PGA_OP_SUBDIVIDE_STATIC: case PGA_OP_REPEAT: case PGA_OP_COMPONENT_SPLIT:
+        case PGA_OP_REPLICATE: case PGA_OP_GENERATE: case PGA_OP_DISCARD:
+          ok = true;
+          break;
+        case PGA_OP_IF_SIZE_LESS: case PGA_OP_IF: case PGA_OP_RANDOM_RULE: case PGA_OP_RANDOM_RULE_STATIC:
+          plain[(size_t)t] = -2;
+          ok = true;
+          for (uint32_t k = 0; k < r.nSucc && ok; k++) ok = self(self, e->hSucc[r.succBase + k], depth + 1);
+          plain[(size_t)t] = -1;
+          if (!ok) return false;  // perhaps only because of the cycle or depth met on this way
+          break;
+        default:
+          break;
+      }
+      plain[(size_t)t] = ok ? 1 : 0;
+      return ok;
+    };
+    for (DevRule& r : e->hRules) {
+      bool sums = r.nSucc > 0;
+      if (r.op == PGA_OP_SUBDIVIDE || r.op == PGA_OP_SUBDIVIDE_STATIC) {
+        const uint32_t n = r.op == PGA_OP_SUBDIVIDE ? (r.nParams >= 1 ? r.nParams - 1u : 0u) : r.nChildren;
+        sums = sums && n > 0 && n < r.nParams + 0u && (r.flags & kRulePure) &&
+               ((r.flags & kRuleScalar) || n <= kSumFactors);
+      } else if (r.op == PGA_OP_REPEAT) {
+        sums = sums && (r.flags & kRulePure);
+      } else {
+        sums = sums && (r.op == PGA_OP_COMPONENT_SPLIT || r.op == PGA_OP_REPLICATE);
+      }
+      for (uint32_t k = 0; k < r.nSucc && sums; k++) sums = isPlain(isPlain, e->hSucc[r.succBase + k], 0);
+      if (sums) r.flags |= kRuleSums;
+    }
+  }
   // Phases: the phase of a rule is the phaseIndex of the successor edges that
   // lead to it (the reference queues a symbol in the phase its edge names,
   // CPUEvaluator.h:155-190); edges into one rule must agree.  A shape reaching

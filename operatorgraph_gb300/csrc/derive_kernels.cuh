@@ -19,7 +19,7 @@ constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr uint32_t kMaxAdjointBlocks = 8192;  // blocks of the reverse launch (slot-map scan)
 // Engines with at least this terminal capacity launch the 3-blocks-per-SM adjoint (k_adjoint_wide).
-constexpr unsigned long long kWideAdjointTerminals = 1ull << 23;
+constexpr unsigned long long kWideAdjointTerminals = 1ull << 21;
 enum Kind { kNone = 0, kTerm = 1, kNode = 2 };
 
 struct __align__(16) Smem {

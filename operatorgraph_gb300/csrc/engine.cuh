@@ -78,6 +78,12 @@ constexpr uint16_t kRuleConstTerminal = 2;  // Generate with a scalar terminal i
 constexpr uint16_t kRuleLeaf = 4;           // Subdivide whose children all end at once (expanded in place)
 constexpr uint16_t kRuleMesh = 8;           // a triangle-mesh Generate (lowered to op GENERATE for the derivation)
 constexpr uint16_t kRuleScalar = 16;        // every parameter a scalar constant
+// The adjoint sums the rule's children in closed form: a split with pure
+// parameters (a Subdivide of at most kSumFactors factors) or a Replicate, and
+// no smooth step (Extrude, Translate, Scale, SwapSize, Rotate) between it and
+// the terminals and work items its children become.
+constexpr uint16_t kRuleSums = 32;
+constexpr uint32_t kSumFactors = 8;
 constexpr uint32_t kRulePhaseShift = 8;     // flags bits 8..11: the phase of the edges into the rule (multi-phase)
 constexpr uint32_t kMaxPhases = 16;
 
