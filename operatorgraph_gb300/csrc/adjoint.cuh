@@ -625,10 +625,6 @@ __device__ __noinline__ void push_to_axiom(const DeriveArgs& a, const AdjArgs& j
 constexpr uint32_t kNoRecord = 0xFFFFFFFFu;
 constexpr uint32_t kItemTag = 0x80000000u;
 
-__device__ __forceinline__ uint32_t page_children(const uint4& ext) {
-  return ext.x == kEmptyItem ? 0u : ext.y - ext.x;
-}
-
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // Slots read ahead per work item (a work item has max(subItem, narrowSubItem)
@@ -813,7 +809,9 @@ __device__ __forceinline__ float column_dot(const Shape& x, uint32_t src, const 
 // The replay kept each child's state, its chain and the Subdivide's terms in
 // local memory and took about three times the instructions; adjoint of 1,024
 // facades 152 -> 79 us, of the 1,500-axiom mix 810 -> 428, of the 8,192-axiom
-// mix with parameter blocks 4.65 -> 2.08 ms.
+// mix with parameter blocks 4.65 -> 2.08 ms.  Only what the sums need of the
+// item is loaded and parameters are read without the general path (which takes
+// a whole shape): 80 registers with little spilled, and 1.83 -> 1.49 ms there.
 struct SumAcc {
   Grad g;                // translation, and the sizes that pass through
   float go;              // Subdivide, Repeat: sum of dL/do
@@ -821,12 +819,40 @@ struct SumAcc {
   float start, mid, end; // Repeat: dL/d startExt, e2, endExt
 };
 
+// A pure parameter: a scalar or a block value (the forward pass has checked
+// the slot).
+__device__ __forceinline__ float pure_param(const DeriveArgs& a, uint32_t k, uint32_t axiom) {
+  const DevParam p = param_at(a, k);
+  if (p.type == PGA_PT_SCALAR) return p.v0;
+  const uint32_t b = __ldg(&a.axioms[axiom].block);
+  return __ldg(&a.blocks[(size_t)b * a.blockStride + f2u(p.v0)]);
+}
+
 __device__ __forceinline__ void adj_sums(const DeriveArgs& a, const AdjArgs& j, unsigned long long i, bool valid,
                                          unsigned long long nodes, uint32_t shift, uint32_t part) {
   constexpr bool kBlocks = PGA_INLINE_BLOCKS || PGA_GENERAL_FRAMES;  // tables with block parameters
+  // Of the item's state only the sizes, the frame and the axiom enter.
   Shape x;
   uint4 ext = make_uint4(kEmptyItem, 0u, 0u, 0u);
-  if (valid) load_node(a, i, x, ext);
+  if (valid) {
+    const Node* rec = a.nodes + i;
+    ext = __ldcg(&rec->ext);
+    const uint2 meta = __ldcg(reinterpret_cast<const uint2*>(&rec->meta));
+    const float4 sf = __ldcg(&rec->sf);
+    x.s[0] = __ldcg(&rec->ts.w);
+    x.s[1] = sf.x;
+    x.s[2] = sf.y;
+#if PGA_GENERAL_FRAMES
+    const float4 r0 = __ldcg(a.nodeRot + 2 * i), r1 = __ldcg(a.nodeRot + 2 * i + 1);
+    x.R[0] = r0.x; x.R[1] = r0.y; x.R[2] = r0.z; x.R[3] = r0.w;
+    x.R[4] = r1.x; x.R[5] = r1.y; x.R[6] = r1.z; x.R[7] = r1.w;
+    x.R[8] = sf.w;
+#else
+    x.frame = __float_as_uint(sf.w);
+#endif
+    x.entry = (int32_t)meta.x;
+    x.axiom = meta.y;
+  }
   if (ext.x == kEmptyItem) return;
   if (x.entry < 0 || (uint32_t)x.entry >= a.tab.numEntries) {
     if (part == 0) raise_error(a.st, PGA_ERR_NO_TAPE, (int)i);
@@ -837,29 +863,32 @@ __device__ __forceinline__ void adj_sums(const DeriveArgs& a, const AdjArgs& j, 
     if (part == 0) adj_page(a, j, i, nodes);
     return;
   }
-  x.kind = r.shape;
   const uint32_t key = __ldcg(j.childKey + i);
   const bool subdivide = r.op == PGA_OP_SUBDIVIDE || r.op == PGA_OP_SUBDIVIDE_STATIC;
   const bool repeat = r.op == PGA_OP_REPEAT;
   const bool scalar = (r.flags & kRuleScalar) != 0;
   uint32_t all = r.op == PGA_OP_COMPONENT_SPLIT ? 6u : r.nSucc;
-  uint32_t axis = 0;
+  uint32_t axis = 0, reps = 0;
   float relSum = 0.0f, scale = 0.0f;
-  RepeatSetup R{};
   if (subdivide) {
     all = r.op == PGA_OP_SUBDIVIDE ? r.nParams - 1u : r.nChildren;
-    axis = f2u(param(a, r, 0, x));
+    axis = f2u(pure_param(a, r.paramBase, x.axiom));
     float absSum = 0.0f;
     for (uint32_t k = 1; k <= all; k++) {
-      const float f = param(a, r, k, x);
+      const float f = pure_param(a, r.paramBase + k, x.axiom);
       absSum += f > 0.0f ? f : 0.0f;
       relSum += f < 0.0f ? -f : 0.0f;
     }
     scale = relSum == 0.0f ? 0.0f : (pick3(x.s, axis) - absSum) / relSum;
   } else if (repeat) {
-    R = repeat_setup(a, r, x, false);
-    axis = R.axis;
-    all = (R.flags & 1u) ? max(R.reps, 1u) : 0u;
+    // the number of pieces, as repeat_setup finds it
+    axis = f2u(pure_param(a, r.paramBase, x.axiom));
+    const float ext1 = pure_param(a, r.paramBase + 1, x.axiom), S = pick3(x.s, axis);
+    const float E = __fadd_rn(__fmul_rn(__fmul_rn((float)(ext1 < 0.0f), S), fabsf(ext1)),
+                              __fmul_rn((float)(ext1 > 0.0f), ext1));
+    const float pieces = __fdiv_rn(S, E);
+    reps = f2u(f2u(pure_param(a, r.paramBase + 2, x.axiom)) == 2u ? floorf(pieces) : ceilf(pieces));
+    all = max(reps, 1u);
   }
   uint32_t c0 = ext.x, c1 = min(ext.y, all);
   if (shift > 0) {  // this lane's run of the children
@@ -877,13 +906,18 @@ __device__ __forceinline__ void adj_sums(const DeriveArgs& a, const AdjArgs& j, 
   float below = 0.0f;  // sum of the negative factors of the children before c
   if (subdivide)
     for (uint32_t k = 0; k < c0; k++) {
-      const float f = param(a, r, k + 1, x);
+      const float f = pure_param(a, r.paramBase + k + 1u, x.axiom);
       below += f < 0.0f ? f : 0.0f;
     }
+  // The slots one child ahead of the gradients they point to, and those
+  // gradients' lines one child ahead of their loads.
+  const uint32_t slot0 = key + (repeat ? 1u : 0u);
+  uint32_t vNext = c0 < c1 ? __ldcg(j.slots + (uint32_t)(slot0 + c0)) : kNoRecord;
   for (uint32_t c = c0; c < c1; c++) {
-    const float f = subdivide ? param(a, r, c + 1, x) : 0.0f;
+    const float f = subdivide ? pure_param(a, r.paramBase + c + 1u, x.axiom) : 0.0f;
     const float relF = f < 0.0f ? f : 0.0f;
-    const uint32_t v = __ldcg(j.slots + (uint32_t)(key + c + (repeat ? 1u : 0u)));
+    const uint32_t v = vNext;
+    vNext = c + 1 < c1 ? __ldcg(j.slots + (uint32_t)(slot0 + c + 1u)) : kNoRecord;
     if (v != kNoRecord) {  // not discarded
       // The child's frame: the item's, or a face's, whose first two columns are
       // columns q0 and q1 of it (ComponentSplit's faces, see expander_child).
@@ -927,9 +961,9 @@ __device__ __forceinline__ void adj_sums(const DeriveArgs& a, const AdjArgs& j, 
 #pragma unroll
             for (uint32_t k = 0; k < kSumFactors; k++) W[k] += k == c ? own : (k < c ? go : 0.0f);
         } else {
-          const bool first = c == 0, last = c > 0 && c + 1 >= R.reps;
+          const bool first = c == 0, last = c > 0 && c + 1 >= reps;
           s.start += first ? 0.5f * go + gN : go;
-          s.mid += first ? 0.0f : (last ? go * (float)(R.reps - 2) : go * ((float)c - 0.5f) + gN);
+          s.mid += first ? 0.0f : (last ? go * (float)(reps - 2) : go * ((float)c - 0.5f) + gN);
           s.end += last ? 0.5f * go + gN : 0.0f;
         }
       } else if (r.op == PGA_OP_COMPONENT_SPLIT) {
@@ -975,18 +1009,18 @@ __device__ __forceinline__ void adj_sums(const DeriveArgs& a, const AdjArgs& j, 
 #pragma unroll
       for (uint32_t k = 0; k < kSumFactors; k++) {
         if (k >= all) break;
-        const float f = param(a, r, k + 1, x);
+        const float f = pure_param(a, r.paramBase + k + 1u, x.axiom);
         const float g = f > 0.0f ? W[k] + q : (f < 0.0f ? -(W[k] + q) * scale : 0.0f);
         param_grad(a, j, r, k + 1, x, g, nullptr);
       }
-  } else if (repeat && all > 0) {
-    const bool start = (R.flags & 2u) != 0;
-    const uint32_t mode = f2u(param(a, r, 2, x));
+  } else if (repeat) {
+    const uint32_t mode = f2u(pure_param(a, r.paramBase + 2, x.axiom));
+    const bool start = mode == 0u;
     const float S = pick3(x.s, axis);
     float gS = -0.5f * s.go, gE = 0.0f;
-    const float ext1 = param(a, r, 1, x);
+    const float ext1 = pure_param(a, r.paramBase + 1, x.axiom);
     if (mode == 2u) {
-      if (R.reps > 0) gS += (s.start + s.mid + s.end) / (float)R.reps;
+      if (reps > 0) gS += (s.start + s.mid + s.end) / (float)reps;
     } else {
       const float E = ext1 < 0.0f ? S * fabsf(ext1) : ext1;
       const float ge1 = start ? s.start : s.end;
@@ -1014,23 +1048,38 @@ __device__ __forceinline__ void adj_sums(const DeriveArgs& a, const AdjArgs& j, 
   __stcg(dst + 2, make_float2(s.g.s[1], s.g.s[2]));
 }
 
-// Block-wide exclusive scan of one value per thread; total receives the sum.
-__device__ __forceinline__ unsigned long long block_excl_scan(uint32_t v, unsigned long long& total) {
-  __shared__ unsigned long long warpSum[kWarps];
-  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-  uint32_t wt;
-  const uint32_t pre = warp_excl_scan(v, wt);
-  if (lane == 0) warpSum[warp] = wt;
+__device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(kFull, v, d);
+  return v;
+}
+
+// The grid barrier between the phases and levels of the sweep: like the
+// derivation's level_barrier, without a leader, on three words in turn.  Block
+// 0 clears the set after the next (its word's arrivals have all been seen: the
+// blocks have arrived at this one) and notes the set that a later launch on
+// the same state starts with.
+__device__ bool adjoint_barrier(const DeriveArgs& a, Smem& sm) {
+  __shared__ int ok;
   __syncthreads();
-  unsigned long long before = 0, all = 0;
-  for (int w = 0; w < kWarps; w++) {
-    const unsigned long long x = warpSum[w];
-    before += (w < (int)warp) ? x : 0ull;
-    all += x;
+  if (threadIdx.x == 0) {
+    DevState* st = a.st;
+    uint32_t* word = &st->adjointWord[sm.turn];
+    __threadfence();
+    atomicAdd(word, 1u);
+    uint32_t seen;
+    ok = await_word<uint32_t>(a, word, 0xFFFFFFFFu, gridDim.x, seen) ? 1 : 0;
+    __threadfence();
+    sm.turn = sm.turn == 2 ? 0u : sm.turn + 1u;
+    if (blockIdx.x == 0) {
+      const uint32_t after = sm.turn == 2 ? 0u : sm.turn + 1u;
+      st->adjointWord[after] = 0;
+      st->adjointCursor[after] = 0;
+      st->adjointTurn = sm.turn;
+    }
   }
   __syncthreads();
-  total = all;
-  return before + pre;
+  return ok != 0;
 }
 
 __device__ __forceinline__ unsigned long long block_sum(unsigned long long v) {
@@ -1061,9 +1110,10 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v) {
 // Two launch shapes of the same pass.  k_adjoint runs 2 blocks of 256 per SM;
 // k_adjoint_wide (frame-code builds) 3, at 80 registers: on large tapes the
 // extra warps hide more of the scattered reads (1,500-axiom mix, 3.4M
-// terminals: 490 us with 2 blocks, 428 with 3, 472 with 4; 8,192 axioms with
-// blocks 2.21 / 2.08 / 2.33 ms), on small ones the spills and the larger
-// grid's barriers cost more (1,024 facades, 0.4M terminals: 78 / 93 / 104 us).
+// terminals: 490 us with 2 blocks against 428; now 354 with 3, 359 with 4, 463
+// with 5; 8,192 axioms with blocks 1.49 / 1.48 / 2.29 ms with 3 / 4 / 5), on
+// small ones the spills and the larger grid's barriers cost more (1,024
+// facades, 0.4M terminals: 66 / 74 / 83 us with 2 / 3 / 4).
 // Engines choose by terminal capacity (kWideAdjointTerminals, 2M).
 // PGA_ADJOINT_MIN_BLOCKS overrides k_adjoint's shape.
 #if defined(PGA_ADJOINT_MIN_BLOCKS)
@@ -1078,6 +1128,7 @@ __device__ __forceinline__ void adjoint_pass(const DeriveArgs& a, const AdjArgs&
   Smem& sm = *reinterpret_cast<Smem*>(smem_raw);
   setup_block(a, sm);
   volatile DevState* vs = a.st;
+  if (threadIdx.x == 0) sm.turn = vs->adjointTurn;  // read in adjoint_barrier, by the same thread, and after it
   // Fixed by the forward launch; nothing below changes them before the first barrier.
   const unsigned long long nodes = min((unsigned long long)vs->nodeNext, a.nodeCap);
   const unsigned long long nTerm = vs->termCount;
@@ -1089,26 +1140,38 @@ __device__ __forceinline__ void adjoint_pass(const DeriveArgs& a, const AdjArgs&
     for (unsigned long long k = tid; k < numParamFloats; k += stride) j.gradParams[k] = 0.0f;
   if (j.gradSizes)
     for (unsigned long long k = tid; k < (unsigned long long)numAxioms * 3; k += stride) j.gradSizes[k] = 0.0f;
-  // Each block owns a contiguous chunk of the work items, each thread a
-  // contiguous run of its block's chunk; loads go kUnroll at a time.
+  // Each block owns a contiguous chunk of the work items, each warp a
+  // contiguous run of its block's chunk in steps of 32, kUnroll steps' loads at
+  // a time.  The slot map reads the items' tape, 16 bytes an item, and not
+  // their records (64 bytes each time): 570 -> 230 us for 10M items and 19M
+  // terminals.
   constexpr int kUnroll = 4;
-  const unsigned long long chunk = (nodes + gridDim.x - 1) / gridDim.x;
-  const unsigned long long lo = min((unsigned long long)blockIdx.x * chunk, nodes), hi = min(lo + chunk, nodes);
-  const unsigned long long run = (hi - lo + kThreads - 1) / kThreads;
-  const unsigned long long tlo = min(lo + threadIdx.x * run, hi), thi = min(tlo + run, hi);
+  const unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const unsigned long long run = ((nodes + gridDim.x - 1) / gridDim.x + kThreads - 1) / kThreads * 32ull;
+  const unsigned long long wlo = min(((unsigned long long)blockIdx.x * kWarps + warp) * run, nodes);
+  const unsigned long long whi = min(wlo + run, nodes);
   uint32_t mine = 0;  // a work item has at most 64 children
-  for (unsigned long long i = tlo; i < thi; i += kUnroll) {
-    uint4 ext[kUnroll];
+  for (unsigned long long i = wlo + lane; i < whi; i += 32 * kUnroll) {
+    uint32_t count[kUnroll];
 #pragma unroll
-    for (int u = 0; u < kUnroll; u++)
-      ext[u] = i + u < thi ? __ldcg(reinterpret_cast<const uint4*>(a.nodes + i + u) + 3)
-                           : make_uint4(kEmptyItem, 0u, 0u, 0u);
+    for (int u = 0; u < kUnroll; u++) count[u] = i + 32 * u < whi ? __ldcg(&a.itemTape[i + 32 * u].x) : 0u;
 #pragma unroll
-    for (int u = 0; u < kUnroll; u++) mine += page_children(ext[u]);
+    for (int u = 0; u < kUnroll; u++) mine += count[u] & ~kOnlyPage;
   }
-  const unsigned long long blockTotal = block_sum(mine);
-  if (threadIdx.x == 0) j.blockSums[blockIdx.x] = blockTotal;
-  if (!grid_barrier(a, [] {})) return;
+  const unsigned long long warpTotal = warp_sum(mine);
+  __shared__ unsigned long long warpFirst[kWarps];  // then: children of the block's earlier warps
+  if (lane == 0) warpFirst[warp] = warpTotal;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned long long sum = 0;
+    for (int w = 0; w < kWarps; w++) {
+      const unsigned long long n = warpFirst[w];
+      warpFirst[w] = sum;
+      sum += n;
+    }
+    j.blockSums[blockIdx.x] = sum;
+  }
+  if (!adjoint_barrier(a, sm)) return;
   if (!ok) {
     if (tid == 0 && vs->status == 0) raise_error(a.st, PGA_ERR_NO_TAPE, -1);
     return;
@@ -1126,33 +1189,25 @@ __device__ __forceinline__ void adjoint_pass(const DeriveArgs& a, const AdjArgs&
     return;
   }
   for (unsigned long long k = tid; k < total; k += stride) j.slots[k] = kNoRecord;
-  {
-    unsigned long long ignored;
-    unsigned long long first = base + block_excl_scan(mine, ignored);
-    for (unsigned long long i = tlo; i < thi; i += kUnroll) {
-      uint4 m[kUnroll], ext[kUnroll];
+  unsigned long long first = base + warpFirst[warp];
+  for (unsigned long long i0 = wlo; i0 < whi; i0 += 32 * kUnroll) {
+    uint2 page[kUnroll];
 #pragma unroll
-      for (int u = 0; u < kUnroll; u++) {
-        const uint4* rec = reinterpret_cast<const uint4*>(a.nodes + min(i + u, thi - 1));
-        m[u] = __ldcg(rec + 2);
-        ext[u] = __ldcg(rec + 3);
-      }
+    for (int u = 0; u < kUnroll; u++) {
+      const unsigned long long i = i0 + 32 * u + lane;
+      page[u] = i < whi ? __ldcg(reinterpret_cast<const uint2*>(a.itemTape + i)) : make_uint2(0u, 0u);
+    }
 #pragma unroll
-      for (int u = 0; u < kUnroll; u++) {
-        if (i + u >= thi) break;
-        const uint32_t cnt = page_children(ext[u]);
-        uint32_t key = 0;
-        if (cnt) {
-          const int32_t e = (int32_t)m[u].x;
-          const bool rep = e >= 0 && (uint32_t)e < a.tab.numEntries && rule_at(a, (uint32_t)e).op == PGA_OP_REPEAT;
-          key = (uint32_t)0u - ext[u].x - (rep ? 1u : 0u);
-        }
-        j.childKey[i + u] = (uint32_t)first + key;
-        first += cnt;
-      }
+    for (int u = 0; u < kUnroll; u++) {
+      const unsigned long long i = i0 + 32 * u + lane;
+      uint32_t all;
+      const uint32_t before = warp_excl_scan(page[u].x & ~kOnlyPage, all);
+      const uint32_t key = (uint32_t)first + before - page[u].y;
+      if (i < whi) j.childKey[i] = key;
+      first += all;
     }
   }
-  if (!grid_barrier(a, [] {})) return;
+  if (!adjoint_barrier(a, sm)) return;
   for (unsigned long long t0 = tid; t0 < nTerm; t0 += stride * kUnroll) {
     uint2 link[kUnroll];
     uint32_t key[kUnroll];
@@ -1178,36 +1233,42 @@ __device__ __forceinline__ void adjoint_pass(const DeriveArgs& a, const AdjArgs&
     }
   }
   for (unsigned long long i0 = tid; i0 < nodes; i0 += stride * kUnroll) {
-    uint4 ext[kUnroll];
+    uint4 page[kUnroll];
     uint32_t key[kUnroll];
 #pragma unroll
     for (int u = 0; u < kUnroll; u++) {
       const unsigned long long i = i0 + u * stride;
-      ext[u] = i < nodes ? __ldcg(reinterpret_cast<const uint4*>(a.nodes + i) + 3) : make_uint4(kEmptyItem, 0u, 0u, 0u);
+      page[u] = i < nodes ? __ldcg(a.itemTape + i) : make_uint4(0u, 0u, kAxiomLink, 0u);
     }
 #pragma unroll
-    for (int u = 0; u < kUnroll; u++) {
-      const bool take = ext[u].x != kEmptyItem && !(ext[u].z & kAxiomLink) && ext[u].z < nodes;
-      ext[u].x = take ? 0u : kEmptyItem;
-      key[u] = take ? __ldcg(j.childKey + ext[u].z) : 0u;
-    }
+    for (int u = 0; u < kUnroll; u++)  // (an axiom's root item and an empty slot carry kAxiomLink)
+      key[u] = page[u].z < nodes ? __ldcg(j.childKey + page[u].z) : 0u;
 #pragma unroll
     for (int u = 0; u < kUnroll; u++) {
-      if (ext[u].x == kEmptyItem) continue;
+      if (page[u].z >= nodes) continue;
       const unsigned long long i = i0 + u * stride;
-      const uint32_t head = atomicExch(j.slots + (uint32_t)(key[u] + ext[u].w), kItemTag | (uint32_t)i);
-      j.pageNext[i] = head == kNoRecord ? kNoRecord : (head & ~kItemTag);
+      uint32_t* slot = j.slots + (uint32_t)(key[u] + page[u].w);
+      if (page[u].x & kOnlyPage) {
+        *slot = kItemTag | (uint32_t)i;
+        j.pageNext[i] = kNoRecord;
+      } else {
+        const uint32_t head = atomicExch(slot, kItemTag | (uint32_t)i);
+        j.pageNext[i] = head == kNoRecord ? kNoRecord : (head & ~kItemTag);
+      }
     }
   }
   // The levels, last first.  A level of at least four rounds of the grid
   // leaves its last 1 / PGA_ADJOINT_DYNAMIC_SHARE (at least two rounds) to
-  // warps that take 32 items at a time from DevState::cursor, reset at each
-  // barrier: pages differ widely in cost, and the gradients are sums of
-  // atomics whose order was never fixed, so the order of the pages changes
-  // nothing a caller sees.
-  if (!grid_barrier(a, [&] { a.st->cursor = 0ull; })) return;
+  // warps that take 32 items at a time from the level's cursor: pages differ
+  // widely in cost, and the gradients are sums of atomics whose order was never
+  // fixed, so the order of the pages changes nothing a caller sees.
+  unsigned long long lvNext = a.levelStart[levels];  // ahead of the barrier
+  if (!adjoint_barrier(a, sm)) return;
+  unsigned long long hvNext = nodes;
   for (int L = (int)levels; L >= 0; L--) {
-    const unsigned long long lv = a.levelStart[L], hv = min(a.levelStart[L + 1], nodes);
+    const unsigned long long lv = lvNext, hv = hvNext;
+    hvNext = min(lv, nodes);
+    if (L > 0) lvNext = a.levelStart[L - 1];
     if (lv >= hv) continue;  // every block reads the same bounds, so all skip the barrier alike
     const uint32_t shift = share_shift(hv - lv);
     if (shift > 0) {  // a narrow level: 2^shift lanes to an item
@@ -1224,10 +1285,10 @@ __device__ __forceinline__ void adjoint_pass(const DeriveArgs& a, const AdjArgs&
         if (i >= dynLo) {
           if (dynLo >= hv) break;
           unsigned long long c = 0;
-          if ((threadIdx.x & 31u) == 0) c = atomicAdd(&a.st->cursor, 32ull);
+          if (lane == 0) c = atomicAdd(&a.st->adjointCursor[sm.turn], 32ull);
           c = dynLo + __shfl_sync(kFull, c, 0);
           if (c >= hv) break;
-          i = c + (threadIdx.x & 31u);  // the loop step never lands below dynLo again
+          i = c + lane;  // the loop step never lands below dynLo again
           if (i >= hv) continue;        // this lane has no item in the last chunk
         } else if (i + stride < dynLo) {  // the next item's record and key, ahead of its turn
           prefetch_l2(a.nodes + i + stride);
@@ -1236,7 +1297,7 @@ __device__ __forceinline__ void adjoint_pass(const DeriveArgs& a, const AdjArgs&
         adj_sums(a, j, i, true, nodes, 0, 0);
       }
     }
-    if (!grid_barrier(a, [&] { a.st->cursor = 0ull; })) return;
+    if (L > 0 && !adjoint_barrier(a, sm)) return;
   }
 }
 

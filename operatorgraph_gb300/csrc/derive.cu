@@ -76,6 +76,7 @@ DeriveArgs make_args(PgaEngine* e, const PgaAxiom* axioms, uint32_t numAxioms, c
   a.nodeRot = e->dNodeRot;
   a.nodeCap = e->cfg.nodeCapacity;
   a.termLinks = e->dTermLinks;
+  a.itemTape = e->dItemTape;
   a.termLinkCap = e->dTermLinks ? e->cfg.maxTerminals : 0;
   a.levelStart = e->dLevelStart;
   a.levelClock = e->dLevelClock;
@@ -227,7 +228,7 @@ static void free_engine(PgaEngine* e) {
     if (p) cudaFree(p);
   void* ptrs[] = {e->dRules, e->dParams, e->dSucc, e->dExpPool, e->dState, e->dNodes, e->dNodeRot, e->dLevelClock,
                   e->dTail, e->dTailLinks, e->dScratch,
-                  e->dTermLinks, e->dLevelStart, e->dScratchCount, e->dSortTemp, e->dKeysA,
+                  e->dTermLinks, e->dItemTape, e->dLevelStart, e->dScratchCount, e->dSortTemp, e->dKeysA,
                   e->dValsA, e->dValsB, e->dOpenTrees, e->dNodeGrad, e->dChildKey, e->dPageNext,
                   e->dSlots, e->dBlockSums, e->dGroupCount};
   for (void* p : ptrs)
@@ -535,6 +536,7 @@ PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* co
     }
     e->slotCap = std::min<unsigned long long>(c.nodeCapacity * std::max(c.subItem, c.narrowSubItem), 0xFFFFFFF0ull);
     ALLOC(e->dTermLinks, c.maxTerminals * sizeof(uint2));
+    ALLOC(e->dItemTape, c.nodeCapacity * sizeof(uint4));
     ALLOC(e->dNodeGrad, c.nodeCapacity * 6 * sizeof(float));
     ALLOC(e->dChildKey, c.nodeCapacity * sizeof(uint32_t));
     ALLOC(e->dPageNext, c.nodeCapacity * sizeof(uint32_t));
@@ -1040,6 +1042,7 @@ PgaStatus pga_derive_plain(PgaEngine* e, const PgaAxiom* dAxioms, uint32_t numAx
   PGA_CUDA_TRY(cudaMemsetAsync(e->dState, 0, sizeof(DevState), s));
   DeriveArgs a = make_args(e, dAxioms, numAxioms, dParamBlocks, dOut, capacity, (unsigned long long*)dCount);
   a.termLinks = nullptr;
+  a.itemTape = nullptr;
   const unsigned threads = (unsigned)e->threads;
   for (uint32_t ax = 0; ax < numAxioms; ax++) {
     // One grammar (axiom) at a time: reset the queue, seed, expand level by level.

@@ -1098,7 +1098,12 @@ __device__ __forceinline__ void emit_round(const DeriveArgs& a, WarpOut& w, int 
         raise_error(a.st, PGA_ERR_QUEUE_OVERFLOW, -1);
         break;
       }
-      store_node(a, slot, y, make_uint4(j * S, min((j + 1) * S, nChild), link, ordinal));
+      const uint32_t c0 = j * S, c1 = min((j + 1) * S, nChild);
+      store_node(a, slot, y, make_uint4(c0, c1, link, ordinal));
+      if (PAGED && a.itemTape != nullptr) {
+        const uint32_t first = c0 + (rule_at(a, (uint32_t)y.entry).op == PGA_OP_REPEAT ? 1u : 0u);
+        __stcg(a.itemTape + slot, make_uint4((c1 - c0) | (m == 1u ? kOnlyPage : 0u), first, link, ordinal));
+      }
     }
   }
 }
@@ -1111,7 +1116,10 @@ __device__ __forceinline__ void close_node_page(const DeriveArgs& a, WarpOut& w)
   for (uint32_t k = lane; k < w.nLeft; k += 32) {
     const unsigned long long slot = w.nNext + k;
     if (slot < a.nodeCap)
+    {
       __stcg(reinterpret_cast<uint4*>(a.nodes + slot) + 3, make_uint4(kEmptyItem, 0u, 0u, 0u));
+      if (a.itemTape != nullptr) __stcg(a.itemTape + slot, make_uint4(0u, 0u, kAxiomLink, 0u));
+    }
   }
   w.nLeft = 0;
 }
@@ -1418,42 +1426,26 @@ __device__ __forceinline__ void setup_block(const DeriveArgs& a, Smem& sm) {
   __syncthreads();
 }
 
-// ---------------------------------------------------- bounded grid barrier
+// --------------------------------------------------- bounded grid barriers
 
-// Thread 0 of every block arrives; the last arriver runs `leader()` and
-// releases the others.  Waits are bounded by spinLimit; a timeout raises
-// PGA_ERR_TIMEOUT and makes the caller leave the kernel.
-template <typename Leader>
-__device__ bool grid_barrier(const DeriveArgs& a, Leader leader) {
-  __shared__ int ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    ok = 1;
-    DevState* st = a.st;
-    volatile uint32_t* gen = &st->barrierGen;
-    uint32_t g = *gen;
-    __threadfence();
-    uint32_t prev = atomicAdd(&st->barrierArrive, 1u);
-    if (prev == gridDim.x - 1) {
-      atomicExch(&st->barrierArrive, 0u);
-      leader();
-      __threadfence();
-      atomicAdd(&st->barrierGen, 1u);
-    } else {
-      uint32_t spins = 0;
-      while (*gen == g) {
-        if (++spins > a.spinLimit) {
-          raise_error(st, PGA_ERR_TIMEOUT, -1);
-          ok = 0;
-          break;
-        }
-        __nanosleep(32);
-      }
+// Waits until `arrivals` (a value of *word masked by `mask`) are in; false when
+// spinLimit polls were not enough (raises PGA_ERR_TIMEOUT).  The polls are
+// relaxed: an acquire would empty the L1 of the SM's other blocks, still at
+// work, at every poll (16,384 trees tested for collisions: 107 -> 188 us).
+template <typename Word>
+__device__ __forceinline__ bool await_word(const DeriveArgs& a, const Word* word, Word mask, Word arrivals, Word& seen) {
+  for (uint32_t spins = 0;;) {
+    if constexpr (sizeof(Word) == 8)
+      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(word) : "memory");
+    else
+      asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(word) : "memory");
+    if ((seen & mask) == arrivals) return true;
+    if (++spins > a.spinLimit) {
+      raise_error(a.st, PGA_ERR_TIMEOUT, -1);
+      return false;
     }
-    __threadfence();
+    __nanosleep(32);
   }
-  __syncthreads();
-  return ok != 0;
 }
 
 // The end of a level: every block adds its arrival, whether it had seen a
@@ -1478,20 +1470,7 @@ __device__ bool level_barrier(const DeriveArgs& a, Smem& sm) {
     __threadfence();
     atomicAdd(word, mine);
     unsigned long long seen;
-    uint32_t spins = 0;
-    int good = 1;
-    for (;;) {
-      // relaxed: an acquire would empty the L1 of the SM's other block, still at
-      // work, at every poll (16,384 trees tested for collisions: 107 -> 188 us)
-      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(seen) : "l"(word) : "memory");
-      if ((seen & ((1u << kArriveBits) - 1u)) == gridDim.x) break;
-      if (++spins > a.spinLimit) {
-        raise_error(st, PGA_ERR_TIMEOUT, -1);
-        good = 0;
-        break;
-      }
-      __nanosleep(32);
-    }
+    const bool good = await_word<unsigned long long>(a, word, (1u << kArriveBits) - 1u, gridDim.x, seen);
     __threadfence();
     const unsigned long long lo = min(sm.levelBase, a.nodeCap);
     sm.levelBase += seen >> 32;
@@ -1500,7 +1479,7 @@ __device__ bool level_barrier(const DeriveArgs& a, Smem& sm) {
     sm.turn = sm.turn == 2 ? 0u : sm.turn + 1u;
     sm.taken = 0;
     sm.stop = ((seen >> kArriveBits) & 0xFFFFull) != 0 ? 1 : 0;
-    ok = good;
+    ok = good ? 1 : 0;
   }
   __syncthreads();
   return ok != 0;

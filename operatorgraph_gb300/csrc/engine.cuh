@@ -54,6 +54,7 @@ namespace pga {
 
 constexpr int kMaxChain = 64;           // inline 1->1 steps before PGA_ERR_DEPTH
 constexpr uint32_t kAxiomLink = 0x80000000u;
+constexpr uint32_t kOnlyPage = 0x80000000u;
 
 // ------------------------------------------------------------ device tables
 
@@ -109,15 +110,17 @@ struct DevState {
   unsigned long long termCount;   // terminals emitted (exact, after compaction in the paged engine)
   unsigned long long nodeNext;    // queued item slots handed out
   unsigned long long termPages;   // terminal pages handed out (paged engine)
-  unsigned long long cursor;      // next dynamic chunk of the level the adjoint is sweeping
   unsigned long long maxLevelNodes;
   int32_t status, detail;
-  uint32_t barrierArrive, barrierGen;
   uint32_t levels, reserved;
   // Paged engine, one set per level in turn (see level_barrier): item slots
   // handed out while it is expanded, its next dynamic chunk
   // (PGA_FLAG_DYNAMIC_CHUNKS), and the arrivals at its end.
   unsigned long long levelSlots[3], levelCursor[3], levelWord[3];
+  // The adjoint's (see adjoint_barrier): arrivals and the next dynamic chunk,
+  // and the set that its next launch starts with.
+  unsigned long long adjointCursor[3];
+  uint32_t adjointWord[3], adjointTurn;
   unsigned long long clockStart;  // %globaltimer when block 0 started (paged engine)
   unsigned long long clockEnd;    // %globaltimer when the last block finished
 };
@@ -138,6 +141,11 @@ struct DeriveArgs {
   float4* nodeRot;           // general frames: rotation entries 0..7 of each item (2 x float4; entry 8 in Node::sf.w)
   uint2* termLinks;
   unsigned long long termLinkCap;
+  // Tape of the work items, apart from their 64-byte records so that the
+  // adjoint's slot map reads 16 bytes an item: children (kOnlyPage: all of the
+  // shape's), ordinal of the first less its slot (see the slot map), tape link
+  // (parent item or kAxiomLink | axiom), the shape's ordinal there.
+  uint4* itemTape;
   unsigned long long* levelStart;
   unsigned long long* levelClock;  // %globaltimer when each level's range was fixed
   uint32_t maxLevels;

@@ -61,6 +61,7 @@ struct PgaEngine {
   uint64_t phaseTerminalsHost = 0;             // its copy for the device count
   uint32_t phasesRun = 0;
   uint2* dTermLinks = nullptr;
+  uint4* dItemTape = nullptr;
   unsigned long long* dLevelStart = nullptr;
   unsigned long long* dLevelClock = nullptr;
   unsigned long long* dScratchCount = nullptr;

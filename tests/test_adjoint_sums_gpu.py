@@ -135,3 +135,28 @@ def test_the_two_launch_shapes_agree(blocks):
         eng.release()
     for x, y in zip(*grads):  # up to 10^4 terminals an axiom
         assert np.abs(y).max() > 0 and np.abs(x - y).max() <= 1e-4 * np.abs(y).max()
+
+
+def test_one_tape_serves_many_reverse_passes():
+    """The reverse launches of one derivation share their barrier words: more launches than there are words."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from operatorgraph_gb300 import scenes
+    from operatorgraph_gb300.autograd import axioms_tensor
+    from operatorgraph_gb300.engine import Engine
+
+    b = scenes.city(50)
+    axioms = axioms_tensor(b["axioms"])
+    eng = Engine(b["entries"], node_capacity=1 << 20, max_terminals=1 << 18, record_tape=True)
+    out, _, _ = eng.execute(axioms, capacity=1 << 18)
+    grads = []
+    for _ in range(7):
+        g = torch.full((50, 3), float("nan"), device="cuda")
+        eng.adjoint_raw(out.data_ptr(), None, 0, g.data_ptr(), grad_stride=16)
+        torch.cuda.synchronize()
+        assert eng.report()["status"] == 0
+        grads.append(g.cpu().numpy().astype(np.float64))
+    eng.release()
+    for g in grads[1:]:  # one building's terminals in another order of summation
+        assert np.abs(g - grads[0]).max() <= 1e-5 * np.abs(grads[0]).max()
