@@ -35,6 +35,26 @@ __device__ __forceinline__ uint32_t spread(uint32_t v) {
   return v;
 }
 
+// The kernels of a small build (kSmallSort) are launched with programmatic
+// stream serialization: a kernel's blocks may be placed while the last ones of
+// the kernel before are still running, so its launch and whatever it does
+// ahead of await_previous (shared memory only) hide behind them.  Every thread
+// passes await_previous before it touches global memory, which makes the whole
+// chain's stores visible, as with ordinary launches.  20,011 leaves: 66 -> 55
+// us.  Large builds lose by it (3.0M leaves 386 -> 418 us): the waiting blocks
+// take the places of blocks with work.
+__device__ __forceinline__ void allow_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// A buffer that an earlier kernel of the chain writes, as the pointer to read
+// it through after the wait: opaque to the compiler, so that no load through it
+// moves ahead of the wait or becomes a read-only (non-coherent) one, which the
+// buffer is not while the waiting kernel already runs.
+template <typename T>
+__device__ __forceinline__ const T* written(const T* p) {
+  asm volatile("" : "+l"(p) : : "memory");
+  return p;
+}
+
 struct Bounds {
   float mn[3];
   float sz[3];
@@ -132,6 +152,7 @@ __global__ void __launch_bounds__(HIST ? kHistThreads : kLbvhThreads)
     k_morton(const PgaTerminal* __restrict__ t, unsigned long long cap, const unsigned long long* __restrict__ dN,
              Bounds b, uint32_t* __restrict__ codes, uint16_t* __restrict__ hashes, uint32_t* __restrict__ hist) {
   __shared__ uint32_t sh[HIST ? kSortPasses * kBins : 1];
+  allow_next();
   if (HIST) {
     for (uint32_t k = threadIdx.x; k < kSortPasses * kBins; k += kHistThreads) sh[k] = 0u;
     __syncthreads();
@@ -224,17 +245,19 @@ __device__ __forceinline__ unsigned long long pair_word(uint32_t flag, uint32_t 
 // groups[g][bin] the group's total.
 constexpr uint32_t kSortGroups = 304;  // two blocks on each of 152 SMs
 template <bool FIRST>
-__global__ void __launch_bounds__(kSortThreads) k_sort_count(const uint32_t* __restrict__ codes,
-                                                             const uint16_t* __restrict__ hashes, unsigned long long n,
-                                                             uint32_t shift, uint32_t tiles, uint32_t perGroup,
-                                                             uint32_t* __restrict__ rows,
-                                                             uint32_t* __restrict__ groups) {
+__global__ void __launch_bounds__(kSortThreads) k_sort_count(const uint32_t* codes, const uint16_t* hashes,
+                                                             unsigned long long n, uint32_t shift, uint32_t tiles,
+                                                             uint32_t perGroup, uint32_t* rows, uint32_t* groups) {
   constexpr uint32_t kTileItems = kSortThreads * kLargeItems;
   __shared__ uint32_t sh[kBins];
   const uint32_t first = blockIdx.x * perGroup, last = min(tiles, first + perGroup);
   uint2* bins = reinterpret_cast<uint2*>(sh) + threadIdx.x;
   uint2 run = make_uint2(0u, 0u);
+  allow_next();
   *bins = run;
+  await_previous();
+  codes = written(codes);
+  hashes = written(hashes);
   __syncthreads();
   for (uint32_t tile = first; tile < last; tile++) {
     const unsigned long long base = (unsigned long long)tile * kTileItems;
@@ -245,16 +268,16 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_count(const uint32_t* __r
       const uint32_t x = (k * kSortThreads + threadIdx.x) * 4u;
       if (x + 4 <= count) {
         if (FIRST) {
-          const ushort4 h = __ldg(reinterpret_cast<const ushort4*>(hashes + base + x));
+          const ushort4 h = *reinterpret_cast<const ushort4*>(hashes + base + x);
           d[k * 4 + 0] = h.x; d[k * 4 + 1] = h.y; d[k * 4 + 2] = h.z; d[k * 4 + 3] = h.w;
         } else {
-          const uint4 c = __ldg(reinterpret_cast<const uint4*>(codes + base + x));
+          const uint4 c = *reinterpret_cast<const uint4*>(codes + base + x);
           d[k * 4 + 0] = c.x; d[k * 4 + 1] = c.y; d[k * 4 + 2] = c.z; d[k * 4 + 3] = c.w;
         }
       } else {
 #pragma unroll
         for (int u = 0; u < 4; u++)
-          d[k * 4 + u] = x + u < count ? (FIRST ? (uint32_t)__ldg(hashes + base + x + u) : __ldg(codes + base + x + u)) : 0u;
+          d[k * 4 + u] = x + u < count ? (FIRST ? (uint32_t)hashes[base + x + u] : codes[base + x + u]) : 0u;
       }
     }
 #pragma unroll
@@ -276,11 +299,13 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_count(const uint32_t* __r
 // groups[g][bin] becomes the bin's count in the groups before g, totals[bin]
 // its count in all.  A block of 32 x 32 threads per 32 bins: lane = bin, each
 // warp a run of ten groups.
-__global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* __restrict__ groups, uint32_t* __restrict__ totals) {
+__global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* groups, uint32_t* totals) {
   constexpr uint32_t kPer = (kSortGroups + 31) / 32;
   __shared__ uint32_t sSum[32][33];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint32_t* col = groups + blockIdx.x * 32u + lane;
+  allow_next();
+  await_previous();
   uint32_t v[kPer], sum = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kPer; k++) {
@@ -303,22 +328,22 @@ __global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* __restrict__ group
 }
 
 struct SortPass {
-  const uint32_t* __restrict__ codesIn;
-  const uint16_t* __restrict__ hashes;
-  const uint32_t* __restrict__ valsIn;
-  uint32_t* __restrict__ codesOut;
-  uint32_t* __restrict__ valsOut;
+  const uint32_t* codesIn;
+  const uint16_t* hashes;
+  const uint32_t* valsIn;
+  uint32_t* codesOut;
+  uint32_t* valsOut;
   unsigned long long n;
   uint32_t shift;
-  const uint32_t* __restrict__ hist;  // the pass's digit counts
+  const uint32_t* hist;  // the pass's digit counts
   // the look-back's words and the tiles' counter
   unsigned long long* status;
   uint32_t* tileCounter;
   int* err;
   uint32_t spinLimit;
   // COUNTED: the rows of k_sort_count and the groups of k_sort_scan (perGroup tiles each)
-  const uint32_t* __restrict__ rows;
-  const uint32_t* __restrict__ groups;
+  const uint32_t* rows;
+  const uint32_t* groups;
   uint32_t perGroup;
 };
 
@@ -339,7 +364,7 @@ __device__ __forceinline__ void sort_tile(const SortPass& a, uint32_t tile, uint
   uint16_t* mine = sHist + warp * kHistStride;
   uint32_t* match = sCodes + warp * kBins;  // while the warps rank: per digit the lanes that have it
   const unsigned long long tileBase = (unsigned long long)tile * kTileItems;
-  const uint32_t* __restrict__ codesIn = a.codesIn + tileBase;
+  const uint32_t* codesIn = a.codesIn + tileBase;
   const uint32_t shift = a.shift;
   const uint32_t local = warp * (32u * ITEMS) + lane;  // + 32 k: this thread's entries in the tile
   unsigned lt;
@@ -421,8 +446,8 @@ __device__ __forceinline__ void sort_tile(const SortPass& a, uint32_t tile, uint
   // decoupled look-back.
   uint32_t prefix0 = 0, prefix1 = 0;
   if (COUNTED) {
-    const uint2 r = __ldg(reinterpret_cast<const uint2*>(a.rows + (size_t)tile * kBins) + threadIdx.x);
-    const uint2 g = __ldg(reinterpret_cast<const uint2*>(a.groups + (size_t)(tile / a.perGroup) * kBins) + threadIdx.x);
+    const uint2 r = reinterpret_cast<const uint2*>(a.rows + (size_t)tile * kBins)[threadIdx.x];
+    const uint2 g = reinterpret_cast<const uint2*>(a.groups + (size_t)(tile / a.perGroup) * kBins)[threadIdx.x];
     prefix0 = r.x + g.x;
     prefix1 = r.y + g.y;
   }
@@ -505,14 +530,23 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort_pass(SortPass a) {
   constexpr uint32_t kTileItems = kSortThreads * ITEMS;
   extern __shared__ __align__(16) unsigned char smem_sort[];
   __shared__ uint32_t sTile;
-  if (!COUNTED && threadIdx.x == 0) sTile = atomicAdd(a.tileCounter, 1u);
-  const uint2 all = __ldg(reinterpret_cast<const uint2*>(a.hist) + threadIdx.x);  // this thread's bins, whole input
+  allow_next();
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint16_t* mine = reinterpret_cast<uint16_t*>(smem_sort + sort_entry_bytes(ITEMS)) + warp * kHistStride;
   for (uint32_t k = lane; k < kBins / 8; k += 32) reinterpret_cast<uint4*>(mine)[k] = make_uint4(0u, 0u, 0u, 0u);
   if (!COUNTED) {
     uint32_t* match = reinterpret_cast<uint32_t*>(smem_sort) + warp * kBins;
     for (uint32_t k = lane; k < kBins / 4; k += 32) reinterpret_cast<uint4*>(match)[k] = make_uint4(0u, 0u, 0u, 0u);
+  }
+  await_previous();
+  a.codesIn = written(a.codesIn);
+  a.hashes = written(a.hashes);
+  a.valsIn = written(a.valsIn);
+  a.rows = written(a.rows);
+  a.groups = written(a.groups);
+  const uint2 all = reinterpret_cast<const uint2*>(written(a.hist))[threadIdx.x];  // this thread's bins, whole input
+  if (!COUNTED) {
+    if (threadIdx.x == 0) sTile = atomicAdd(a.tileCounter, 1u);
     __syncthreads();
   } else {
     __syncwarp();  // the warp's histogram is clear
@@ -698,7 +732,7 @@ __device__ __forceinline__ uint32_t open_rank(const uint32_t* open, int e) {
 // The terminal index at sorted position i (bounded by the leaf count, should a
 // look-back wait of the sort have given up and left old contents).
 __device__ __forceinline__ uint32_t leaf_value(const TreeArgs& a, unsigned long long i, unsigned long long n) {
-  return min(__ldg(a.vals + i), (uint32_t)n - 1u);
+  return min(*(a.vals + i), (uint32_t)n - 1u);
 }
 
 // The leaves' final order.  The radix sort orders the Morton code and the path
@@ -735,14 +769,14 @@ __device__ __forceinline__ void tie_run(const uint32_t* eq, int q, int& s, int& 
 
 // What the sort ordered at position i: Morton code, then hash digit.
 __device__ __forceinline__ uint64_t tie_key(const TreeArgs& a, unsigned long long n, unsigned long long i) {
-  return ((uint64_t)__ldg(a.codes + i) << kRadixBits) | (term_path(a.t, leaf_value(a, i, n)) >> kHashShift);
+  return ((uint64_t)*(a.codes + i) << kRadixBits) | (term_path(a.t, leaf_value(a, i, n)) >> kHashShift);
 }
 
 // Whether the leaf at position i has code c and hash digit h; its value and
 // path when the code agrees.
 __device__ __forceinline__ bool tie_leaf(const TreeArgs& a, unsigned long long n, unsigned long long i, uint32_t c,
                                          uint32_t h, uint32_t& val, uint64_t& path) {
-  if (__ldg(a.codes + i) != c) return false;
+  if (*(a.codes + i) != c) return false;
   val = leaf_value(a, i, n);
   path = term_path(a.t, val);
   return (uint32_t)(path >> kHashShift) == h;
@@ -815,6 +849,10 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
   TieWindow& win = *reinterpret_cast<TieWindow*>(sNodeBox);
   uint64_t* fPath = reinterpret_cast<uint64_t*>(sNodeBox + sizeof(TieWindow) / 4);
   static_assert(sizeof(TieWindow) + kTile * 8 <= kTile * 24, "window and paths in the node boxes' place");
+  allow_next();
+  await_previous();
+  a.codes = written(a.codes);
+  a.vals = written(a.vals);
   const unsigned long long n = leaf_count(a.dN, a.cap);
   const unsigned long long base = (unsigned long long)blockIdx.x * kTile;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -829,11 +867,11 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
   uint64_t path = 0;
   float mn[3], mx[3];
   if (valid) {
-    code = __ldg(a.codes + k);
+    code = *(a.codes + k);
     val = leaf_value(a, k, n);
     int d = -1;
     if (k > 0) {
-      before = __ldg(a.codes + k - 1);
+      before = *(a.codes + k - 1);
       d = boundary_delta(before, code, (uint32_t)k);
     }
     sDelta[tid] = (signed char)d;
@@ -848,7 +886,7 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
   if (tid == cnt - 1) {  // the tile's right end
     int d = -1;
     if (k + 1 < n) {
-      const uint32_t after = __ldg(a.codes + k + 1);
+      const uint32_t after = *(a.codes + k + 1);
       d = boundary_delta(code, after, (uint32_t)(k + 1));
       sameEnd = after == code;  // then cnt == kTile
     }
@@ -895,7 +933,7 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
         if (more) atomicOr(&sLong, 1);
       }
     } else if (warp == 1 && (sEq[kWindowWords - 1] & 1u)) {
-      const uint32_t c = __ldg(a.codes + base + kTile - 1);
+      const uint32_t c = *(a.codes + base + kTile - 1);
       const uint32_t h = (uint32_t)(win.path[kHalo + kTile - 1] >> kHashShift);
       const unsigned long long i = base + kTile + lane;
       const bool in = i < n && tie_leaf(a, n, min(i, n - 1), c, h, val, hPath);
@@ -1136,6 +1174,10 @@ __global__ void __launch_bounds__(kTile) k_join(TreeArgs a) {
   __shared__ uint32_t sAt[kGroup];
   __shared__ uint32_t sCount, sTaken, sLast;
   signed char* delta = sMin[0];
+  await_previous();
+  a.codes = written(a.codes);
+  a.open = const_cast<OpenTree*>(written(a.open));
+  a.openCount = const_cast<uint32_t*>(written(a.openCount));
   const unsigned long long n = leaf_count(a.dN, a.cap);
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
   if (n <= (unsigned long long)blockIdx.x * kGroup * kTile || n <= kTile) return;
@@ -1186,7 +1228,7 @@ __global__ void __launch_bounds__(kTile) k_join(TreeArgs a) {
       if (tid == 0) {
         const unsigned long long end = min(n, (first + next) * stride * kTile);
         sLeft[count] = (uint32_t)end;
-        delta[count] = (signed char)(end < n ? boundary_delta(__ldg(a.codes + end - 1), __ldg(a.codes + end), (uint32_t)end)
+        delta[count] = (signed char)(end < n ? boundary_delta(*(a.codes + end - 1), *(a.codes + end), (uint32_t)end)
                                              : -1);
       }
       __syncthreads();
@@ -1391,6 +1433,24 @@ struct LbvhScratch {
 // Polls of a look-back wait before it gives up (each followed by a 32 ns sleep).
 constexpr uint32_t kSortSpinLimit = 1u << 22;
 
+// Launches a kernel of a build behind the one before it; early: with its blocks
+// placed ahead of that one's end (see await_previous).
+template <typename... Params, typename... Args>
+static cudaError_t launch_behind(bool early, void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem,
+                                 cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
+}
+
 struct SortBuffers {
   uint32_t *codesA, *codesB;
   const uint16_t* hashes;
@@ -1419,17 +1479,15 @@ static PgaStatus launch_sort_pass(int q, unsigned long long n, const SortBuffers
   uint32_t* groups = rows + (size_t)tiles * kBins;
   const uint32_t perGroup = (tiles + kSortGroups - 1) / kSortGroups;
   if (!SMALL) {
-    k_sort_count<FIRST><<<kSortGroups, kSortThreads, 0, s>>>(cIn, b.hashes, n, shift, tiles, perGroup, rows, groups);
-    PGA_CUDA_TRY(cudaGetLastError());
-    k_sort_scan<<<kBins / 32, 1024, 0, s>>>(groups, hist);
-    PGA_CUDA_TRY(cudaGetLastError());
+    PGA_CUDA_TRY(launch_behind(false, k_sort_count<FIRST>, kSortGroups, kSortThreads, 0, s, cIn, b.hashes, n, shift, tiles,
+                               perGroup, rows, groups));
+    PGA_CUDA_TRY(launch_behind(false, k_sort_scan, kBins / 32, 1024, 0, s, groups, hist));
   }
   PGA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const SortPass a{cIn, b.hashes, vIn, cOut, vOut, n, shift, hist,
                    reinterpret_cast<unsigned long long*>(b.words) + (SMALL ? (size_t)q * tiles * (kBins / 2) : 0),
                    b.counters + q, b.err, kSortSpinLimit, rows, groups, perGroup};
-  kernel<<<tiles, kSortThreads, smem, s>>>(a);
-  PGA_CUDA_TRY(cudaGetLastError());
+  PGA_CUDA_TRY(launch_behind(SMALL, +kernel, tiles, kSortThreads, smem, s, a));
   return PGA_OK;
 }
 
@@ -1486,12 +1544,8 @@ static PgaStatus launch_lbvh(const PgaTerminal* t, unsigned long long cap, const
   const TreeArgs a{codesA, w.valsA, t, cap, dN, out->nodes, out->leafParents, out->aabbs, out->leafTerminal,
                    (unsigned long long*)out->keys, open,
                    reinterpret_cast<uint32_t*>(open + (size_t)blocks * kMaxOpen), joins};
-  k_tree<<<blocks, kTile, 0, s>>>(a);
-  PGA_CUDA_TRY(cudaGetLastError());
-  if (blocks > 1) {
-    k_join<<<(blocks + kGroup - 1) / kGroup, kTile, 0, s>>>(a);
-    PGA_CUDA_TRY(cudaGetLastError());
-  }
+  PGA_CUDA_TRY(launch_behind(small, k_tree, blocks, kTile, 0, s, a));
+  if (blocks > 1) PGA_CUDA_TRY(launch_behind(small, k_join, (blocks + kGroup - 1) / (unsigned)kGroup, kTile, 0, s, a));
   return PGA_OK;
 }
 
