@@ -66,26 +66,21 @@ struct Bounds {
 // smallest corner sum is the sum with every term negative and the largest the
 // one with every term positive; where those are finite so is every corner, and
 // the eight corners need not be formed.
-__device__ __noinline__ void leaf_aabb_corners(float4 r0, float4 r1, float4 r2, bool quad, float mn[3], float mx[3]) {
-  const float4 r[3] = {r0, r1, r2};
-#pragma unroll
-  for (int k = 0; k < 3; k++) { mn[k] = FLT_MAX; mx[k] = -FLT_MAX; }
+// (One row of the box at a time and by value: a box passed by pointer would
+// live in local memory for the leaves that never come here, too.)
+__device__ __noinline__ float2 leaf_aabb_corners(float4 r, bool quad) {
+  float mn = FLT_MAX, mx = -FLT_MAX;
   for (int cz = 0; cz < (quad ? 1 : 2); cz++)
-#pragma unroll
     for (int cy = 0; cy < 2; cy++)
-#pragma unroll
       for (int cx = 0; cx < 2; cx++) {
-        float x = cx ? 0.5f : -0.5f, y = cy ? 0.5f : -0.5f, z = quad ? 0.0f : (cz ? 0.5f : -0.5f);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          float v = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(r[k].x, x), __fmul_rn(r[k].y, y)), __fmul_rn(r[k].z, z)), r[k].w);
-          mn[k] = fminf(mn[k], v);
-          mx[k] = fmaxf(mx[k], v);
-        }
+        const float x = cx ? 0.5f : -0.5f, y = cy ? 0.5f : -0.5f, z = quad ? 0.0f : (cz ? 0.5f : -0.5f);
+        const float v = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(r.x, x), __fmul_rn(r.y, y)), __fmul_rn(r.z, z)), r.w);
+        mn = fminf(mn, v);
+        mx = fmaxf(mx, v);
       }
+  return make_float2(mn, mx);
 }
 __device__ __forceinline__ void leaf_aabb(const float4 r[3], bool quad, float mn[3], float mx[3]) {
-  bool finite = true;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     const float hx = fabsf(__fmul_rn(r[k].x, 0.5f)), hy = fabsf(__fmul_rn(r[k].y, 0.5f));
@@ -93,9 +88,12 @@ __device__ __forceinline__ void leaf_aabb(const float4 r[3], bool quad, float mn
     const float h = __fadd_rn(__fadd_rn(hx, hy), hz);
     mn[k] = __fsub_rn(r[k].w, h);
     mx[k] = __fadd_rn(r[k].w, h);
-    finite = finite && fabsf(mn[k]) < FLT_MAX && fabsf(mx[k]) < FLT_MAX;
+    if (!(fabsf(mn[k]) < FLT_MAX && fabsf(mx[k]) < FLT_MAX)) {
+      const float2 c = leaf_aabb_corners(r[k], quad);
+      mn[k] = c.x;
+      mx[k] = c.y;
+    }
   }
-  if (!finite) leaf_aabb_corners(r[0], r[1], r[2], quad, mn, mx);
 }
 
 // Leaf count of a build: the host value `n`, or, when the count lives on the
@@ -583,7 +581,7 @@ __device__ __forceinline__ uint64_t term_path(const PgaTerminal* t, uint32_t i) 
 // through memory three times and each node's links twice.  Here a leaf costs
 // its key, value and record read once (76 bytes) and the results written once
 // (52 bytes).  Measured with k_join: 51 -> 21 us at 20,011 leaves, 251 -> 166
-// us at 3.0M, 421 -> 311 us for the city's 5.9M, of which 135 us are the bytes
+// us at 3.0M, 421 -> 309 us for the city's 5.9M, of which 135 us are the bytes
 // at the copy rate and the rest the climb (93 us) and its barriers.  Tile of
 // 256: a climb in it is eight to fifteen steps, and six blocks of it fit on an
 // SM (five 276 us, eight, with spills, 321 us on the city; six 264), so that
