@@ -120,6 +120,7 @@ using namespace pga;
 namespace pga {
 FrameKernels general_frame_kernels();  // derive_gen.cu
 FrameKernels block_frame_kernels();    // derive_blk.cu
+FrameKernels simple_frame_kernels();   // derive_simple.cu
 inline namespace PGA_FRAMES_NS {
 inline const void* adjoint_kernel();       // this build's k_adjoint (adjoint.cuh, included below)
 inline const void* adjoint_kernel_wide();  // and k_adjoint_wide
@@ -480,6 +481,18 @@ PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* co
     e->kernels = frame_kernels();
     e->kernels.adjoint = adjoint_kernel();
     e->kernels.adjointWide = adjoint_kernel_wide();
+  }
+  // Tables whose parameters need nothing of a shape but its axiom derive with
+  // the kernels that can evaluate no others.
+  bool simple = !e->generalFrames && !e->phased && !e->useSeeds;
+  for (const DevParam& p : e->hParams)
+    simple = simple && (p.type == PGA_PT_SCALAR || p.type == PGA_PT_BLOCK ||
+                        (p.type == PGA_PT_SHAPE_ATTR && p.v0 >= 16.0f && p.v0 < 17.0f));
+  if (simple) {
+    const FrameKernels tape = e->kernels;
+    e->kernels = simple_frame_kernels();
+    e->kernels.adjoint = tape.adjoint;
+    e->kernels.adjointWide = tape.adjointWide;
   }
   // Large tapes take the 3-blocks-per-SM adjoint (see k_adjoint_wide).
   if (c.maxTerminals >= kWideAdjointTerminals && e->kernels.adjointWide) e->kernels.adjoint = e->kernels.adjointWide;

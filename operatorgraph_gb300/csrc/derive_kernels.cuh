@@ -1,9 +1,10 @@
 // Derivation kernels (device code of derive.cu), compiled once per frame
 // representation: derive.cu includes it with signed-permutation frame codes,
-// derive_gen.cu with PGA_GENERAL_FRAMES (general rotations, for Rotate) and
+// derive_gen.cu with PGA_GENERAL_FRAMES (general rotations, for Rotate),
 // derive_blk.cu with PGA_INLINE_BLOCKS (frame codes, block parameters read
-// inline).  Everything here is in the build's inline namespace
-// (pga::perm / pga::gen / pga::permb).
+// inline) and derive_simple.cu with PGA_SIMPLE_PARAMS as well (no other
+// parameters than those and the custom attribute).  Everything here is in the
+// build's inline namespace (pga::perm / pga::gen / pga::permb / pga::simple).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -114,6 +115,7 @@ __device__ __forceinline__ float block_param(const DeriveArgs& a, const DevParam
 // Non-scalar parameters (random ranges, shape attributes, expressions, and
 // block values outside the block build) take this out-of-line path so the
 // common scalar case stays small.
+#if !PGA_SIMPLE_PARAMS
 __device__ __noinline__ float eval_param_slow(const DeriveArgs& a, DevParam p, Shape x) {
   switch (p.type) {
     case PGA_PT_SCALAR:
@@ -135,13 +137,20 @@ __device__ __noinline__ float eval_param_slow(const DeriveArgs& a, DevParam p, S
   }
 }
 
+#endif
+
 __device__ __forceinline__ float param(const DeriveArgs& a, const DevRule& r, uint32_t k, const Shape& x) {
   const DevParam p = param_at(a, r.paramBase + k);
   if (p.type == PGA_PT_SCALAR) return p.v0;
 #if PGA_INLINE_BLOCKS
   if (p.type == PGA_PT_BLOCK) return block_param(a, p, x);
 #endif
+#if PGA_SIMPLE_PARAMS
+  PGA_GUARD(x.axiom < a.numAxioms, 7, return 0.0f);
+  return __ldg(&a.axioms[x.axiom].custom);  // the only other kind in a simple table
+#else
   return eval_param_slow(a, p, x);
+#endif
 }
 
 __device__ __forceinline__ bool axis_param(const DeriveArgs& a, const DevRule& r, const Shape& x, uint32_t& axis) {
@@ -154,7 +163,7 @@ __device__ __forceinline__ bool axis_param(const DeriveArgs& a, const DevRule& r
 }
 
 __device__ __forceinline__ float seed_of(const DeriveArgs& a, float base, uint32_t modifier) {
-  return a.useSeeds ? next_seed(base, modifier) : 0.0f;
+  return !PGA_SIMPLE_PARAMS && a.useSeeds ? next_seed(base, modifier) : 0.0f;
 }
 
 // ------------------------------------------------- 1 -> 1 chain resolution
@@ -596,26 +605,13 @@ struct RepeatSetup {
   uint32_t flags;  // bit 0: arguments valid, bit 1: anchored to start
 };
 
-__device__ __noinline__ RepeatSetup repeat_setup(const DeriveArgs& a, DevRule r, Shape x, bool raise) {
-  RepeatSetup R{0u, 0u, 0.0f, 0.0f, 0.0f, 0u};
-  if (r.nParams < 3 || r.nSucc < 1) {
-    if (raise) raise_error(a.st, PGA_ERR_BAD_PARAM, x.entry);
-    return R;
-  }
-  R.axis = f2u(param(a, r, 0, x));
-  if (R.axis > 2) {
-    if (raise) raise_error(a.st, PGA_ERR_BAD_PARAM, x.entry);
-    return R;
-  }
-  const uint32_t mode = f2u(param(a, r, 2, x));
-  const float ext = param(a, r, 1, x);
-  const float total = pick3(x.s, R.axis);
+// Pieces of `total` by the extent parameter ext in a mode; flags 0 when the
+// reference rejects them.
+__device__ __forceinline__ RepeatSetup repeat_pieces(uint32_t axis, float ext, float total, uint32_t mode) {
+  RepeatSetup R{axis, 0u, 0.0f, 0.0f, 0.0f, 0u};
   const float extent = __fadd_rn(__fmul_rn(__fmul_rn((float)(ext < 0.0f), total), fabsf(ext)),
                                  __fmul_rn((float)(ext > 0.0f), ext));
-  if (extent <= 0.0f || total < 0.0f) {
-    if (raise) raise_error(a.st, PGA_ERR_BAD_PARAM, x.entry);
-    return R;
-  }
+  if (extent <= 0.0f || total < 0.0f) return R;
   const float division = __fdiv_rn(total, extent);
   if (mode == 0u || mode == 1u) {
     const float rest = fmodf(total, extent);
@@ -627,12 +623,42 @@ __device__ __noinline__ RepeatSetup repeat_setup(const DeriveArgs& a, DevRule r,
     R.reps = f2u(floorf(division));
     R.e1 = R.e2 = R.e3 = (R.reps > 0) ? __fdiv_rn(total, __uint2float_rn(R.reps)) : 0.0f;
   } else {
-    if (raise) raise_error(a.st, PGA_ERR_BAD_PARAM, x.entry);
     return R;
   }
   R.flags = 1u | (mode == 0u ? 2u : 0u);
   return R;
 }
+
+#if PGA_SIMPLE_PARAMS
+// Parameters are cheap to read where the call is: only numbers go out of line.
+__device__ __noinline__ RepeatSetup repeat_numbers(uint32_t axis, float ext, float total, uint32_t mode) {
+  return repeat_pieces(axis, ext, total, mode);
+}
+__device__ __forceinline__ RepeatSetup repeat_setup(const DeriveArgs& a, const DevRule& r, const Shape& x, bool raise) {
+  RepeatSetup R{0u, 0u, 0.0f, 0.0f, 0.0f, 0u};
+  if (r.nParams >= 3 && r.nSucc >= 1) {
+    R.axis = f2u(param(a, r, 0, x));
+    if (R.axis <= 2)
+      R = repeat_numbers(R.axis, param(a, r, 1, x), pick3(x.s, R.axis), f2u(param(a, r, 2, x)));
+  }
+  if (!(R.flags & 1u) && raise) raise_error(a.st, PGA_ERR_BAD_PARAM, x.entry);
+  return R;
+}
+#else
+__device__ __noinline__ RepeatSetup repeat_setup(const DeriveArgs& a, DevRule r, Shape x, bool raise) {
+  RepeatSetup R{0u, 0u, 0.0f, 0.0f, 0.0f, 0u};
+  if (r.nParams >= 3 && r.nSucc >= 1) {
+    R.axis = f2u(param(a, r, 0, x));
+    if (R.axis <= 2) {
+      const uint32_t mode = f2u(param(a, r, 2, x));
+      const float ext = param(a, r, 1, x);
+      R = repeat_pieces(R.axis, ext, pick3(x.s, R.axis), mode);
+    }
+  }
+  if (!(R.flags & 1u) && raise) raise_error(a.st, PGA_ERR_BAD_PARAM, x.entry);
+  return R;
+}
+#endif
 
 // Number of children a branching shape produces (decides how many work items
 // it is queued as).  Errors are raised when the item is executed.
@@ -1753,7 +1779,11 @@ inline FrameKernels frame_kernels() {
   k.persistentDyn[0] = (const void*)k_derive_persistent<false, 0, true>;
   k.persistentDyn[1] = (const void*)k_derive_persistent<false, 1, true>;
 #endif
+#if PGA_SIMPLE_PARAMS
+  k.phased = k.persistent[0];  // multi-phase tables run the other builds
+#else
   k.phased = (const void*)k_derive_persistent<false, 2>;
+#endif
   k.seed = (const void*)k_seed;
   k.expand = (const void*)k_expand_level;
   k.adjoint = nullptr;  // set by the builds that include adjoint.cuh
