@@ -245,11 +245,22 @@ __device__ __forceinline__ bool swap_size(const DeriveArgs& a, const DevRule& r,
 
 // ------------------------------------------------------ phases and colliders
 
+// The next slot of a counter: one addition for the lanes that are here together
+// (phase 0 of 18,432 axioms, most of them deferred: 41 us with one each, 29).
+__device__ __forceinline__ unsigned long long next_slot(unsigned long long* counter) {
+  const unsigned m = __activemask();
+  const unsigned lane = threadIdx.x & 31u;
+  const int leader = __ffs((int)m) - 1;
+  unsigned long long first = 0;
+  if ((int)lane == leader) first = atomicAdd(counter, (unsigned long long)__popc(m));
+  return __shfl_sync(m, first, leader) + (unsigned long long)__popc(m & ((1u << lane) - 1u));
+}
+
 // A shape reaching a rule of a later phase waits there: it is written to the
 // deferred buffer, which seeds the next phase's launch (the reference puts it
 // in that phase's queue, CPUEvaluator.h:155-190).
 __device__ __noinline__ void defer_shape(const DeriveArgs& a, const Shape& x) {
-  const unsigned long long i = atomicAdd(a.phaseCounters + 1, 1ull);
+  const unsigned long long i = next_slot(a.phaseCounters + 1);
   if (i >= a.deferCap) {
     raise_error(a.st, PGA_ERR_QUEUE_OVERFLOW, x.entry);
     return;
@@ -273,7 +284,7 @@ __device__ __noinline__ void defer_shape(const DeriveArgs& a, const Shape& x) {
 // LBVH (model * scale, tag, shape bit, path) and as an oriented box of 5
 // float4: rotation columns u0 u1 u2 (9) and centre (3), half extents (3), tag.
 __device__ __noinline__ void store_collider(const DeriveArgs& a, const Shape& x, uint32_t tag) {
-  const unsigned long long i = atomicAdd(a.phaseCounters, 1ull);
+  const unsigned long long i = next_slot(a.phaseCounters);
   if (i >= a.colCap) {
     raise_error(a.st, PGA_ERR_QUEUE_OVERFLOW, x.entry);
     return;
@@ -402,40 +413,78 @@ __device__ __noinline__ bool collides(const DeriveArgs& a, const Shape& x, uint3
     lo[r] = me.c[r] - h;
     hi[r] = me.c[r] + h;
   }
-  auto leaf_hits = [&](uint32_t leaf) -> bool {
-    const uint32_t rec = __ldg(a.colLeaf + leaf);
+  // Does the collider at this record overlap x?  One whose world box misses x's
+  // (both widened as above, and with the extents' absolute values, a quad's z
+  // among them: no smaller than what the axis tests see) needs no axis tests.
+  auto hits = [&](uint32_t rec) -> bool {
     bool cq;
     int ctag;
     const Obb other = collider_obb(a.colShape + 5ull * rec, cq, ctag);
     if (ctag != (int)tag) return false;
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      float h = 0.0f;
+#pragma unroll
+      for (int j = 0; j < 3; j++) h += fabsf(me.u[j][r] * me.e[j]) + fabsf(other.u[j][r] * other.e[j]);
+      h = h * 1.00001f + 1e-5f * (fabsf(me.c[r]) + fabsf(other.c[r]) + 2.0f);
+      if (fabsf(other.c[r] - me.c[r]) > h) return false;
+    }
     // Collision::check(Quad, Box) is check(Box, Quad) (Collision.cuh:734-737)
     return (cq && !quad) ? obb_overlap(me, other) : obb_overlap(other, me);
   };
-  if (n == 1) return leaf_hits(0);
+  if (n == 1) return hits(__ldg(a.colLeaf));
+  auto node_hit = [&](const float2& p, const float2& q, const float2& r) -> bool {
+    return p.x <= hi[0] && q.y >= lo[0] && p.y <= hi[1] && r.x >= lo[1] && q.x <= hi[2] && r.y >= lo[2];
+  };
+  // Bound by the latency of its loads: a tree among 2,048 colliders looks at 29
+  // nodes and 5 leaves, one after another.  Each step fetches the boxes, the
+  // links and the leaf values of a node's children together, so that it waits
+  // for memory once, and a warp's lanes come out of the inner loop to test
+  // leaves together.  16,384 trees against two tags: 156 us with a wait per box
+  // and per link, 86 with the boxes together (and 8 shapes a warp), 70 now.
+  // (Two nodes a step: 66, for twice the stack.)
   int stack[64];
   int top = 0;
-  stack[top++] = 0;
-  while (top > 0) {
-    const int node = stack[--top];
-#pragma unroll
-    for (int side = 1; side <= 2; side++) {
-      const int child = __ldg(a.colNodes + 3 * node + side);
-      if (child >= 0) {
-        if (leaf_hits((uint32_t)child)) return true;
-      } else {
-        const float* bx = a.colAabbs + 6ll * (-child);
-        const bool overlap = __ldg(bx) <= hi[0] && __ldg(bx + 3) >= lo[0] && __ldg(bx + 1) <= hi[1] &&
-                             __ldg(bx + 4) >= lo[1] && __ldg(bx + 2) <= hi[2] && __ldg(bx + 5) >= lo[2];
-        if (overlap) {
-          if (top >= 64) {
-            raise_error(a.st, PGA_ERR_DEPTH, x.entry);
-            return false;
-          }
-          stack[top++] = -child;
+  int c0 = __ldg(a.colNodes + 1), c1 = __ldg(a.colNodes + 2);  // the children to look at
+  bool more = true;
+  do {
+    uint32_t rec[2];
+    int found = 0;
+    while (more && found == 0) {
+      const int n0 = max(-c0, 0), n1 = max(-c1, 0);  // a leaf child: the root's, unused
+      const float2* b0 = reinterpret_cast<const float2*>(a.colAabbs + 6ll * n0);
+      const float2* b1 = reinterpret_cast<const float2*>(a.colAabbs + 6ll * n1);
+      const float2 p0 = __ldg(b0), q0 = __ldg(b0 + 1), r0 = __ldg(b0 + 2);
+      const float2 p1 = __ldg(b1), q1 = __ldg(b1 + 1), r1 = __ldg(b1 + 2);
+      const int c00 = __ldg(a.colNodes + 3 * n0 + 1), c01 = __ldg(a.colNodes + 3 * n0 + 2);
+      const int c10 = __ldg(a.colNodes + 3 * n1 + 1), c11 = __ldg(a.colNodes + 3 * n1 + 2);
+      const uint32_t v0 = __ldg(a.colLeaf + max(c0, 0)), v1 = __ldg(a.colLeaf + max(c1, 0));
+      const bool in0 = c0 < 0 && node_hit(p0, q0, r0), in1 = c1 < 0 && node_hit(p1, q1, r1);
+      rec[0] = c0 >= 0 ? v0 : v1;
+      rec[1] = v1;
+      found = (c0 >= 0 ? 1 : 0) + (c1 >= 0 ? 1 : 0);
+      if (in0 && in1) {
+        if (top >= 64) {
+          raise_error(a.st, PGA_ERR_DEPTH, x.entry);
+          return false;
         }
+        stack[top++] = n1;
+      }
+      if (in0 || in1) {
+        c0 = in0 ? c00 : c10;
+        c1 = in0 ? c01 : c11;
+      } else if (top > 0) {
+        const int node = stack[--top];
+        c0 = __ldg(a.colNodes + 3 * node + 1);
+        c1 = __ldg(a.colNodes + 3 * node + 2);
+      } else {
+        more = false;
       }
     }
-  }
+#pragma unroll 1
+    for (int i = 0; i < found; i++)
+      if (hits(rec[i])) return true;
+  } while (more);
   return false;
 }
 
@@ -1316,20 +1365,32 @@ __device__ void seed_axioms(const DeriveArgs& a, WarpOut& w, uint32_t first, uin
   }
 }
 
+// How many warps (2^shift: 1, 2, 4 or 8) a narrow level's chunks of 32 items
+// are shared by (see expand_level).
+__device__ __forceinline__ uint32_t share_shift(unsigned long long items) {
+  const unsigned long long threads = (unsigned long long)gridDim.x * kThreads;
+  uint32_t shift = 0;
+  while (shift < 3 && (items << (shift + 1)) <= threads) shift++;
+  return shift;
+}
+
 // Seeds the shapes deferred to this phase (multi-phase derivation): each is
-// loaded as it was stored and resolved from the rule it was waiting at.
+// loaded as it was stored and resolved from the rule it was waiting at.  What
+// waits is mostly an IfCollides, whose traversals differ from lane to lane: a
+// warp takes as few shapes as the grid has warps for, down to 4.
 template <bool PAGED, bool LEAF, int AFF>
 __device__ void seed_deferred(const DeriveArgs& a, WarpOut& w) {
   const unsigned lane = threadIdx.x & 31u;
   const unsigned long long warpId = ((unsigned long long)blockIdx.x * kThreads + threadIdx.x) >> 5;
   const unsigned long long numWarps = ((unsigned long long)gridDim.x * kThreads) >> 5;
   const unsigned long long end = a.numDeferIn;
-  for (unsigned long long b = warpId * 32ull; b < end; b += numWarps * 32ull) {
+  const unsigned take = 32u >> share_shift(end);
+  for (unsigned long long b = warpId * take; b < end; b += numWarps * take) {
     const unsigned long long i = b + lane;
     int kind = kNone;
     Shape y;
     uint32_t tidx = 0;
-    if (i < end) {
+    if (lane < take && i < end) {
       const float4* p = reinterpret_cast<const float4*>(a.deferIn + i);
       const float4 p0 = __ldcg(p), p1 = __ldcg(p + 1);
       const uint4 m = __ldcg(reinterpret_cast<const uint4*>(p + 2));
@@ -1379,13 +1440,6 @@ __device__ void seed_deferred(const DeriveArgs& a, WarpOut& w) {
 // facades 98 -> 65, 4,096 buildings 264 -> 237).  The warps take item pages of
 // kNodePage >> shift slots, so that the slots left empty at the level's end are
 // as few as with one warp a chunk.
-__device__ __forceinline__ uint32_t share_shift(unsigned long long items) {
-  const unsigned long long threads = (unsigned long long)gridDim.x * kThreads;
-  uint32_t shift = 0;
-  while (shift < 3 && (items << (shift + 1)) <= threads) shift++;
-  return shift;
-}
-
 template <bool PAGED, bool LEAF, int AFF, bool DYN = false>
 __device__ __forceinline__ void expand_level(const DeriveArgs& a, WarpOut& w, unsigned long long lo,
                                              unsigned long long hi, uint32_t K, uint32_t shift) {
