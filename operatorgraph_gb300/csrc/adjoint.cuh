@@ -8,13 +8,13 @@
 // of Rotate's scalar angles -- are changed by no continuous input, so the
 // state that carries gradient is a shape's translation t and size s.
 //
-// Tape: every queued work item stores (parent item or kAxiomLink | axiom,
-// child ordinal) in its ext field, every terminal the same pair in termLinks.
-// The reverse sweep first visits every terminal, then the levels from the
-// deepest up: a record recomputes its creating child from the parent item (or
-// the axiom), replays the 1 -> 1 chain to itself, and pushes its gradient
-// through the chain and the operator that created it into the parent item's
-// accumulator (atomicAdd) and the parameter / axiom-size gradients.
+// Tape: every queued work item has (parent item or kAxiomLink | axiom, child
+// ordinal, entry, child range) in itemTape, every terminal the first two in
+// termLinks.  The reverse sweep maps terminals and items to their parents' child
+// slots, then takes the levels from the deepest up: an item sums its children's
+// gradients -- in closed form where its rule's children pass them on unchanged
+// (adj_sums), else replaying its expansion and each child's 1 -> 1 chain
+// (adj_page) -- into its own and into the parameter and axiom-size gradients.
 //
 // Operator VJPs (o = offset along the split axis a, S = size[a]):
 //  Subdivide  size_c = N_c, o_c = -S/2 + sum_{i<c} N_i + N_c/2, N_i = f_i (f > 0)
