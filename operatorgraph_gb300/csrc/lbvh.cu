@@ -80,20 +80,22 @@ __device__ __noinline__ float2 leaf_aabb_corners(float4 r, bool quad) {
       }
   return make_float2(mn, mx);
 }
+// One axis of the box, from the matrix's row.
+__device__ __forceinline__ void leaf_extent(const float4& r, bool quad, float& mn, float& mx) {
+  const float hx = fabsf(__fmul_rn(r.x, 0.5f)), hy = fabsf(__fmul_rn(r.y, 0.5f));
+  const float hz = fabsf(__fmul_rn(r.z, quad ? 0.0f : 0.5f));
+  const float h = __fadd_rn(__fadd_rn(hx, hy), hz);
+  mn = __fsub_rn(r.w, h);
+  mx = __fadd_rn(r.w, h);
+  if (!(fabsf(mn) < FLT_MAX && fabsf(mx) < FLT_MAX)) {
+    const float2 c = leaf_aabb_corners(r, quad);
+    mn = c.x;
+    mx = c.y;
+  }
+}
 __device__ __forceinline__ void leaf_aabb(const float4 r[3], bool quad, float mn[3], float mx[3]) {
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const float hx = fabsf(__fmul_rn(r[k].x, 0.5f)), hy = fabsf(__fmul_rn(r[k].y, 0.5f));
-    const float hz = fabsf(__fmul_rn(r[k].z, quad ? 0.0f : 0.5f));
-    const float h = __fadd_rn(__fadd_rn(hx, hy), hz);
-    mn[k] = __fsub_rn(r[k].w, h);
-    mx[k] = __fadd_rn(r[k].w, h);
-    if (!(fabsf(mn[k]) < FLT_MAX && fabsf(mx[k]) < FLT_MAX)) {
-      const float2 c = leaf_aabb_corners(r[k], quad);
-      mn[k] = c.x;
-      mx[k] = c.y;
-    }
-  }
+  for (int k = 0; k < 3; k++) leaf_extent(r[k], quad, mn[k], mx[k]);
 }
 
 // Leaf count of a build: the host value `n`, or, when the count lives on the
@@ -580,8 +582,8 @@ __device__ __forceinline__ uint64_t term_path(const PgaTerminal* t, uint32_t i) 
 // the root through counters at GPU scope; and they moved each leaf's box
 // through memory three times and each node's links twice.  Here a leaf costs
 // its key, value and record read once (76 bytes) and the results written once
-// (52 bytes).  Measured with k_join: 51 -> 21 us at 20,011 leaves, 251 -> 166
-// us at 3.0M, 421 -> 309 us for the city's 5.9M, of which 135 us are the bytes
+// (52 bytes).  Measured with k_join: 51 -> 21 us at 20,011 leaves, 251 -> 148
+// us at 3.0M, 421 -> 287 us for the city's 5.9M, of which 110 us are the bytes
 // at the copy rate and the rest the climb (93 us) and its barriers.  Tile of
 // 256: a climb in it is eight to fifteen steps, and six blocks of it fit on an
 // SM (five 276 us, eight, with spills, 321 us on the city; six 264), so that
@@ -873,12 +875,39 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
       d = boundary_delta(before, code, (uint32_t)k);
     }
     sDelta[tid] = (signed char)d;
-    gather_leaf(a.t, val, mn, mx, path);
-    win.path[kHalo + tid] = path;
     win.val[kHalo + tid] = val;
-    store_box(sBox + tid * 6, mn, mx);
-    fPath[tid] = path;
     fVal[tid] = val;
+  }
+  // The warp's 32 records, eight at a time: four lanes fetch a record's four 16
+  // bytes, so that a load touches 8 lines and not 32; three of them make an
+  // axis of the box each, the fourth has the path.  (A lane per record kept the
+  // L1 at 70% of its throughput with line look-ups: 5.9M leaves of the city 263
+  // us, 240 this way; 19M of the mixed batch 932 and 850; 3.0M records 130 and
+  // 117.)
+  {
+    const uint32_t part = lane & 3u;
+    float4 row[4];
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      const uint32_t v = __shfl_sync(kAll, val, (int)(q * 8 + (lane >> 2)));
+      row[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (warp * 32 + q * 8 + (lane >> 2) < cnt) row[q] = __ldg(reinterpret_cast<const float4*>(a.t + v) + part);
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < 4; q++) {
+      const uint32_t e = warp * 32 + q * 8 + (lane >> 2);
+      const bool quad = (__shfl_sync(kAll, __float_as_uint(row[q].x), (int)(lane | 3u)) >> 31) != 0;
+      if (e >= cnt) continue;
+      if (part < 3) {
+        leaf_extent(row[q], quad, sBox[e * 6 + part], sBox[e * 6 + 3 + part]);
+      } else {
+        const uint64_t p = ((uint64_t)__float_as_uint(row[q].w) << 32) | __float_as_uint(row[q].z);
+        win.path[kHalo + e] = p;
+        fPath[e] = p;
+      }
+    }
+    __syncwarp();
+    if (valid) path = fPath[tid];
   }
   bool sameEnd = false;
   if (tid == cnt - 1) {  // the tile's right end
@@ -899,6 +928,7 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
   if (tid == cnt - 1) sEq[kWindowWords - 1] = 0u;
   const bool same = valid && k > 0 && before == code;
   if (__syncthreads_or(same || sameEnd)) {
+    if (valid) load_box(sBox + tid * 6, mn, mx);
     // Equal to the left neighbour?  (The first leaf's and the right end's
     // neighbours are in other tiles.)
     bool eq = same;
