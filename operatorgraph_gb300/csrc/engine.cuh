@@ -20,11 +20,11 @@
 // perm_a and a signed zero elsewhere, so a translation is one rounded add.
 //
 // Rotate (Rotate.cuh:24-41) leaves that set.  The device code is therefore
-// compiled twice: by default with frame codes, and with PGA_GENERAL_FRAMES
+// compiled with frame codes (three builds, below) and with PGA_GENERAL_FRAMES
 // (derive_gen.cu, for tables with Rotate rules) with the rotation as nine
 // floats and the reference's 4x4 products written out term by term.  The shape
 // state and the kernels of each build live in an inline namespace of their
-// own (pga::perm, pga::gen), so the two sets of kernels have distinct names.
+// own (pga::perm, pga::gen, ...), so the sets of kernels have distinct names.
 #pragma once
 
 #include <cstdint>
