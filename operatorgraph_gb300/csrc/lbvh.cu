@@ -856,11 +856,13 @@ __global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
   const unsigned long long n = leaf_count(a.dN, a.cap);
   const unsigned long long base = (unsigned long long)blockIdx.x * kTile;
   const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-  if (base + tid >= n && base + tid < a.cap) a.outKeys[base + tid] = ~0ull;  // padding past a device count
+  const unsigned long long k = base + tid;
+  if (k >= n && k < a.cap) a.outKeys[k] = ~0ull;  // padding past a device count
+  // a single leaf has a key and no tree (out->keys held the sort's hash digits until here)
+  if (n == 1 && k == 0) a.outKeys[0] = ((unsigned long long)*a.codes << 34) | (term_path(a.t, 0) >> 30);
   if (n < 2 || base >= n) return;
   const uint32_t cnt = (uint32_t)min((unsigned long long)kTile, n - base);
   const bool valid = tid < cnt;
-  const unsigned long long k = base + tid;
 
   uint32_t code = 0, before = ~0u;  // this leaf's and its left neighbour's
   uint32_t val = 0;
