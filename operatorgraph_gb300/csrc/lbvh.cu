@@ -405,7 +405,7 @@ __device__ __forceinline__ void sort_tile(const SortPass& a, uint32_t tile, uint
     }
     old = __shfl_sync(0xFFFFFFFFu, old, leader);
     digit[k] = (d << 16) | (old + __popc(peers & lt));
-    if (!kMasks) __syncwarp();
+    __syncwarp();  // the leader's stores, before the next turn's accesses to the same words by other lanes
   }
   __syncthreads();
   // Thread t owns bins 2t and 2t + 1: the warps' exclusive prefixes in place,
