@@ -129,6 +129,11 @@ def _stream_handle(stream):
     return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
+def _bounds(bounds):
+    """PgaBounds of six numbers in any layout (min xyz, max xyz)."""
+    return PgaBounds.from_buffer_copy(np.ascontiguousarray(bounds, np.float32).reshape(6))
+
+
 def _dev(arr_or_tensor):
     """Device copy (torch uint8) of a numpy record array, or the tensor itself."""
     import torch
@@ -243,7 +248,7 @@ class Engine:
             "leafTerminal": torch.empty(n, dtype=torch.int32, device=dev),
             "keys": torch.empty(n, dtype=torch.int64, device=dev),
         }
-        pb = PgaBounds.from_buffer_copy(np.asarray(bounds, np.float32).reshape(6))
+        pb = _bounds(bounds)
         out = PgaLbvh(res["nodes"].data_ptr(), res["leafParents"].data_ptr(), res["aabbs"].data_ptr(),
                       res["leafTerminal"].data_ptr(), res["keys"].data_ptr())
         if count is None:
