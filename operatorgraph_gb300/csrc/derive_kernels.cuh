@@ -34,8 +34,7 @@ struct __align__(16) Smem {
   uint32_t turn;                 // which of DevState's per-level sets this level uses
   uint32_t taken;                // item slots this block has taken for the next level
   uint32_t shareShift;            // 2^shareShift warps share a chunk of items
-  int32_t seen;                  // DevState::status, read while the level was expanded
-  int32_t stop;                  // some block had seen a status by the end of the level before
+  int32_t stop;                  // a status had been raised by the end of the level before
   unsigned long long maxItems;   // of a level (block 0)
 };
 
@@ -1479,7 +1478,7 @@ __device__ __forceinline__ void setup_block(const DeriveArgs& a, Smem& sm) {
   if (threadIdx.x == 0) {
     sm.levelBase = 0;
     sm.turn = sm.taken = sm.shareShift = 0;
-    sm.seen = sm.stop = 0;
+    sm.stop = 0;
     sm.maxItems = 0;
   }
   uint32_t dynBytes;
@@ -1528,9 +1527,9 @@ __device__ __forceinline__ bool await_word(const DeriveArgs& a, const Word* word
   }
 }
 
-// The end of a level: every block adds its arrival, whether it had seen a
-// raised status, and the item slots it took to one word, and goes on when all
-// blocks' arrivals are in it.  The word then holds what each block needs to
+// The end of a level: every block adds its arrival, whether it saw a raised
+// status (those of its own threads at least), and the item slots it took to one
+// word, and goes on when all blocks' arrivals are in it.  The word then holds what each block needs to
 // know of the next level (its size, whether to stop), the same for all, so no
 // block has to set the level up for the others: with a leader that did, a
 // level of the Menger sponge (24 items) took 7-8 us, now 5.  The words, like the slot counters and cursors, are three in turn:
@@ -1545,9 +1544,12 @@ __device__ bool level_barrier(const DeriveArgs& a, Smem& sm) {
   if (threadIdx.x == 0) {
     DevState* st = a.st;
     unsigned long long* word = &st->levelWord[sm.turn];
-    const unsigned long long mine =
-        1ull | (sm.seen != 0 ? 1ull << kArriveBits : 0ull) | ((unsigned long long)sm.taken << 32);
+    // Not earlier: a status raised in this level ends the derivation with it.
+    // (The load waits beside the fence: no level got slower by it.)
+    const int32_t status = ((volatile DevState*)st)->status;
     __threadfence();
+    const unsigned long long mine =
+        1ull | (status != 0 ? 1ull << kArriveBits : 0ull) | ((unsigned long long)sm.taken << 32);
     atomicAdd(word, mine);
     unsigned long long seen;
     const bool good = await_word<unsigned long long>(a, word, (1u << kArriveBits) - 1u, gridDim.x, seen);
@@ -1786,7 +1788,6 @@ __global__ void __launch_bounds__(kThreads, PGA_PERSISTENT_MIN_BLOCKS) k_derive_
       if (deep) raise_error(a.st, PGA_ERR_DEPTH, (int)level);
     }
     if (stop) break;
-    if (threadIdx.x == 32) sm.seen = ((volatile DevState*)a.st)->status;  // counted at the level's end
     warpout_level(a, w, hi - lo);
     expand_level<true, LEAF, AFF, DYN>(a, w, lo, hi, a.itemsPerLane, sm.shareShift);
   }
