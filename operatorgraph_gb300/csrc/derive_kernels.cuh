@@ -280,8 +280,10 @@ __device__ __noinline__ void defer_shape(const DeriveArgs& a, const Shape& x) {
 
 // Collider<Tag, Next> (Collider.cuh:20-45) stores the shape with its tag
 // (IntermediateSymbolsBufferAdapter.cuh:200-215): here as a record for the
-// LBVH (model * scale, tag, shape bit, path) and as an oriented box of 5
-// float4: rotation columns u0 u1 u2 (9) and centre (3), half extents (3), tag.
+// LBVH (model * scale, tag, path) and as an oriented box of 5 float4: rotation
+// columns u0 u1 u2 (9) and centre (3), half extents (3) with a quad's mark, tag.
+// The record has no shape bit: the axis tests take a quad's z half extent along
+// its normal (obb_overlap), so its box in the LBVH has to hold it, as a Box's.
 __device__ __noinline__ void store_collider(const DeriveArgs& a, const Shape& x, uint32_t tag) {
   const unsigned long long i = next_slot(a.phaseCounters);
   if (i >= a.colCap) {
@@ -294,8 +296,7 @@ __device__ __noinline__ void store_collider(const DeriveArgs& a, const Shape& x,
   rec[0] = make_float4(m[0][0], m[0][1], m[0][2], x.t[0]);
   rec[1] = make_float4(m[1][0], m[1][1], m[1][2], x.t[1]);
   rec[2] = make_float4(m[2][0], m[2][1], m[2][2], x.t[2]);
-  const uint32_t quad = x.kind == PGA_SHAPE_QUAD ? 0x80000000u : 0u;
-  reinterpret_cast<uint4*>(rec)[3] = make_uint4((tag & 0xFFFFFFu) | quad, 0u, (uint32_t)x.path, (uint32_t)(x.path >> 32));
+  reinterpret_cast<uint4*>(rec)[3] = make_uint4(tag & 0xFFFFFFu, 0u, (uint32_t)x.path, (uint32_t)(x.path >> 32));
   float u[3][3];
 #pragma unroll
   for (uint32_t j = 0; j < 3; j++)
@@ -306,7 +307,7 @@ __device__ __noinline__ void store_collider(const DeriveArgs& a, const Shape& x,
   sh[1] = make_float4(u[1][1], u[1][2], u[2][0], u[2][1]);
   sh[2] = make_float4(u[2][2], x.t[0], x.t[1], x.t[2]);
   sh[3] = make_float4(__fmul_rn(x.s[0], 0.5f), __fmul_rn(x.s[1], 0.5f), __fmul_rn(x.s[2], 0.5f),
-                      __uint_as_float(quad ? 1u : 0u));
+                      __uint_as_float(x.kind == PGA_SHAPE_QUAD ? 1u : 0u));
   sh[4] = make_float4(__int_as_float((int)tag), 0.0f, 0.0f, 0.0f);
 }
 
