@@ -80,7 +80,6 @@ class PathTarget:
         order = torch.argsort(paths)
         self.paths = paths[order]
         self.c, self.e = centres_extents(M.detach()[order])
-        self.unique = bool((self.paths[1:] != self.paths[:-1]).all())
 
     def sse(self, M, paths, check=True):
         """Sum of squared errors of centres and extents against the target;
@@ -95,13 +94,14 @@ class PathTarget:
         # The target's terminals are put in the derivation's order and not the
         # other way round: they need no gradient, so no backward pass has to
         # undo the gather.
-        if check and self.unique and n > 0:
-            at = torch.searchsorted(self.paths, paths).clamp_(max=n - 1)
+        at = None
+        if check and n > 0:
+            at = torch.searchsorted(self.paths, paths.contiguous()).clamp_(max=n - 1)
             found = torch.zeros(n, dtype=torch.bool, device=paths.device)
             found[at] = self.paths[at] == paths  # a path of the target nobody has stays False
-            if not found.all():
-                raise ValueError("the derivation's paths differ from the target's")
-        else:
+            if not found.all():  # other paths, or one that occurs twice: sorting both sides decides
+                at = None
+        if at is None:
             order = torch.argsort(paths)
             if check and not torch.equal(paths[order], self.paths):
                 raise ValueError("the derivation's paths differ from the target's")
