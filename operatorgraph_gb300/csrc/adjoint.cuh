@@ -957,7 +957,8 @@ __device__ __forceinline__ void adj_sums(const DeriveArgs& a, const AdjArgs& j, 
         s.go += go;
         if (subdivide) {
           const float own = gN + 0.5f * go;
-          s.q += go * below + own * relF;
+          // (a term without a share is left out, not multiplied by zero: go may be infinite)
+          s.q += (below != 0.0f ? go * below : 0.0f) + (relF != 0.0f ? own * relF : 0.0f);
           if (kBlocks && !scalar)
 #pragma unroll
             for (uint32_t k = 0; k < kSumFactors; k++) W[k] += k == c ? own : (k < c ? go : 0.0f);
