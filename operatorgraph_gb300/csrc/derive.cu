@@ -711,11 +711,14 @@ static PgaStatus group_axioms(PgaEngine* e, const PgaAxiom* dAxioms, uint32_t n,
 
 // Copies a small device record to the host once `s` has reached it, through the
 // engine's pinned buffer (a copy to pageable memory is staged by the driver).
+// While another thread waits with that buffer, for a stream of its own, the
+// record goes straight to dst: neither waits for the other's stream.
 static PgaStatus read_back(PgaEngine* e, void* dst, const void* src, size_t bytes, cudaStream_t s) {
-  std::lock_guard<std::mutex> lock(e->hostMutex);
-  PGA_CUDA_TRY(cudaMemcpyAsync(e->hReadBack, src, bytes, cudaMemcpyDeviceToHost, s));
+  std::unique_lock<std::mutex> lock(e->hostMutex, std::try_to_lock);
+  void* landing = lock.owns_lock() ? e->hReadBack : dst;
+  PGA_CUDA_TRY(cudaMemcpyAsync(landing, src, bytes, cudaMemcpyDeviceToHost, s));
   PGA_CUDA_TRY(cudaStreamSynchronize(s));
-  memcpy(dst, e->hReadBack, bytes);
+  if (landing != dst) memcpy(dst, landing, bytes);
   return PGA_OK;
 }
 

@@ -110,7 +110,7 @@ struct PgaEngine {
   PgaTerminal* dStageOut = nullptr;
   uint64_t* dStageCount = nullptr;
   size_t stageAxiomBytes = 0, stageOutBytes = 0, stageCountBytes = 0;
-  // Pinned landing place of the small records the host waits for, one caller at a time.
+  // Pinned landing place of the small records the host waits for, one caller at a time (see read_back).
   void* hReadBack = nullptr;
   std::mutex hostMutex;
   cudaStream_t copyStream = nullptr;
