@@ -483,8 +483,18 @@ PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* co
     e->kernels.adjointWide = adjoint_kernel_wide();
   }
   // Tables whose parameters need nothing of a shape but its axiom derive with
-  // the kernels that can evaluate no others.
+  // the kernels that can evaluate no others.  Not so very large batches of
+  // several grammars without block parameters, grouped: the simple kernels run
+  // their wide levels slower once the items and terminals fill some 14 GB (mix
+  // of 65,536 axioms, 152M terminals, the two builds in turn: 9.65 ms against
+  // 9.30 with the general kernels, with a tape 9.18 and 8.84; 80,000 axioms
+  // 11.4 and 11.2, 11.0 and 10.4).  At 49,152 axioms (capacity 124M) they tie
+  // (6.96 and 7.00, 6.69 and 6.64), below they win (24,000: 3.44 and 3.53);
+  // with block parameters (65,536: 10.8 and 11.5) and in index order (13.0 and
+  // 13.2) they win at any size.
+  constexpr unsigned long long kSimpleGroupedTerminals = 1ull << 27;
   bool simple = !e->generalFrames && !e->phased && !e->useSeeds;
+  if ((c.flags & PGA_FLAG_GROUP_AXIOMS) && !blockParams && c.maxTerminals >= kSimpleGroupedTerminals) simple = false;
   for (const DevParam& p : e->hParams)
     simple = simple && (p.type == PGA_PT_SCALAR || p.type == PGA_PT_BLOCK ||
                         (p.type == PGA_PT_SHAPE_ATTR && p.v0 >= 16.0f && p.v0 < 17.0f));
