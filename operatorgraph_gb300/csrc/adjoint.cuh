@@ -1117,10 +1117,7 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v) {
 // small ones the spills and the larger grid's barriers cost more (1,024
 // facades, 0.4M terminals: 66 / 74 / 83 us with 2 / 3 / 4).
 // Engines choose by terminal capacity (kWideAdjointTerminals, 2M).
-// PGA_ADJOINT_MIN_BLOCKS overrides k_adjoint's shape.
-#if defined(PGA_ADJOINT_MIN_BLOCKS)
-#define PGA_ADJOINT_BOUNDS __launch_bounds__(kThreads, PGA_ADJOINT_MIN_BLOCKS)
-#elif PGA_INLINE_BLOCKS
+#if PGA_INLINE_BLOCKS
 #define PGA_ADJOINT_BOUNDS __launch_bounds__(kThreads, 2)
 #else
 #define PGA_ADJOINT_BOUNDS __launch_bounds__(kThreads)
@@ -1309,10 +1306,7 @@ __global__ void PGA_ADJOINT_BOUNDS k_adjoint(DeriveArgs a, AdjArgs j, unsigned l
 }
 
 #if !PGA_GENERAL_FRAMES
-#ifndef PGA_ADJOINT_WIDE_BLOCKS
-#define PGA_ADJOINT_WIDE_BLOCKS 3
-#endif
-__global__ void __launch_bounds__(kThreads, PGA_ADJOINT_WIDE_BLOCKS) k_adjoint_wide(DeriveArgs a, AdjArgs j,
+__global__ void __launch_bounds__(kThreads, 3) k_adjoint_wide(DeriveArgs a, AdjArgs j,
                                                               unsigned long long numParamFloats, uint32_t numAxioms) {
   adjoint_pass(a, j, numParamFloats, numAxioms);
 }

@@ -411,7 +411,7 @@ PgaStatus pga_engine_create(const PgaRuleTable* table, const PgaEngineConfig* co
       bool sums = r.nSucc > 0;
       if (r.op == PGA_OP_SUBDIVIDE || r.op == PGA_OP_SUBDIVIDE_STATIC) {
         const uint32_t n = r.op == PGA_OP_SUBDIVIDE ? (r.nParams >= 1 ? r.nParams - 1u : 0u) : r.nChildren;
-        sums = sums && n > 0 && n < r.nParams + 0u && (r.flags & kRulePure) &&
+        sums = sums && n > 0 && n < r.nParams && (r.flags & kRulePure) &&
                ((r.flags & kRuleScalar) || n <= kSumFactors);
       } else if (r.op == PGA_OP_REPEAT) {
         sums = sums && (r.flags & kRulePure);

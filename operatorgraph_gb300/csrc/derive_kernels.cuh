@@ -33,7 +33,7 @@ struct __align__(16) Smem {
   unsigned long long levelBase;  // first item slot of the next level: where this level's children go
   uint32_t turn;                 // which of DevState's per-level sets this level uses
   uint32_t taken;                // item slots this block has taken for the next level
-  uint32_t shareShift;            // 2^shareShift warps share a chunk of items
+  uint32_t shareShift;           // 2^shareShift warps share a chunk of items
   int32_t stop;                  // a status had been raised by the end of the level before
   unsigned long long maxItems;   // of a level (block 0)
 };
@@ -1190,8 +1190,7 @@ __device__ __forceinline__ void close_node_page(const DeriveArgs& a, WarpOut& w)
   const unsigned lane = threadIdx.x & 31u;
   for (uint32_t k = lane; k < w.nLeft; k += 32) {
     const unsigned long long slot = w.nNext + k;
-    if (slot < a.nodeCap)
-    {
+    if (slot < a.nodeCap) {
       __stcg(reinterpret_cast<uint4*>(a.nodes + slot) + 3, make_uint4(kEmptyItem, 0u, 0u, 0u));
       if (a.itemTape != nullptr) __stcg(a.itemTape + slot, make_uint4(0u, 0u, kAxiomLink, 0u));
     }

@@ -253,11 +253,7 @@ __global__ void __launch_bounds__(kSortThreads) k_sort_count(const uint32_t* cod
   const uint32_t first = blockIdx.x * perGroup, last = min(tiles, first + perGroup);
   uint2* bins = reinterpret_cast<uint2*>(sh) + threadIdx.x;
   uint2 run = make_uint2(0u, 0u);
-  allow_next();
   *bins = run;
-  await_previous();
-  codes = written(codes);
-  hashes = written(hashes);
   __syncthreads();
   for (uint32_t tile = first; tile < last; tile++) {
     const unsigned long long base = (unsigned long long)tile * kTileItems;
@@ -304,8 +300,6 @@ __global__ void __launch_bounds__(1024) k_sort_scan(uint32_t* groups, uint32_t* 
   __shared__ uint32_t sSum[32][33];
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint32_t* col = groups + blockIdx.x * 32u + lane;
-  allow_next();
-  await_previous();
   uint32_t v[kPer], sum = 0;
 #pragma unroll
   for (uint32_t k = 0; k < kPer; k++) {
@@ -530,7 +524,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort_pass(SortPass a) {
   constexpr uint32_t kTileItems = kSortThreads * ITEMS;
   extern __shared__ __align__(16) unsigned char smem_sort[];
   __shared__ uint32_t sTile;
-  allow_next();
+  if (!COUNTED) allow_next();
   const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   uint16_t* mine = reinterpret_cast<uint16_t*>(smem_sort + sort_entry_bytes(ITEMS)) + warp * kHistStride;
   for (uint32_t k = lane; k < kBins / 8; k += 32) reinterpret_cast<uint4*>(mine)[k] = make_uint4(0u, 0u, 0u, 0u);
@@ -538,13 +532,14 @@ __global__ void __launch_bounds__(kSortThreads, 2) k_sort_pass(SortPass a) {
     uint32_t* match = reinterpret_cast<uint32_t*>(smem_sort) + warp * kBins;
     for (uint32_t k = lane; k < kBins / 4; k += 32) reinterpret_cast<uint4*>(match)[k] = make_uint4(0u, 0u, 0u, 0u);
   }
-  await_previous();
-  a.codesIn = written(a.codesIn);
-  a.hashes = written(a.hashes);
-  a.valsIn = written(a.valsIn);
-  a.rows = written(a.rows);
-  a.groups = written(a.groups);
-  const uint2 all = reinterpret_cast<const uint2*>(written(a.hist))[threadIdx.x];  // this thread's bins, whole input
+  if (!COUNTED) {
+    await_previous();
+    a.codesIn = written(a.codesIn);
+    a.hashes = written(a.hashes);
+    a.valsIn = written(a.valsIn);
+    a.hist = written(a.hist);
+  }
+  const uint2 all = reinterpret_cast<const uint2*>(a.hist)[threadIdx.x];  // this thread's bins, whole input
   if (!COUNTED) {
     if (threadIdx.x == 0) sTile = atomicAdd(a.tileCounter, 1u);
     __syncthreads();
@@ -828,10 +823,7 @@ __device__ __forceinline__ void gather_leaf(const PgaTerminal* t, uint32_t v, fl
   path = ((uint64_t)meta.w << 32) | meta.z;
 }
 
-#ifndef PGA_TREE_BLOCKS
-#define PGA_TREE_BLOCKS 6
-#endif
-__global__ void __launch_bounds__(kTile, PGA_TREE_BLOCKS) k_tree(TreeArgs a) {
+__global__ void __launch_bounds__(kTile, 6) k_tree(TreeArgs a) {
   constexpr unsigned kAll = 0xFFFFFFFFu;
   __shared__ __align__(16) float sBox[kTile * 6];
   // the joined nodes' boxes; before the climb, the window and the final paths
@@ -1509,9 +1501,10 @@ static PgaStatus launch_sort_pass(int q, unsigned long long n, const SortBuffers
   uint32_t* groups = rows + (size_t)tiles * kBins;
   const uint32_t perGroup = (tiles + kSortGroups - 1) / kSortGroups;
   if (!SMALL) {
-    PGA_CUDA_TRY(launch_behind(false, k_sort_count<FIRST>, kSortGroups, kSortThreads, 0, s, cIn, b.hashes, n, shift, tiles,
-                               perGroup, rows, groups));
-    PGA_CUDA_TRY(launch_behind(false, k_sort_scan, kBins / 32, 1024, 0, s, groups, hist));
+    k_sort_count<FIRST><<<kSortGroups, kSortThreads, 0, s>>>(cIn, b.hashes, n, shift, tiles, perGroup, rows, groups);
+    PGA_CUDA_TRY(cudaGetLastError());
+    k_sort_scan<<<kBins / 32, 1024, 0, s>>>(groups, hist);
+    PGA_CUDA_TRY(cudaGetLastError());
   }
   PGA_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const SortPass a{cIn, b.hashes, vIn, cOut, vOut, n, shift, hist,
