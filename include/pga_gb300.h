@@ -360,6 +360,10 @@ PgaStatus pga_lbvh_build_static(const PgaTerminal* dTerminals, uint64_t n, const
 
 /* Adjoint of the last pga_derive (recordTape = 1): dGradTerminals holds
  * dL/dm (12 floats per terminal, same order as that derivation's output).
+ * The derivation's axioms and parameter blocks are read again and must hold
+ * what they held then: the tape records how each shape ended, not why, and a
+ * change that would have it end otherwise is found out (PGA_ERR_NO_TAPE) for
+ * some rules only; the gradients mean nothing after one.
  * Accumulates dL/dDynParam into dGradParams (numBlocks x blockStride; may be NULL)
  * and dL/d(axiom size) into dGradAxiomSizes (3 per axiom; may be NULL).
  * Both outputs are overwritten, not added to.  One cooperative launch on

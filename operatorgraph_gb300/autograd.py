@@ -9,7 +9,8 @@ pga_adjoint on the engine's recorded tape: the discrete derivation (branches,
 repetition counts, discards) is the one of this forward pass.
 
 The engine must be created with record_tape=True, and backward must run before
-the engine derives again (the tape holds one derivation).
+the engine derives again (the tape holds one derivation) and before `blocks` is
+changed in place (backward reads its values again).
 
 `PathTarget` holds a target derivation's terminal centres and extents keyed
 by derivation path, and `PathTarget.sse(M, paths)` is the fitting loss of

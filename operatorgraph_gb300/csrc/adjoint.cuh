@@ -8,9 +8,12 @@
 // of Rotate's scalar angles -- are changed by no continuous input, so the
 // state that carries gradient is a shape's translation t and size s.
 //
-// Tape: every queued work item has (parent item or kAxiomLink | axiom, child
-// ordinal, entry, child range) in itemTape, every terminal the first two in
-// termLinks.  The reverse sweep maps terminals and items to their parents' child
+// Tape: every queued work item has in itemTape the number of its children (with
+// kOnlyPage when they are all of its shape's), the ordinal of the first, and its
+// own parent item (or kAxiomLink | axiom) and ordinal there; every terminal has
+// the last two in termLinks.  Entry and child range stay in the item's record.
+// The axioms and parameter blocks are read again as the derivation read them.
+// The reverse sweep maps terminals and items to their parents' child
 // slots, then takes the levels from the deepest up: an item sums its children's
 // gradients -- in closed form where its rule's children pass them on unchanged
 // (adj_sums), else replaying its expansion and each child's 1 -> 1 chain
@@ -794,7 +797,8 @@ __device__ __forceinline__ float column_dot(const Shape& x, uint32_t src, const 
 // and the sums of lanes that share an item add up.  2^shift neighbouring lanes
 // share item i (the same i, valid and shift in all of them); `part` is the
 // lane's number among them.  Items of other rules are left to the first lane
-// and adj_page.
+// and adj_page.  (adj_page finds out when a child's chain no longer ends as the
+// tape says, because an input has changed since; here nothing does.)
 //
 // With c a child, o_c its offset along the split axis, N_c its size there,
 // S the item's size, go / gN the gradients with respect to o_c and N_c:
@@ -1103,7 +1107,7 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v) {
 //   2. each block scans its chunk into child keys and marks its slots empty;
 //   3. every terminal and work item enters its slot (a terminal of an axiom's
 //      root goes straight to the axiom's sizes);
-//   4. the levels from the deepest up, one adj_page per work item.
+//   4. the levels from the deepest up, each work item by adj_sums or adj_page.
 // The level bounds, the item and the terminal counts are the forward launch's
 // final state, read on the device, so no host round trip is needed.  A failed
 // or overflowed forward pass leaves the gradients zero (the engine report
